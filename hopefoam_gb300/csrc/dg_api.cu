@@ -72,11 +72,19 @@ EulerArgs base_args(dg_ctx* c, int flux) {
 
 int run_stage(dg_ctx* c, const EulerArgs& a, int precision) {
     cudaError_t e;
-    if (precision == DG_PREC_FP64) e = launch_euler_fp64(c->N, a, c->stream);
+    if (precision == DG_PREC_FP64) e = launch_euler_fp64(c->N, a, c->oz, c->stream);
     else if (precision == DG_PREC_SPLIT) e = launch_euler_split(c->N, a, c->split, c->stream);
     else return fail(c, DG_ERR_ARG, "unknown precision");
     if (e != cudaSuccess) return cuda_fail(c, e, "euler stage launch");
     return DG_OK;
+}
+
+// The FP64 stage reports bounded-wait timeouts in a mapped host word, read
+// once the stream has been synchronised.
+int fp64_status(dg_ctx* c) {
+    if (!c->oz.h_status || !*(volatile int*)c->oz.h_status) return DG_OK;
+    *(volatile int*)c->oz.h_status = 0;
+    return fail(c, DG_ERR_TIMEOUT, "FP64 stage: tensor-core completion wait timed out");
 }
 
 // The split kernel reports bounded-wait timeouts in a device status word.
@@ -259,6 +267,10 @@ int dg_ctx_create(const dg_mesh_desc* m, const dg_opts* o, dg_ctx** out) {
     if (m->EToV) c->etov_host.assign(m->EToV, m->EToV + 3 * (size_t)K);
     c->vxy_host.assign(m->VXY, m->VXY + 6 * (size_t)K);
     if (split_setup(c) != DG_OK) c->split.ready = false;
+    if (setup_euler_fp64_tc(c->N, c->ops, c->oz) != cudaSuccess) {
+        dg_ctx_destroy(c);
+        return DG_ERR_CUDA;
+    }
     if (cudaDeviceSynchronize() != cudaSuccess) { dg_ctx_destroy(c); return DG_ERR_CUDA; }
     *out = c;
     return DG_OK;
@@ -268,6 +280,7 @@ int dg_ctx_destroy(dg_ctx* c) {
     if (!c) return DG_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
     split_teardown(c);
+    teardown_euler_fp64_tc(c->oz);
     ipdg_teardown(c);
     limiter_teardown(c);
     for (void* p : c->allocs) cudaFree(p);
@@ -349,7 +362,7 @@ int dg_download_state(dg_ctx* c, double* q_host) {
     if (rc) return rc;
     DG_CUDA(c, cudaMemcpyAsync(q_host, c->d_stage, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
-    return DG_OK;
+    return fp64_status(c);
 }
 
 int dg_set_boundary_traces(dg_ctx* c, const double* tr) {
@@ -380,7 +393,7 @@ int dg_euler_rhs(dg_ctx* c, int flux, int precision, double* rhs_host) {
     DG_CUDA(c, cudaMemcpyAsync(rhs_host, c->d_stage, (size_t)c->K * 4 * c->Np * sizeof(double), cudaMemcpyDeviceToHost,
                                c->stream));
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
-    return DG_OK;
+    return fp64_status(c);
 }
 
 int dg_euler_rhs_device(dg_ctx* c, int flux, int precision, double* rhs_dev) {
@@ -417,9 +430,12 @@ int dg_forward_euler_stage(dg_ctx* c, double dt, int flux, int precision) {
 
 int dg_sync(dg_ctx* c) {
     if (!c) return DG_ERR_ARG;
-    if (c->split.ready) return check_split_status(c, DG_PREC_SPLIT);
+    if (c->split.ready) {
+        const int rc = check_split_status(c, DG_PREC_SPLIT);
+        if (rc) return rc;
+    }
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
-    return DG_OK;
+    return fp64_status(c);
 }
 
 int dg_lserk4_step(dg_ctx* c, double dt, int nsteps, int flux, int precision) {

@@ -66,6 +66,7 @@ struct dg_ctx {
     int cur = 0;
     bool btrace_set = false;
     dgk::SplitPlan split;
+    dgk::OzPlan oz;  // FP64 stage on the tensor cores
     struct IpdgState* ipdg = nullptr;
     std::vector<void*> allocs;
     size_t bytes = 0;

@@ -54,8 +54,22 @@ struct EulerArgs {
     const float* dtk32;    // FP32 copy of dtk (the split-precision path)
 };
 
+// operator images and status word of the tensor-core FP64 stage (euler_fp64_tc.cu)
+struct OzPlan {
+    bool ready = false;
+    int sms = 0;
+    void* d_image = nullptr;
+    int* d_eb = nullptr;
+    int* status = nullptr;    // device address of h_status
+    int* h_status = nullptr;  // mapped host word: a bounded wait gave up
+};
+
+cudaError_t setup_euler_fp64_tc(int N, const dgb::RefOps& ops, OzPlan& plan);
+void teardown_euler_fp64_tc(OzPlan& plan);
+cudaError_t launch_euler_fp64_tc(int N, const EulerArgs& a, const OzPlan& plan, cudaStream_t s);
+
 // launchers (return cudaError_t of the launch)
-cudaError_t launch_euler_fp64(int N, const EulerArgs& a, cudaStream_t s);
+cudaError_t launch_euler_fp64(int N, const EulerArgs& a, const OzPlan& plan, cudaStream_t s);
 cudaError_t launch_to_internal(const double* ref, double* q, const int* ring, int K, int Np, cudaStream_t s);
 cudaError_t launch_to_reference(const double* q, double* ref, const int* ring, int K, int Np, cudaStream_t s);
 

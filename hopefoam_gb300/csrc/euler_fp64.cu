@@ -16,8 +16,11 @@
 // Each element evaluates the flux of its own three faces with its own outward
 // normal; F*(q-,q+,n) = -F*(q+,q-,-n) makes this the reference's
 // owner/neighbour lift (defaultConvectionScheme.C:93-128) up to round-off.
-// On GB300 the FP64 pipe (~2 DFMA/clk/SM) bounds this kernel; it is the
-// parity path, the split-precision kernel is the fast one.
+// On GB300 the FP64 pipe (~2 DFMA/clk/SM) bounds this kernel (2.67 ms per
+// stage at K = 32768, N = 5), so the stage normally runs in
+// euler_fp64_tc.cu (0.42 ms), whose contractions are exact integer products
+// on the tensor cores.  This kernel serves cubature rules (the caller's, with
+// every context) whose digit sums cannot be shown to stay exact there.
 #include "dg_internal.hpp"
 #include "euler_flux.cuh"
 
@@ -206,7 +209,8 @@ static cudaError_t launch_n(const EulerArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_euler_fp64(int N, const EulerArgs& a, cudaStream_t s) {
+cudaError_t launch_euler_fp64(int N, const EulerArgs& a, const OzPlan& plan, cudaStream_t s) {
+    if (plan.ready) return launch_euler_fp64_tc(N, a, plan, s);
     switch (N) {
         case 1: return launch_n<1>(a, s);
         case 2: return launch_n<2>(a, s);

@@ -102,7 +102,7 @@ extern "C" int dg_euler_rhs_noalloc(dg_ctx* c, const double* q_dev, double* rhs_
     a.flux = flux;
     a.mode = dgk::MODE_RHS;
     a.gamma = c->gamma;
-    e = dgk::launch_euler_fp64(c->N, a, c->stream);
+    e = dgk::launch_euler_fp64(c->N, a, c->oz, c->stream);
     if (e != cudaSuccess) return nfail(c, DG_ERR_CUDA, std::string("euler rhs: ") + cudaGetErrorString(e));
     e = dgk::launch_to_reference(rhs_int, rhs_dev, c->d_ring, c->K, c->Np, c->stream);
     if (e != cudaSuccess) return nfail(c, DG_ERR_CUDA, std::string("to_reference: ") + cudaGetErrorString(e));

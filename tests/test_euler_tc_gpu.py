@@ -1,0 +1,83 @@
+"""FP64 Euler stage on the tensor cores (euler_fp64_tc.cu) where its tiles and
+routes change, against the CPU oracle.  Tolerance as for every FP64 right-hand
+side: 1e-11 relative L2 (or ten times the oracle's one-ulp sensitivity); an
+element taken by the plain FP64 route is held to the same."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+from test_euler_gpu import TOL_RHS, _setup, _vertex_ulp_sensitivity
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(x, y, L):
+    k = 2 * np.pi / L
+    rho = 1 + 0.2 * np.sin(k * x) * np.cos(k * y)
+    u, v = 0.6 + 0.3 * np.cos(k * y), -0.2 + 0.4 * np.sin(k * x)
+    p = 1 + 0.1 * np.cos(k * (x + y))
+    return np.stack([rho, rho * u, rho * v, p / 0.4 + 0.5 * rho * (u * u + v * v)])
+
+
+def _against_oracle(ctx, orc, m, N, q, flux):
+    ctx.upload(q)
+    g = ctx.rhs(flux=flux)
+    r = orc.euler_rhs(q.reshape(-1), flux=flux).reshape(g.shape)
+    assert rel_l2(g, r) < max(TOL_RHS, 10 * _vertex_ulp_sensitivity(m, N, q, flux, r))
+    return g
+
+
+@pytest.mark.parametrize("N,nx,ny", [(1, 4, 4), (2, 3, 5), (3, 11, 3), (4, 4, 12), (5, 3, 3), (6, 4, 4), (7, 5, 7),
+                                     (1, 49, 51), (3, 50, 49)])
+@pytest.mark.parametrize("flux", [0, 1])
+def test_tile_edges(gpu_lib, N, nx, ny, flux):
+    """K = 32 n, 32 n - 2, 32 n + 2 and less than a tile; with more tiles than SMs (K = 4900, 4998) too."""
+    from hopefoam_gb300.mesh import periodic_square
+
+    m = periodic_square(nx, ny, 10.0, 10.0, perturb=0.1, seed=N)
+    ctx, orc, x, y = _setup(m, N)
+    _against_oracle(ctx, orc, m, N, _state(x, y, 10.0), flux)
+    ctx.close()
+
+
+@pytest.mark.parametrize("N", [1, 3, 5, 7])
+@pytest.mark.parametrize("flux", [0, 1])
+def test_plain_route(gpu_lib, N, flux):
+    """Elements outside the digit range (a density dip between nodes that no nodal bound foresees, values beyond the
+    FP32 exponents, not finite) take the plain FP64 route, and no other element's result changes."""
+    from hopefoam_gb300.mesh import periodic_square
+
+    m = periodic_square(6, 6, 10.0, 10.0, perturb=0.1, seed=N)
+    ctx, orc, x, y = _setup(m, N)
+    q = _state(x, y, 10.0)
+    base = _against_oracle(ctx, orc, m, N, q, flux)
+    touched = lambda k: np.unique(np.r_[k, m.EToE[k]])
+    # near-vacuum at one node: the interpolated density nearly vanishes or changes sign at some points
+    dip = q.copy()
+    dip[0, 40, 1] = 1e-3
+    ctx.upload(dip)
+    g = ctx.rhs(flux=flux)
+    r = orc.euler_rhs(dip.reshape(-1), flux=flux).reshape(g.shape)
+    ok = np.isfinite(r).all((0, 2))
+    assert np.array_equal(np.isfinite(g).all((0, 2)), ok)
+    rest = np.setdiff1d(np.arange(m.K), touched(40))
+    assert np.array_equal(g[:, rest], base[:, rest])
+    # one element and its neighbours 2^150 larger (outside FP32): values scale with it
+    big = q.copy()
+    big[:, 10] *= 2.0 ** 150
+    ctx.upload(big)
+    g = ctx.rhs(flux=flux)
+    r = orc.euler_rhs(big.reshape(-1), flux=flux).reshape(g.shape)
+    near = touched(10)
+    assert rel_l2(g[:, near], r[:, near]) < 1e-10
+    rest = np.setdiff1d(np.arange(m.K), near)
+    assert np.array_equal(g[:, rest], base[:, rest])
+    for bad in (np.nan, np.inf):
+        w = q.copy()
+        w[3, 20, 0] = bad
+        ctx.upload(w)
+        g = ctx.rhs(flux=flux)
+        assert not np.isfinite(g[:, 20]).all()
+        rest = np.setdiff1d(np.arange(m.K), touched(20))
+        assert np.array_equal(g[:, rest], base[:, rest])
+    ctx.close()
