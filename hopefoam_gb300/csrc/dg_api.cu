@@ -267,7 +267,7 @@ int dg_ctx_create(const dg_mesh_desc* m, const dg_opts* o, dg_ctx** out) {
     if (m->EToV) c->etov_host.assign(m->EToV, m->EToV + 3 * (size_t)K);
     c->vxy_host.assign(m->VXY, m->VXY + 6 * (size_t)K);
     if (split_setup(c) != DG_OK) c->split.ready = false;
-    if (setup_euler_fp64_tc(c->N, c->ops, c->oz) != cudaSuccess) {
+    if (setup_euler_fp64_tc(c->N, c->ops, c->K, c->oz) != cudaSuccess) {
         dg_ctx_destroy(c);
         return DG_ERR_CUDA;
     }

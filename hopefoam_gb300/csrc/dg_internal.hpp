@@ -60,11 +60,12 @@ struct OzPlan {
     int sms = 0;
     void* d_image = nullptr;
     int* d_eb = nullptr;
+    unsigned char* d_flags = nullptr;
     int* status = nullptr;    // device address of h_status
     int* h_status = nullptr;  // mapped host word: a bounded wait gave up
 };
 
-cudaError_t setup_euler_fp64_tc(int N, const dgb::RefOps& ops, OzPlan& plan);
+cudaError_t setup_euler_fp64_tc(int N, const dgb::RefOps& ops, int K, OzPlan& plan);
 void teardown_euler_fp64_tc(OzPlan& plan);
 cudaError_t launch_euler_fp64_tc(int N, const EulerArgs& a, const OzPlan& plan, cudaStream_t s);
 

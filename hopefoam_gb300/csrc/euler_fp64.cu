@@ -18,7 +18,7 @@
 // owner/neighbour lift (defaultConvectionScheme.C:93-128) up to round-off.
 // On GB300 the FP64 pipe (~2 DFMA/clk/SM) bounds this kernel (2.67 ms per
 // stage at K = 32768, N = 5), so the stage normally runs in
-// euler_fp64_tc.cu (0.42 ms), whose contractions are exact integer products
+// euler_fp64_tc.cu (0.40 ms), whose contractions are exact integer products
 // on the tensor cores.  This kernel serves cubature rules (the caller's, with
 // every context) whose digit sums cannot be shown to stay exact there.
 #include "dg_internal.hpp"

@@ -16,26 +16,33 @@
 // only the four warps of one such group ever wait for each other (named
 // barriers); warp 16 feeds the tensor core (operator pieces arrive by bulk
 // copies in a ring, consumed in a fixed order) and all hand-overs are
-// mbarriers, so warps in their integer phases overlap warps in their FP64
-// phase.  Per tile:
+// mbarriers.  Per tile:
 //   1. own nodes and neighbour face nodes -> digit operands;
 //   2. traces at the face points (two products), numerical flux, digits;
 //   3. per chunk of 16 cubature points: state at the points (product),
 //      fluxes, digits, product into the result accumulators;
 //   4. result rows -> FP64, stage update.
+// The metrics carry the element's time step, so the results are dt R.
 // The digits of a row share one exponent.  For the nodal rows it is the row's
 // own; for the flux rows it comes from the face fluxes and from a bound on
 // the volume fluxes formed from the element's nodal extremes.  An element
 // whose fluxes leave that bound, or with values that are not finite or
-// outside the FP32 exponent range, is recomputed by its warps in plain FP64,
-// as euler_fp64.cu does it (plain_element).  All of this is per element:
-// results do not depend on an element's place in the mesh.
+// outside the FP32 exponent range, is left to plain FP64 after the tiles, as
+// euler_fp64.cu does it (plain_element).  All of this is per element: results
+// do not depend on an element's place in the mesh.
 //
-// Measured, LSERK4 step with the state's layout changes, against the kernel of
-// euler_fp64.cu: K = 32768, N = 5, LF 13.36 -> 2.13 ms; K = 9798, N = 7, Roe
-// 13.14 -> 1.10 ms; K = 3200, N = 3, LF 392 -> 139 us; SSP-RK2 step at
-// K = 512, N = 2 42 -> 31 us.  So it is taken at every order and size.
+// Measured, LSERK4 stage, against the kernel of euler_fp64.cu: K = 32768,
+// N = 5, LF 2.66 ms -> 396 us; K = 9800, N = 7, Roe 2.62 ms -> 281 us;
+// K = 3200, N = 3, LF 78 -> 41 us; so it is taken at every order and size.
 // Right-hand sides against 80-bit arithmetic: 2.7e-13 relative at N = 5, both.
+// What bounds it now: the FP64 pipe is busy half of the time (58,000 of
+// 117,000 cycles per tile at N = 5: 25,000 in the face fluxes, 30,000 in the
+// volume fluxes); the four warps of a scheduler run their integer phases
+// (digits, sums) in step, and the pipe idles through them.  Measured and left
+// out: a second flux operand with the next tile's operands made during this
+// tile's last product (400 us), the next chunk's sums interleaved with this
+// chunk's fluxes (400 us), MMA issue in rolled loops (456 us: one thread
+// issues them, and at 100 cycles an MMA the products fell behind).
 //
 // Every mbarrier wait is bounded; on a timeout the CTA stops waiting, sets
 // the status word, lets its copies and MMAs in flight end, frees its tensor
@@ -59,6 +66,7 @@ struct OzArgs {
     const unsigned char* image;
     const int* eb;
     int* status;
+    unsigned char* flags;  // [tiles][4] elements per group left to plain FP64
 };
 
 __device__ __forceinline__ uint32_t idesc_f16(int n) {
@@ -85,6 +93,15 @@ __device__ __forceinline__ void transpose4(double x[4], int lane) {
     }
 }
 
+// waits for the columns requested into d; their uses stay behind the wait
+// because the values pass through it
+template <int R>
+__device__ __forceinline__ void arrived(float (&d)[R][4]) {
+    umma::tmem_ld_wait();
+#pragma unroll
+    for (int s = 0; s < R; s++) asm volatile("" : "+f"(d[s][0]), "+f"(d[s][1]), "+f"(d[s][2]), "+f"(d[s][3]));
+}
+
 // four consecutive columns of seven digit groups (stride P) -> FP64 values
 // of the lane's row
 template <int P>
@@ -92,12 +109,11 @@ __device__ __forceinline__ void load7(uint32_t taddr, int ebab, double x[4]) {
     float d[7][4];
 #pragma unroll
     for (int s = 0; s < 7; s++) umma::tmem_ld4(taddr + s * P, d[s]);
-    umma::tmem_ld_wait();
+    arrived(d);
 #pragma unroll
     for (int c = 0; c < 4; c++)
-        x[c] = oz::combine7(oz::acc_int22(d[0][c]), oz::acc_int22(d[1][c]), oz::acc_int22(d[2][c]),
-                            oz::acc_int22(d[3][c]), oz::acc_int22(d[4][c]), oz::acc_int22(d[5][c]),
-                            oz::acc_int22(d[6][c]), ebab);
+        x[c] = oz::combine7(oz::acc_int22(d[0][c]), oz::acc_int22(d[1][c]), oz::acc_int22(d[2][c]), oz::acc_int22(d[3][c]),
+                            oz::acc_int22(d[4][c]), oz::acc_int22(d[5][c]), oz::acc_int22(d[6][c]), ebab);
 }
 
 struct FaceSide {
@@ -155,7 +171,50 @@ __device__ __forceinline__ void roe_flux_fast(double g1, double nx, double ny, c
     F[3] = 0.5 * fe;
 }
 
+// bounded wait on an mbarrier phase
+__device__ __forceinline__ bool bounded_wait(uint64_t* bar, uint32_t phase) {
+    uint32_t left;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mov.u32 %0, %3;\n\t"
+        "OZ_POLL:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra OZ_DONE;\n\t"
+        "sub.u32 %0, %0, 1;\n\t"
+        "setp.ne.u32 p, %0, 0;\n\t"
+        "@p bra OZ_POLL;\n\t"
+        "OZ_DONE:\n\t}"
+        : "=&r"(left)
+        : "r"(umma::smem_u32(bar)), "r"(phase), "n"(kWaitLimit)
+        : "memory");
+    return left != 0u;
+}
+
 __device__ __forceinline__ void group_sync(int sub) { asm volatile("bar.sync %0, 128;" ::"r"(sub + 1) : "memory"); }
+
+// One operator piece: operand slices at `as` (AS bytes apart, reduction KP)
+// times the piece's digit blocks of P rows, digit pairs into columns d + P s.
+// Nodal operands keep the pairs i + j <= 6, flux operands i + j <= 7 (the zero
+// block 7 of their operator starts every group).  Unrolled: one thread issues
+// every MMA, and their rate is the piece's latency.
+template <int AS, int KP, int P, bool FLUX>
+__device__ __forceinline__ void digit_product(uint32_t d, uint32_t as, uint32_t bs, bool start) {
+    constexpr uint32_t SBO = (uint32_t)(KP / 8) << 7;
+    const uint64_t ad = umma::smem_desc(as, 128, SBO), bd = umma::smem_desc(bs, 128, SBO);
+#pragma unroll
+    for (int i = 0; i < oz::kSlices; i++) {
+        constexpr int S = oz::kSlices;
+        const int nj = FLUX ? (i == 0 ? S + 1 : S + 1 - i) : S - i;
+        const int n = (nj * P + 15) & ~15;
+#pragma unroll
+        for (int ks = 0; ks < KP / 16; ks++)
+#pragma unroll
+            for (int n0 = 0; n0 < n; n0 += 256)
+                umma::mma_bf16(d + i * P + n0, ad + (uint32_t)((i * AS + ks * 256) >> 4),
+                               bd + (uint32_t)(((n0 >> 3) * SBO + ks * 256) >> 4), idesc_f16(n - n0 < 256 ? n - n0 : 256),
+                               i + ks > 0 || !start ? 1u : 0u);
+    }
+}
 
 // place of scratch value i of element group `sub` in an operand whose slices
 // are `stride` bytes and hold `per` bytes of the group's rows each
@@ -164,22 +223,47 @@ __device__ __forceinline__ double* striped(unsigned char* base, int sub, int i, 
     return reinterpret_cast<double*>(base + (size_t)s * stride + (size_t)sub * per) + (i - s * n);
 }
 
-// Right-hand side of element k in plain FP64 by the 128 threads of its group,
+// factor of the fluxes: the element's time step (1 for a right-hand side)
+__device__ __forceinline__ double step_of(const EulerArgs& a, int k) {
+    return a.mode == MODE_RHS ? 1.0 : a.dtk ? a.dt * a.dtk[k] : a.dt;
+}
+
+// the stage's update of one value: right-hand side times the step, state q0,
+// and the RK register or the old state o0
+__device__ __forceinline__ void stage_update(const EulerArgs& a, size_t idx, double dR, double q0, double o0) {
+    if (a.mode == MODE_RHS) {
+        a.rhs[idx] = dR;
+    } else if (a.mode == MODE_LSERK) {
+        const double r = fma(a.rka, o0, dR);
+        a.res[idx] = r;
+        a.qout[idx] = fma(a.rkb, r, q0);
+    } else if (a.mode == MODE_EULER) {
+        a.qout[idx] = q0 + dR;
+    } else {
+        a.qout[idx] = 0.5 * (o0 + (q0 + dR));
+    }
+}
+
+// Stage of element k in plain FP64 by the 128 threads of its group,
 // operation for operation as euler_stage_fp64_kernel forms it
-template <int N, typename Sc, typename Out>
-__device__ __noinline__ void plain_element(const EulerArgs& a, int k, int t, int sub, Sc sc, Out out) {
+template <int N, typename Sc>
+__device__ __noinline__ void plain_element(const EulerArgs& a, int k, int t, int sub, Sc sc) {
     using D = OzDims<N>;
     constexpr int Np = D::Np, Ng = D::Ng, Nfp = D::Nfp, Nfq = D::Nfq, NB = D::NB, NF = D::NF;
     const double* qe = a.qin + (size_t)k * 4 * Np;
     const double* gk = a.geo + (size_t)k * 4;
     const double rx = gk[0], sx = gk[1], ry = gk[2], sy = gk[3], gamma = a.gamma;
+#pragma unroll 1
     for (int g = t; g < Ng; g += 128) {
         double q[4] = {0, 0, 0, 0}, fx[4], fy[4];
+#pragma unroll 1
         for (int p = 0; p < Np; p++) {
             const double w = a.ops.Vg[g * Np + p];
+#pragma unroll 1
             for (int v = 0; v < 4; v++) q[v] += w * qe[v * Np + p];
         }
         euler_phys_flux(gamma, q, fx, fy);
+#pragma unroll 1
         for (int v = 0; v < 4; v++) {
             *sc(v * Ng + g) = rx * fx[v] + ry * fy[v];
             *sc((4 + v) * Ng + g) = sx * fx[v] + sy * fy[v];
@@ -190,8 +274,10 @@ __device__ __noinline__ void plain_element(const EulerArgs& a, int k, int t, int
         double nx, ny, fsc, lam = 0;
         face_normal(f, rx, sx, ry, sy, nx, ny, fsc);
         auto side = [&](int i, double qm[4], double qp[4]) {
+#pragma unroll 1
             for (int v = 0; v < 4; v++) {
                 double m = 0, p = 0;
+#pragma unroll 1
                 for (int j = 0; j < Nfp; j++) {
                     const double w = a.ops.If[i * Nfp + j];
                     m += w * qe[v * Np + (f * N + j) % NB];
@@ -209,31 +295,39 @@ __device__ __noinline__ void plain_element(const EulerArgs& a, int k, int t, int
             }
         };
         if (a.flux != 1)
+#pragma unroll 1
             for (int i = 0; i < Nfq; i++) {
                 double qm[4], qp[4];
                 side(i, qm, qp);
                 lam = fmax(lam, wave_speed(gamma, nx, ny, qm));
                 lam = fmax(lam, wave_speed(gamma, nx, ny, qp));
             }
+#pragma unroll 1
         for (int i = 0; i < Nfq; i++) {
             double qm[4], qp[4], F[4];
             side(i, qm, qp);
             if (a.flux == 1) roe_flux(gamma, nx, ny, qm, qp, F);
             else lf_flux(gamma, nx, ny, lam, qm, qp, F);
+#pragma unroll 1
             for (int v = 0; v < 4; v++) *sc(8 * Ng + v * NF + f * Nfq + i) = fsc * F[v];
         }
     }
     group_sync(sub);
+#pragma unroll 1
     for (int it = t; it < 4 * Np; it += 128) {
         const int v = it / Np, p = it - v * Np;
         double acc = 0, acc2 = 0, accf = 0;
+#pragma unroll 1
         for (int g = 0; g < Ng; g++) {
             acc += a.ops.Sr[p * Ng + g] * *sc(v * Ng + g);
             acc2 += a.ops.Ss[p * Ng + g] * *sc((4 + v) * Ng + g);
         }
         acc += acc2;
+#pragma unroll 1
         for (int q = 0; q < NF; q++) accf += a.ops.Lift[p * NF + q] * *sc(8 * Ng + v * NF + q);
-        *out(it) = acc - accf;
+        const size_t idx = (size_t)k * 4 * Np + it;
+        stage_update(a, idx, step_of(a, k) * (acc - accf), a.qin[idx],
+                     a.mode == MODE_LSERK ? a.res[idx] : a.mode == MODE_SSP2 ? a.qold[idx] : 0.0);
     }
     group_sync(sub);
 }
@@ -261,19 +355,19 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
     volatile int* dead = reinterpret_cast<volatile int*>(smem + D::OFF_DEAD);
     uint32_t* tmemS = reinterpret_cast<uint32_t*>(smem + D::OFF_TMEM);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + D::OFF_BAR);
-    uint64_t *bAready = bars, *bTrFull = bars + 1, *bTrRead = bars + 2, *bA2w = bars + 3, *bA2free = bars + 4,
-             *bD1full = bars + 5, *bD1read = bars + 6, *bFin = bars + 7, *bFull = bars + 8, *bEmpty = bFull + D::NSLOT;
+    uint64_t *bOwn = bars, *bTrFull = bars + 1, *bTrRead = bars + 2, *bD1full = bars + 3, *bD1read = bars + 4,
+             *bFin = bars + 5, *bA2w = bars + 6, *bA2free = bars + 7, *bFull = bars + 8, *bEmpty = bFull + D::NSLOT;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        umma::mbar_init(bAready, 16);
+        umma::mbar_init(bOwn, 16);
         umma::mbar_init(bTrFull, 1);
         umma::mbar_init(bTrRead, 16);
-        umma::mbar_init(bA2w, 16);
-        umma::mbar_init(bA2free, 1);
         umma::mbar_init(bD1full, 1);
         umma::mbar_init(bD1read, 16);
         umma::mbar_init(bFin, 1);
+        umma::mbar_init(bA2w, 16);
+        umma::mbar_init(bA2free, 1);
         for (int i = 0; i < D::NSLOT; i++) {
             umma::mbar_init(bFull + i, 1);
             umma::mbar_init(bEmpty + i, 1);
@@ -291,7 +385,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
 
     auto wait = [&](uint64_t* bar, uint32_t phase) {
         if (*dead) return;
-        if (!umma::mbar_wait(bar, phase, kWaitLimit)) *dead = 1;
+        if (!bounded_wait(bar, phase)) *dead = 1;
     };
 
     if (warp == 16) {
@@ -307,8 +401,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 const int s = (int)(nload % D::NSLOT);
                 if (nload >= D::NSLOT) wait(bEmpty + s, (uint32_t)((nload / D::NSLOT - 1) & 1));
                 if (*dead) return;
-                const uint32_t n = loadp == 0 ? D::B1F : loadp == 1 ? D::B3 : loadp == 2 ? D::B1
-                                   : loadp == 3 || loadp == D::PIECES - 1 ? D::B2 : (loadp & 1) ? D::B2 : D::B1;
+                const uint32_t n = loadp == 0 ? D::B1F : loadp == 1 ? D::B3 : D::piece_flux(loadp) ? D::B2 : D::B1;
                 umma::mbar_arrive_expect_tx(bFull + s, n);
                 umma::bulk_g2s(smem + D::OFF_RING + s * D::SLOT, oa.image + loado, n, bFull + s);
                 loado += n;
@@ -329,84 +422,39 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 nuse++;
                 load();
             };
-            // digit product of a nodal operand (slice stride AS, reduction KP) with P points
-            auto product = [&](uint32_t d, uint32_t as, int AS, int KP, uint32_t bs, int P) {
-                const uint32_t sbo = (uint32_t)(KP >> 3) << 7;
-                for (int i = 0; i < oz::kSlices; i++) {
-                    const uint32_t id = idesc_f16((oz::kSlices - i) * P);
-                    for (int ks = 0; ks < KP / 16; ks++)
-                        umma::mma_bf16(d + i * P, umma::smem_desc(as + i * AS + ks * 256, 128, sbo),
-                                       umma::smem_desc(bs + ks * 256, 128, sbo), id, i + ks > 0 ? 1u : 0u);
-                }
-            };
-            // flux operand times a B2 piece into the result groups (pairs i + j <= 7;
-            // digit block 7 of the operator is zero and starts every group)
-            auto product2 = [&](uint32_t bs, bool first) {
-                const uint32_t as = umma::smem_u32(A2), sbo = 4u << 7;
-                for (int i = 0; i < oz::kSlices; i++) {
-                    const int nj = i == 0 ? 8 : 8 - i;
-                    const int n = (nj * D::NP2 + 15) & ~15;
-                    for (int ks = 0; ks < 2; ks++)
-                        for (int n0 = 0; n0 < n; n0 += 256) {
-                            const int nn = n - n0 < 256 ? n - n0 : 256;
-                            umma::mma_bf16(tmem + D::T_RES + i * D::NP2 + n0,
-                                           umma::smem_desc(as + i * D::A2S + ks * 256, 128, sbo),
-                                           umma::smem_desc(bs + (uint32_t)(n0 >> 3) * sbo + ks * 256, 128, sbo), idesc_f16(nn),
-                                           first && i + ks == 0 ? 0u : 1u);
-                        }
-                }
-            };
-            uint32_t phA = 0, phTR = 0, phW = 0, phR = 0;
-            for (int tile = blockIdx.x; tile < ntiles && !*dead; tile += gridDim.x) {
-                wait(bAready, phA);
-                phA ^= 1;
-                uint32_t b = take();
-                if (*dead) break;
-                umma::fence_after_sync();
-                product(tmem + D::T_OWN, umma::smem_u32(A1), D::A1S, K1, b, 32);
-                done();
-                b = take();
-                if (*dead) break;
-                product(tmem + D::T_NBR, umma::smem_u32(A2), D::A2S, 32, b, 32);
-                umma::commit(bTrFull);
-                done();
-                wait(bTrRead, phTR);
-                phTR ^= 1;
-                b = take();
-                if (*dead) break;
-                umma::fence_after_sync();
-                product(tmem + D::T_CUB, umma::smem_u32(A1), D::A1S, K1, b, 16);
-                umma::commit(bD1full);
-                done();
-                wait(bA2w, phW);
-                phW ^= 1;
-                b = take();
-                if (*dead) break;
-                umma::fence_after_sync();
-                product2(b, true);
-                umma::commit(bA2free);
-                done();
-                for (int c = 0; c < D::NC; c++) {
-                    wait(bD1read, phR);
-                    phR ^= 1;
-                    if (c + 1 < D::NC) {
-                        b = take();
-                        if (*dead) break;
-                        umma::fence_after_sync();
-                        product(tmem + D::T_CUB, umma::smem_u32(A1), D::A1S, K1, b, 16);
-                        umma::commit(bD1full);
-                        done();
+            const uint32_t a1 = umma::smem_u32(A1), a2 = umma::smem_u32(A2);
+            uint32_t phO = 0, phTR = 0, phR = 0, phW = 0;
+#pragma unroll 1
+            for (int tile = blockIdx.x; tile < ntiles && !*dead; tile += gridDim.x)
+#pragma unroll 1
+                for (int p = 0; p < D::PIECES; p++) {
+                    const bool last = p == D::PIECES - 1, flux = D::piece_flux(p);
+                    if (p == 0) {
+                        wait(bOwn, phO);
+                        phO ^= 1;
+                    } else if (p == 2) {
+                        wait(bTrRead, phTR);
+                        phTR ^= 1;
+                    } else if (p > 3 && (!flux || last)) {
+                        wait(bD1read, phR);
+                        phR ^= 1;
                     }
-                    wait(bA2w, phW);
-                    phW ^= 1;
-                    b = take();
+                    if (flux || p == 1) {
+                        wait(bA2w, phW);
+                        phW ^= 1;
+                    }
+                    const uint32_t b = take();
                     if (*dead) break;
                     umma::fence_after_sync();
-                    product2(b, false);
-                    umma::commit(bA2free);
+                    if (flux) digit_product<D::A2S, 32, D::NP2, true>(tmem + D::T_RES, a2, b, p == 3);
+                    else if (p == 0) digit_product<D::A1S, K1, 32, false>(tmem + D::T_OWN, a1, b, true);
+                    else if (p == 1) digit_product<D::A2S, 32, 32, false>(tmem + D::T_NBR, a2, b, true);
+                    else digit_product<D::A1S, K1, 16, false>(tmem + D::T_CUB, a1, b, true);
+                    if (flux || p == 1) umma::commit(bA2free);
+                    if (p == 1) umma::commit(bTrFull);
+                    else if (!flux && p > 1) umma::commit(bD1full);
                     done();
                 }
-            }
             // everything issued ends before the CTA does
             umma::commit(bFin);
             umma::mbar_wait(bFin, 0, kWaitLimit);
@@ -427,7 +475,9 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
         const int ebV = ebS[D::NP2], ebI = ebS[D::NP2 + 1];
         const double g1 = a.gamma - 1.0;
         const float g1f = fabsf((float)g1);
-        uint32_t phT = 0, phD = 0, phF = 0;
+        constexpr int IT = (32 * Np + 127) / 128;
+        uint32_t phT = 0, phD = 0;
+        int use = 0;
         auto waitw = [&](uint64_t* bar, uint32_t phase) {
             wait(bar, phase);
             __syncwarp();
@@ -436,26 +486,46 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
             __syncwarp();
             if (lane == 0) umma::mbar_arrive(bar);
         };
+        // The second operand (neighbour traces, face fluxes, then each chunk's fluxes)
+        // has one buffer: free once its last product is done, and handed over
+        auto flux_free = [&]() {
+            if (use) waitw(bA2free, (uint32_t)(use - 1) & 1u);
+        };
+        auto flux_written = [&]() {
+            umma::fence_async_smem();
+            arrive(bA2w);
+            use++;
+        };
+#pragma unroll 1
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            const int k0 = tile * 32;
-            const int gk0 = k0 + 8 * sub;  // the group's elements
+            const int gk0 = tile * 32 + 8 * sub;  // the group's elements
+            const int nval = max(0, min(8, a.K - gk0)) * 4 * Np;
+            const size_t g0 = (size_t)gk0 * 4 * Np;
+            double q0[IT], o0[IT];
+            int eb2[4];
             // ---- 1. geometry, digits of the nodal rows
+            group_sync(sub);
             if (t < 24) {
                 const int e8 = t / 3, f = t - 3 * e8, k = min(gk0 + e8, a.K - 1);
                 const double* gk = a.geo + (size_t)k * 4;
                 double* nr = nrmS + (8 * sub + e8) * 9 + f * 3;
-                face_normal(f, gk[0], gk[1], gk[2], gk[3], nr[0], nr[1], nr[2]);
+                const double gx = f == 0 ? -gk[1] : f == 1 ? gk[0] + gk[1] : -gk[0];
+                const double gy = f == 0 ? -gk[3] : f == 1 ? gk[2] + gk[3] : -gk[2];
+                const double s2 = fma(gx, gx, gy * gy), is = oz::rsqrt64(s2);
+                nr[0] = gx * is;
+                nr[1] = gy * is;
+                nr[2] = s2 * is * step_of(a, k);
                 connS[(8 * sub + e8) * 3 + f] = a.conn[(size_t)k * 3 + f];
             } else if (t >= 32 && t < 64) {
-                const int i = t - 32;
-                geoS[sub * 32 + i] = a.geo[(size_t)min(gk0 + (i >> 2), a.K - 1) * 4 + (i & 3)];
+                const int i = t - 32, k = min(gk0 + (i >> 2), a.K - 1);
+                geoS[sub * 32 + i] = a.geo[(size_t)k * 4 + (i & 3)] * step_of(a, k);
             } else if (t >= 64 && t < 96) {
                 maxf[sub * 32 + t - 64] = 0u;
             } else if (t == 96) {
                 flagS[sub] = 0u;
             }
             constexpr int LPR = D::LPR, RPW = 32 / LPR;  // rows per warp pass
-#pragma unroll
+#pragma unroll 1
             for (int pass = 0; pass < 8 / RPW; pass++) {
                 const int i = pass * RPW + lane / LPR, kb = lane % LPR, v = cg;
                 const bool in = gk0 + i < a.K;
@@ -495,28 +565,34 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                                        oz::digit_pair(y[4], y[5], s), oz::digit_pair(y[6], y[7], s));
                 }
             }
+            umma::fence_async_smem();
+            arrive(bOwn);
             group_sync(sub);
-            {   // neighbour traces: 4 lanes per row, 8 face nodes each
-                const int i = lane >> 2, kb = lane & 3, v = cg;
+            {
+                const int i = lane >> 2, kb = lane & 3, v = cg;  // neighbour traces: 4 lanes per row, 8 face nodes each
                 const bool in = gk0 + i < a.K;
                 double x[8];
-                uint32_t mx = 0;
+                const double* src[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
                     const int k = 8 * kb + j, f = k / Nfp, jn = k - f * Nfp;
-                    x[j] = 0.0;
+                    src[j] = nullptr;
                     if (in && k < D::NT) {
                         const int c = connS[(8 * sub + i) * 3 + f];
-                        if (c >= 0) {
-                            const int fn = c & 3, jj = ((c >> 2) & 1) ? (N - jn) : jn;
-                            int pos = fn * N + jj;
-                            if (pos >= NB) pos -= NB;
-                            x[j] = a.qin[((size_t)(c >> 3) * 4 + v) * Np + pos];
-                        } else {
-                            x[j] = a.btrace[((size_t)(-1 - c) * 4 + v) * Nfp + jn];
-                        }
+                        const int fn = c & 3, jj = ((c >> 2) & 1) ? (N - jn) : jn;
+                        int pos = fn * N + jj;
+                        if (pos >= NB) pos -= NB;
+                        src[j] = c >= 0 ? a.qin + ((size_t)(c >> 3) * 4 + v) * Np + pos
+                                        : a.btrace + ((size_t)(-1 - c) * 4 + v) * Nfp + jn;
                     }
                 }
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    x[j] = 0.0;
+                    if (src[j]) x[j] = *src[j];
+                }
+                uint32_t mx = 0;
+                flux_free();
 #pragma unroll
                 for (int j = 0; j < 8; j++) mx = max(mx, oz::mag_hi(x[j]));
                 mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
@@ -535,11 +611,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                     *reinterpret_cast<uint4*>(dst + s * D::A2S) =
                         make_uint4(oz::digit_pair(y[0], y[1], s), oz::digit_pair(y[2], y[3], s),
                                    oz::digit_pair(y[4], y[5], s), oz::digit_pair(y[6], y[7], s));
+                flux_written();
             }
-            umma::fence_async_smem();
-            arrive(bAready);
             // a bound on the volume flux rows of element e from its nodal extremes (FP32)
-            const bool live = k0 + e < a.K;
+            const bool live = tile * 32 + e < a.K;
             const double rx = geoS[e * 4], sx = geoS[e * 4 + 1], ry = geoS[e * 4 + 2], sy = geoS[e * 4 + 3];
             float est[4];
             {
@@ -562,64 +637,60 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
             umma::fence_after_sync();
             const int ownrow = e * 4 + jv;
             const int eb1 = oz::row_bound(maxq[ownrow]);
-            constexpr int GR = (D::NG4 + 3) / 4;  // rounds of 4-point groups per warp
-            double qm[GR][4], qp[GR][4];
-#pragma unroll
-            for (int r = 0; r < GR; r++) {
-                const int gi = cg + 4 * r;
-                if (gi < D::NG4) {
-                    load7<32>(tlane + D::T_OWN + 4 * gi, eb1 + ebI, qm[r]);
-                    load7<32>(tlane + D::T_NBR + 4 * gi, e3S[ownrow] + ebI, qp[r]);
-                }
-            }
-            umma::fence_before_sync();
-            arrive(bTrRead);
-#pragma unroll
-            for (int r = 0; r < GR; r++)
-                if (cg + 4 * r < D::NG4) {
-                    transpose4(qm[r], lane);
-                    transpose4(qp[r], lane);
-                }
+            // A warp takes the 4-point groups cg and cg + 4 (when there are more than
+            // four).  The rounds are rolled loops that shift their results (F, and the
+            // jump for the Lax-Friedrichs flux) from one register set to the other.
+            constexpr int GR = (D::NG4 + 3) / 4;
+            double F[4], J[4], F0[4] = {0, 0, 0, 0}, J0[4] = {0, 0, 0, 0};
             uint32_t bad = 0;
-            double F[GR][4];
-            if (a.flux == 1) {
+#pragma unroll 1
+            for (int r = 0; r < GR; r++) {
+                const int gi = cg + 4 * r, pt = 4 * gi + jv;
 #pragma unroll
-                for (int r = 0; r < GR; r++) {
-                    const int pt = 4 * (cg + 4 * r) + jv;
-                    if (cg + 4 * r < D::NG4) {
-                        const int f = min(pt, NF - 1) / Nfq;
-                        const double* nr = nrmS + e * 9 + f * 3;
-                        roe_flux_fast(g1, nr[0], nr[1], qm[r], qp[r], F[r]);
-#pragma unroll
-                        for (int v = 0; v < 4; v++) F[r][v] = pt < NF && live ? nr[2] * F[r][v] : 0.0;
-                    }
+                for (int v = 0; v < 4; v++) {
+                    F0[v] = F[v];
+                    J0[v] = J[v];
                 }
-            } else {
+                if (gi < D::NG4) {
+                    double qm[4], qp[4];
+                    load7<32>(tlane + D::T_OWN + 4 * gi, eb1 + ebI, qm);
+                    load7<32>(tlane + D::T_NBR + 4 * gi, e3S[ownrow] + ebI, qp);
+                    transpose4(qm, lane);
+                    transpose4(qp, lane);
+                    const double* nr = nrmS + e * 9 + min(pt, NF - 1) / Nfq * 3;
+                    if (a.flux == 1) {
+                        roe_flux_fast(g1, nr[0], nr[1], qm, qp, F);
 #pragma unroll
-                for (int r = 0; r < GR; r++) {
-                    const int pt = 4 * (cg + 4 * r) + jv;
-                    if (cg + 4 * r < D::NG4) {
-                        const int f = min(pt, NF - 1) / Nfq;
-                        const double nx = nrmS[e * 9 + f * 3], ny = nrmS[e * 9 + f * 3 + 1];
-                        const FaceSide m = face_side(g1, nx, ny, qm[r]), p = face_side(g1, nx, ny, qp[r]);
-                        const double um = m.mn * m.r, up = p.mn * p.r;
-                        const double wm = fabs(um) + oz::sqrt64(fabs(a.gamma * m.p * m.r));
-                        const double wp = fabs(up) + oz::sqrt64(fabs(a.gamma * p.p * p.r));
+                        for (int v = 0; v < 4; v++) F[v] = pt < NF && live ? nr[2] * F[v] : 0.0;
+                    } else {
+                        // half the scaled normal in place of the normal: every term of the
+                        // flux and the wave speeds carry the factor h = sJ/J / 2
+                        const double h = 0.5 * nr[2], nx = h * nr[0], ny = h * nr[1], gh = a.gamma * (h * h);
+                        const FaceSide m = face_side(g1, nx, ny, qm), p = face_side(g1, nx, ny, qp);
+                        const double um = m.mn * m.r, up = p.mn * p.r, ps = m.p + p.p;
+                        const double wm = fabs(um) + oz::sqrt64(fabs(gh * m.p * m.r));
+                        const double wp = fabs(up) + oz::sqrt64(fabs(gh * p.p * p.r));
                         // magnitudes compare as integers (a NaN is the largest)
                         const long long wmi = __double_as_longlong(wm) & 0x7FFFFFFFFFFFFFFFll,
                                         wpi = __double_as_longlong(wp) & 0x7FFFFFFFFFFFFFFFll;
                         if (pt < NF) lamS[e * NF + pt] = __longlong_as_double(wmi > wpi ? wmi : wpi);
-                        F[r][0] = m.mn + p.mn;
-                        F[r][1] = fma(qm[r][1], um, fma(qp[r][1], up, nx * (m.p + p.p)));
-                        F[r][2] = fma(qm[r][2], um, fma(qp[r][2], up, ny * (m.p + p.p)));
-                        F[r][3] = fma(qm[r][3] + m.p, um, (qp[r][3] + p.p) * up);
+                        F[0] = m.mn + p.mn;
+                        F[1] = fma(qm[1], um, fma(qp[1], up, nx * ps));
+                        F[2] = fma(qm[2], um, fma(qp[2], up, ny * ps));
+                        F[3] = fma(qm[3] + m.p, um, (qp[3] + p.p) * up);
+#pragma unroll
+                        for (int v = 0; v < 4; v++) J[v] = qm[v] - qp[v];
                     }
                 }
-                group_sync(sub);
-#pragma unroll
-                for (int r = 0; r < GR; r++) {
-                    const int pt = 4 * (cg + 4 * r) + jv;
-                    if (cg + 4 * r < D::NG4) {
+            }
+            umma::fence_before_sync();
+            arrive(bTrRead);
+            if (a.flux != 1) group_sync(sub);
+#pragma unroll 1
+            for (int r = 0; r < GR; r++) {
+                const int gi = cg + 4 * (GR - 1 - r), pt = 4 * gi + jv;  // last round first
+                if (gi < D::NG4) {
+                    if (a.flux != 1) {
                         const int f = min(pt, NF - 1) / Nfq;
                         long long l = 0;
 #pragma unroll
@@ -627,26 +698,29 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                             const long long w = __double_as_longlong(lamS[e * NF + f * Nfq + i]);
                             l = w > l ? w : l;
                         }
-                        const double lam = __longlong_as_double(l), h = 0.5 * nrmS[e * 9 + f * 3 + 2];
+                        const double lam = __longlong_as_double(l);
 #pragma unroll
-                        for (int v = 0; v < 4; v++)
-                            F[r][v] = pt < NF && live ? h * fma(lam, qm[r][v] - qp[r][v], F[r][v]) : 0.0;
+                        for (int v = 0; v < 4; v++) F[v] = pt < NF && live ? fma(lam, J[v], F[v]) : 0.0;
                     }
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < GR; r++)
-                if (cg + 4 * r < D::NG4) {
 #pragma unroll
                     for (int v = 0; v < 4; v++) {
-                        const uint32_t h = oz::mag_hi(F[r][v]);
+                        const uint32_t h = oz::mag_hi(F[v]);
                         if (h >= 0x7FF00000u) bad = 1u;
                         else atomicMax(maxf + e * 4 + v, h);
                     }
                 }
+                if (GR == 2) {
+#pragma unroll
+                    for (int v = 0; v < 4; v++) {
+                        const double w = F[v];
+                        F[v] = F0[v];
+                        F0[v] = w;
+                        J[v] = J0[v];
+                    }
+                }
+            }
             if (bad) atomicOr(flagS + sub, 1u << el);
             group_sync(sub);
-            int eb2[4];
 #pragma unroll
             for (int v = 0; v < 4; v++) {
                 // one bit above the estimate for points between the nodes
@@ -655,23 +729,28 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 eb2[v] = max(oz::row_bound(maxf[e * 4 + v]), ee);
                 if (eb2[v] > 1700 || (eb2[v] != 0 && eb2[v] < 300)) bad = 1u;
             }
-#pragma unroll
+            flux_free();
+#pragma unroll 1
             for (int r = 0; r < GR; r++) {
-                const int gi = cg + 4 * r, pt = 4 * gi + jv;
+                const int gi = cg + 4 * (GR - 1 - r), pt = 4 * gi + jv;
                 if (gi < D::NG4) {
 #pragma unroll
                     for (int v = 0; v < 4; v++) {
-                        const uint64_t y = oz::biased(F[r][v], eb2[v]);
+                        const uint64_t y = oz::biased(F[v], eb2[v]);
                         unsigned char* dst = A2 + (((4 * sub + v) * 4 + (pt >> 3)) << 7) + (el << 4) + ((pt & 7) << 1);
 #pragma unroll
                         for (int s = 0; s < oz::kSlices; s++)
                             *reinterpret_cast<uint16_t*>(dst + s * D::A2S) = (uint16_t)oz::digit_pair(y, y, s);
                     }
                 }
+                if (GR == 2) {
+#pragma unroll
+                    for (int v = 0; v < 4; v++) F[v] = F0[v];
+                }
             }
-            umma::fence_async_smem();
-            arrive(bA2w);
+            flux_written();
             // ---- 3. volume fluxes, 16 cubature points per chunk
+#pragma unroll 1
             for (int c = 0; c < D::NC; c++) {
                 const int p0 = 16 * c + 4 * cg, pt = p0 + jv;
                 waitw(bD1full, phD);
@@ -701,8 +780,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                         ys[w] = oz::biased(Fs[w], eb2[w]);
                     }
                 }
-                waitw(bA2free, phF);  // the previous product has read the operand
-                phF ^= 1;
+                flux_free();
                 if (p0 < Ng) {
 #pragma unroll
                     for (int w = 0; w < 4; w++) {
@@ -712,63 +790,63 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                             *reinterpret_cast<uint32_t*>(dst + s * D::A2S) = oz::digit_pair(yr[w], ys[w], s);
                     }
                 }
-                umma::fence_async_smem();
-                arrive(bA2w);
+                flux_written();
             }
             if (bad) atomicOr(flagS + sub, 1u << el);
-            // ---- 4. result rows
-            waitw(bA2free, phF);
-            phF ^= 1;
+            // ---- 4. result rows; the update's operands are on their way meanwhile
+            const double* other = a.mode == MODE_LSERK ? a.res : a.mode == MODE_SSP2 ? a.qold : nullptr;
+#pragma unroll
+            for (int it = 0; it < IT; it++) {
+                const int i = t + 128 * it;
+                q0[it] = i < nval && a.mode != MODE_RHS ? a.qin[g0 + i] : 0.0;
+                o0[it] = i < nval && other ? other[g0 + i] : 0.0;
+            }
+            flux_free();
             umma::fence_after_sync();
             int ebr = 0;
 #pragma unroll
             for (int v = 0; v < 4; v++) ebr = jv == v ? eb2[v] : ebr;
-            auto R = [&](int i) { return striped(A2, sub, i, D::A2S, 2048); };
-#pragma unroll
+#pragma unroll 1
             for (int n0 = 0; n0 < D::NP2; n0 += 16) {
                 const int n4 = n0 + 4 * cg;
                 if (n4 < Np) {
                     float d[8][4];
 #pragma unroll
                     for (int s = 0; s < 8; s++) umma::tmem_ld4(tlane + D::T_RES + s * D::NP2 + n4, d[s]);
-                    umma::tmem_ld_wait();
+                    arrived(d);
 #pragma unroll
                     for (int j = 0; j < 4; j++)
                         if (n4 + j < Np) {
                             int ds[8];
 #pragma unroll
                             for (int s = 0; s < 8; s++) ds[s] = oz::acc_int24(d[s][j]);
-                            *R((el * 4 + jv) * Np + n4 + j) = oz::combine8(ds, ebr + ebS[n4 + j]);
+                            *striped(A2, sub, (el * 4 + jv) * Np + n4 + j, D::A2S, 2048) = oz::combine8(ds, ebr + ebS[n4 + j]);
                         }
                 }
             }
             umma::fence_before_sync();
             group_sync(sub);
-            for (uint32_t fl = flagS[sub]; fl; fl &= fl - 1) {
-                const int i = __ffs((int)fl) - 1;
-                if (gk0 + i < a.K)
-                    plain_element<N>(a, gk0 + i, t, sub,
-                                     [&](int j) { return striped(A1, sub, j, D::A1S, 32 * K1 * 2); },
-                                     [&](int j) { return R(i * 4 * Np + j); });
-            }
-            const int nval = max(0, min(8, a.K - gk0)) * 4 * Np;
-            for (int i = t; i < nval; i += 128) {
-                const double Rv = *R(i);
-                const size_t idx = (size_t)gk0 * 4 * Np + i;
-                const double dt = a.dtk ? a.dt * a.dtk[gk0 + i / (4 * Np)] : a.dt;
-                switch (a.mode) {
-                    case MODE_RHS: a.rhs[idx] = Rv; break;
-                    case MODE_LSERK: {
-                        const double r = a.rka * a.res[idx] + dt * Rv;
-                        a.res[idx] = r;
-                        a.qout[idx] = a.qin[idx] + a.rkb * r;
-                    } break;
-                    case MODE_EULER: a.qout[idx] = a.qin[idx] + dt * Rv; break;
-                    default: a.qout[idx] = 0.5 * a.qold[idx] + 0.5 * (a.qin[idx] + dt * Rv); break;
+            const uint32_t fl = flagS[sub];
+            if (t == 0) oa.flags[4 * tile + sub] = (unsigned char)fl;
+            // stage update, coalesced
+#pragma unroll
+            for (int it = 0; it < IT; it++) {
+                const int i = t + 128 * it;
+                if (i < nval && !((fl >> (i / (4 * Np))) & 1u)) {
+                    const double Rv = *striped(A2, sub, i, D::A2S, 2048);
+                    const size_t idx = g0 + i;
+                    stage_update(a, idx, Rv, q0[it], o0[it]);
                 }
             }
-            group_sync(sub);  // staging, flags and geometry are rewritten by the next tile
         }
+        // the elements left to plain FP64 (none, as a rule), after the tiles so that
+        // the call costs the loop above no registers
+        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+            for (uint32_t fl = oa.flags[4 * tile + sub]; fl; fl &= fl - 1) {
+                const int k = tile * 32 + 8 * sub + __ffs((int)fl) - 1;
+                if (k < a.K)
+                    plain_element<N>(a, k, t, sub, [&](int j) { return striped(A1, sub, j, D::A1S, 32 * K1 * 2); });
+            }
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -780,7 +858,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
 }
 
 template <int N>
-static cudaError_t setup_tc(const dgb::RefOps& ops, OzPlan& plan) {
+static cudaError_t setup_tc(const dgb::RefOps& ops, int K, OzPlan& plan) {
     const OzImage im = oz_build<N>(ops);
     if (!im.exact) return cudaSuccess;  // not representable: the plain kernel stays
     cudaError_t e = cudaFuncSetAttribute(euler_stage_fp64_tc_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -793,24 +871,25 @@ static cudaError_t setup_tc(const dgb::RefOps& ops, OzPlan& plan) {
         *plan.h_status = 0;
         e = cudaHostGetDevicePointer((void**)&plan.status, plan.h_status, 0);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&plan.d_image, im.bytes.size() + im.eb.size() * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&plan.d_image, im.bytes.size() + im.eb.size() * sizeof(int) + (size_t)(K + 31) / 32 * 4);
     if (e != cudaSuccess) return e;
     plan.d_eb = reinterpret_cast<int*>((unsigned char*)plan.d_image + im.bytes.size());
+    plan.d_flags = reinterpret_cast<unsigned char*>(plan.d_eb + im.eb.size());
     e = cudaMemcpy(plan.d_image, im.bytes.data(), im.bytes.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(plan.d_eb, im.eb.data(), im.eb.size() * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) plan.ready = true;
     return e;
 }
 
-cudaError_t setup_euler_fp64_tc(int N, const dgb::RefOps& ops, OzPlan& plan) {
+cudaError_t setup_euler_fp64_tc(int N, const dgb::RefOps& ops, int K, OzPlan& plan) {
     switch (N) {
-        case 1: return setup_tc<1>(ops, plan);
-        case 2: return setup_tc<2>(ops, plan);
-        case 3: return setup_tc<3>(ops, plan);
-        case 4: return setup_tc<4>(ops, plan);
-        case 5: return setup_tc<5>(ops, plan);
-        case 6: return setup_tc<6>(ops, plan);
-        case 7: return setup_tc<7>(ops, plan);
+        case 1: return setup_tc<1>(ops, K, plan);
+        case 2: return setup_tc<2>(ops, K, plan);
+        case 3: return setup_tc<3>(ops, K, plan);
+        case 4: return setup_tc<4>(ops, K, plan);
+        case 5: return setup_tc<5>(ops, K, plan);
+        case 6: return setup_tc<6>(ops, K, plan);
+        case 7: return setup_tc<7>(ops, K, plan);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -829,7 +908,7 @@ static cudaError_t launch_tc(const OzArgs& oa, const OzPlan& plan, cudaStream_t 
 }
 
 cudaError_t launch_euler_fp64_tc(int N, const EulerArgs& a, const OzPlan& plan, cudaStream_t s) {
-    const OzArgs oa{a, (const unsigned char*)plan.d_image, plan.d_eb, plan.status};
+    const OzArgs oa{a, (const unsigned char*)plan.d_image, plan.d_eb, plan.status, plan.d_flags};
     switch (N) {
         case 1: return launch_tc<1>(oa, plan, s);
         case 2: return launch_tc<2>(oa, plan, s);

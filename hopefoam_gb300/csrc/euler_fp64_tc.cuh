@@ -33,11 +33,15 @@ struct OzDims {
     static constexpr int B3 = oz::kSlices * 32 * 32 * 2;    // neighbour face nodes -> face points
     static constexpr int B1 = oz::kSlices * 16 * K1 * 2;    // own nodes -> one chunk of cubature points
     static constexpr int B2 = (oz::kSlices + 1) * NP2 * 32 * 2;  // one chunk's fluxes (or the face fluxes) -> nodes
+    // order: own traces, neighbour traces, chunk 0's interpolation, face fluxes,
+    // then per chunk c the interpolation of chunk c + 1 and the fluxes of chunk c
     static constexpr int PIECES = 2 * NC + 3;
-    static constexpr int piece_bytes(int i) {
-        return i == 0 ? B1F : i == 1 ? B3 : i == 2 ? B1 : i == 3 ? B2
-               : i == PIECES - 1 ? B2 : (i % 2 == 0 ? B1 : B2);
+    OZ_HD static constexpr bool piece_flux(int p) {
+        return p == 3 || p == PIECES - 1 || (p > 3 && (p & 1));
     }
+    static constexpr int piece_b1(int c) { return c == 0 ? 2 : 4 + 2 * (c - 1); }
+    static constexpr int piece_b2(int c) { return c == NC - 1 ? PIECES - 1 : 5 + 2 * c; }
+    static constexpr int piece_bytes(int p) { return p == 0 ? B1F : p == 1 ? B3 : piece_flux(p) ? B2 : B1; }
     static constexpr size_t piece_off(int i) {
         size_t o = 0;
         for (int j = 0; j < i; j++) o += piece_bytes(j);
@@ -128,16 +132,14 @@ OzImage oz_build(const dgb::RefOps& o) {
         for (long long x : a1) worst1 = std::max(worst1, x);
         for (long long x : a3) worst1 = std::max(worst1, x);
     }
-    auto piece_b1 = [](int c) { return c == 0 ? 2 : 4 + 2 * (c - 1); };
-    auto piece_b2 = [](int c) { return c == D::NC - 1 ? D::PIECES - 1 : 5 + 2 * c; };
     for (int c = 0; c < D::NC; c++) {
         std::vector<long long> a((size_t)8 * 16, 0);
         for (int p = 0; p < 16 && 16 * c + p < D::Ng; p++) {
             const int g = 16 * c + p;
-            for (int k = 0; k < D::Np; k++) put(piece_b1(c), 16, D::K1, p, k, o.dVg[(size_t)g * D::Np + k], ebV, &a);
+            for (int k = 0; k < D::Np; k++) put(D::piece_b1(c), 16, D::K1, p, k, o.dVg[(size_t)g * D::Np + k], ebV, &a);
             for (int n = 0; n < D::Np; n++) {
-                put(piece_b2(c), D::NP2, 32, n, 2 * p, o.dSr[(size_t)n * D::Ng + g], im.eb[n], &acc2);
-                put(piece_b2(c), D::NP2, 32, n, 2 * p + 1, o.dSs[(size_t)n * D::Ng + g], im.eb[n], &acc2);
+                put(D::piece_b2(c), D::NP2, 32, n, 2 * p, o.dSr[(size_t)n * D::Ng + g], im.eb[n], &acc2);
+                put(D::piece_b2(c), D::NP2, 32, n, 2 * p + 1, o.dSs[(size_t)n * D::Ng + g], im.eb[n], &acc2);
             }
         }
         for (long long x : a) worst1 = std::max(worst1, x);

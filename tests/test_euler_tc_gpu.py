@@ -72,6 +72,15 @@ def test_plain_route(gpu_lib, N, flux):
     assert rel_l2(g[:, near], r[:, near]) < 1e-10
     rest = np.setdiff1d(np.arange(m.K), near)
     assert np.array_equal(g[:, rest], base[:, rest])
+    # the stage update of such elements: q + dt R
+    from hopefoam_gb300 import _lib as L
+
+    dt = 1e-4
+    ctx.upload(big)
+    assert ctx.lib.dg_forward_euler_stage(ctx.h, dt, flux, L.DG_PREC_FP64) == L.DG_OK
+    s = ctx.download()
+    assert rel_l2(s[:, near], big[:, near] + dt * r[:, near]) < 1e-12
+    assert rel_l2(s[:, rest], q[:, rest] + dt * base[:, rest]) < 1e-15
     for bad in (np.nan, np.inf):
         w = q.copy()
         w[3, 20, 0] = bad
