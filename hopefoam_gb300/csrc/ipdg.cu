@@ -1218,9 +1218,9 @@ static cudaError_t pcg_precondition(const IpdgArgs& a, const PcgVecs& v, const L
         if (e == cudaSuccess)
             e = launch_schwarz_collect(*lpc->sw, v.zb, lpc->U, nullptr, v.zl, v.dz, LPC_APPLY, v.S, v.part, s);
         if (e != cudaSuccess) return e;
-        return launch_mg_correction(*v.mg, v.r, v.zl, v.z, v.dz, lmode, v.S, v.part, v.nmax, nullptr, s);
+        return launch_mg_correction(*v.mg, v.r, v.zl, v.z, v.dz, lmode, v.S, v.part, v.nmax, s);
     }
-    if (v.mg) return launch_mg_correction(*v.mg, v.r, v.zb, v.z, v.dz, lmode, v.S, v.part, v.nmax, nullptr, s);
+    if (v.mg) return launch_mg_correction(*v.mg, v.r, v.zb, v.z, v.dz, lmode, v.S, v.part, v.nmax, s);
     if (lpc->sw) {
         e = launch_schwarz_local(*lpc->sw, v.r, v.r32, lpc->U, nullptr, s);
         if (e != cudaSuccess) return e;
@@ -1252,9 +1252,9 @@ cudaError_t launch_pcg_iteration(const IpdgArgs& a, const PcgVecs& v, bool fp32,
         if (e == cudaSuccess)
             e = launch_schwarz_collect(*lpc->sw, v.zb, lpc->U, nullptr, v.zl, v.dz, LPC_APPLY, v.S, v.part, s);
         if (e == cudaSuccess)
-            e = launch_mg_correction(*v.mg, v.r, v.zl, v.z, v.dz, LPC_PCG_ITERATION, v.S, v.part, v.nmax, nullptr, s);
+            e = launch_mg_correction(*v.mg, v.r, v.zl, v.z, v.dz, LPC_PCG_ITERATION, v.S, v.part, v.nmax, s);
     } else if (v.zb && v.mg) {
-        e = launch_mg_correction(*v.mg, v.r, v.zb, v.z, v.dz, LPC_PCG_ITERATION, v.S, v.part, v.nmax, nullptr, s);
+        e = launch_mg_correction(*v.mg, v.r, v.zb, v.z, v.dz, LPC_PCG_ITERATION, v.S, v.part, v.nmax, s);
     } else if (v.zb) {
         if (lpc->sw) {
             e = launch_schwarz_local(*lpc->sw, v.r, v.r32, lpc->U, &v.S->done, s);

@@ -29,7 +29,8 @@ struct IpdgState {
     MgLevels mg{};
     bool mg_ready = false;
     std::string mg_err;
-    std::vector<void*> mg_allocs;
+    void* d_mg = nullptr;  // its matrices and work vectors (kept when a rebuild fits)
+    size_t mg_bytes = 0;
     std::vector<double> fc_host;  // face coefficients as built (boundary types reset sJ from it)
     std::vector<unsigned char> lane_tab;  // IpLaneTab<N> of the two-pass FP32 apply (N <= 5)
     std::vector<int> btype;       // per boundary slot: 0 fixesValue, 1 fixesGradient, 2 neither
@@ -345,7 +346,7 @@ static void build_lane_tab(const dg_ctx* c, const std::vector<double>& DrfT, con
 void ipdg_teardown(dg_ctx* c) {
     if (!c->ipdg) return;
     for (void* p : c->ipdg->allocs) cudaFree(p);
-    for (void* p : c->ipdg->mg_allocs) cudaFree(p);
+    if (c->ipdg->d_mg) cudaFree(c->ipdg->d_mg);
     delete c->ipdg;
     c->ipdg = nullptr;
 }
@@ -370,8 +371,6 @@ static int build_blocks(dg_ctx* c) {
 // (re)builds the multilevel preconditioner of the current operator
 static int mg_setup(dg_ctx* c) {
     IpdgState* s = c->ipdg;
-    for (void* p : s->mg_allocs) cudaFree(p);
-    s->mg_allocs.clear();
     s->mg_ready = false;
     if (c->etov_host.empty()) {
         s->mg_err = "the mesh descriptor has no vertex ids (EToV)";
@@ -385,46 +384,64 @@ static int mg_setup(dg_ctx* c) {
         return ifail(c, DG_ERR_UNSUPPORTED, s->mg_err);
     }
     int rc = 0;
+    // one allocation for everything: places first, then one upload
+    std::vector<unsigned char> blob;
+    std::vector<std::pair<void**, size_t>> place;
     auto up = [&](auto** dst, const auto& h) {
         using T = typename std::remove_reference<decltype(h)>::type::value_type;
-        T* p = nullptr;
-        if (cudaMalloc((void**)&p, std::max<size_t>(h.size(), 1) * sizeof(T)) != cudaSuccess) { rc = 1; return; }
-        s->mg_allocs.push_back(p);
-        if (!h.empty() && cudaMemcpy(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) rc = 1;
-        *dst = p;
-    };
-    auto work = [&](double** dst, int n) {
-        double* p = nullptr;
-        if (cudaMalloc((void**)&p, std::max(n, 1) * sizeof(double)) != cudaSuccess) { rc = 1; return; }
-        s->mg_allocs.push_back(p);
-        *dst = p;
+        place.emplace_back((void**)dst, blob.size());
+        const unsigned char* p = (const unsigned char*)h.data();
+        blob.insert(blob.end(), p, p + h.size() * sizeof(T));
+        blob.resize((blob.size() + 255) / 256 * 256);
     };
     MgLevels& m = s->mg;
     m = MgLevels();
-    m.nl = (int)b.levels.size();
+    m.nl = b.nd + 1;
     m.K = c->K;
     m.Np = c->Np;
     up((int**)&m.etov, c->etov_host);
     up((double**)&m.lam, b.lam);
     up((int**)&m.vptr, b.vptr);
     up((int**)&m.vinc, b.vinc);
-    up((double**)&m.Cinv, b.Cinv);
+    up((double**)&m.V, b.V);
+    size_t work = 0;
     for (int l = 0; l < m.nl; l++) {
         const MgBuild::Level& L = b.levels[l];
         MgLevel& d = m.lv[l];
         d.n = L.n;
-        up((int**)&d.rowptr, L.rowptr);
-        up((int**)&d.col, L.col);
-        up((double**)&d.val, L.val);
-        up((double**)&d.dinv, L.dinv);
-        if (l + 1 < m.nl) {
-            up((int**)&d.agg, L.agg);
-            up((int**)&d.cptr, L.cptr);
-            up((int**)&d.cmem, L.cmem);
-        }
-        work(&d.r, L.n);
-        work(&d.x, L.n);
-        work(&d.t, L.n);
+        work += 3 * ((size_t)L.n + 31) / 32 * 32;
+        if (l + 1 == m.nl) continue;
+        up((int**)&d.bptr, L.B.ptr);
+        up((int**)&d.bcol, L.B.col);
+        up((double**)&d.bval, L.B.val);
+        up((int**)&d.tptr, L.Bt.ptr);
+        up((int**)&d.tcol, L.Bt.col);
+        up((double**)&d.tval, L.Bt.val);
+        up((int**)&d.mptr, L.M.ptr);
+        up((int**)&d.mcol, L.M.col);
+        up((double**)&d.mval, L.M.val);
+    }
+    const size_t need = blob.size() + (work + 96 * m.nl) * sizeof(double);
+    if (need > s->mg_bytes) {
+        if (s->d_mg) cudaFree(s->d_mg);
+        s->d_mg = nullptr;
+        s->mg_bytes = 0;
+        if (cudaMalloc(&s->d_mg, need) != cudaSuccess) rc = 1;
+        else s->mg_bytes = need;
+    }
+    if (!rc) {
+        unsigned char* base = (unsigned char*)s->d_mg;
+        // solves of the previous operator may still be queued on the stream
+        if (cudaStreamSynchronize(c->stream) != cudaSuccess ||
+            cudaMemcpy(base, blob.data(), blob.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            rc = 1;
+        for (auto& q : place) *q.first = base + q.second;
+        double* w = (double*)(base + blob.size());
+        for (int l = 0; l < m.nl; l++)
+            for (double** p : {&m.lv[l].r, &m.lv[l].x, &m.lv[l].w}) {
+                *p = w;
+                w += ((size_t)m.lv[l].n + 31) / 32 * 32;
+            }
     }
     if (!s->d_zb) rc |= ialloc(c, s, &s->d_zb, (size_t)c->K * c->Np);
     if (rc) return ifail(c, DG_ERR_NOMEM, "multilevel preconditioner: device allocation failed");
@@ -934,7 +951,7 @@ int lpc_forward_vec(dg_ctx* c, const double* r, bool with_bj_loss) {
         const double* zref = s->d_zb;
         if (s->lpc_coarse) {
             IP_CUDA(c, launch_mg_correction(s->mg, r, s->d_zb, s->d_zt, nullptr, LPC_PCG_INIT, s->d_S, s->d_ppart,
-                                            s->nmax, nullptr, c->stream));
+                                            s->nmax, c->stream));
             zref = s->d_zt;
         }
         IP_CUDA(c, launch_ipdg_apply(s->args, true, zref, s->d_w, c->stream));
@@ -947,7 +964,7 @@ int lpc_forward_vec(dg_ctx* c, const double* r, bool with_bj_loss) {
                                           nullptr, c->stream));
         if (s->lpc_coarse)  // z = learned local stage + P V(P^T r), in place (the preconditioner it is trained for)
             IP_CUDA(c, launch_mg_correction(s->mg, r, s->d_zt, s->d_zt, nullptr, LPC_PCG_INIT, s->d_S, s->d_ppart,
-                                            s->nmax, nullptr, c->stream));
+                                            s->nmax, c->stream));
     } else {
         IP_CUDA(c, launch_lpc_features(fa, s->d_X, s->d_sc, c->stream));
         IP_CUDA(c, launch_lpc_forward(net, s->d_X, nullptr, K, s->d_Hs, s->d_y, s->d_lpart + 4 * s->G, s->G,

@@ -3,7 +3,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <numeric>
 #include <string>
 #include <vector>
 
@@ -17,35 +16,16 @@ namespace {
 
 constexpr double kOmega = 0.6;  // weighted-Jacobi factor of the smoother
 constexpr int kCoarsest = 500;  // largest operator solved by its dense inverse
-
-// sums duplicate (i, j) triplets into CSR
-void to_csr(int n, std::vector<long long>& key, std::vector<double>& v, MgBuild::Level& L) {
-    std::vector<size_t> ord(key.size());
-    std::iota(ord.begin(), ord.end(), 0);
-    std::sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return key[a] < key[b]; });
-    L.n = n;
-    L.rowptr.assign(n + 1, 0);
-    L.col.clear();
-    L.val.clear();
-    long long last = -1;
-    for (size_t q : ord) {
-        if (key[q] != last) {
-            L.col.push_back((int)(key[q] % n));
-            L.val.push_back(v[q]);
-            L.rowptr[key[q] / n + 1]++;
-            last = key[q];
-        } else {
-            L.val.back() += v[q];
-        }
-    }
-    for (int i = 0; i < n; i++) L.rowptr[i + 1] += L.rowptr[i];
-}
+// Largest level whose whole cycle is held as one dense matrix.  A product with
+// it costs its n^2 doubles from L2 (33 MB at 2000: 5 us) where the levels it
+// stands for cost two launches each (4 us and up).
+constexpr int kDense = 2000;
 
 void jacobi_of(MgBuild::Level& L) {
     L.dinv.assign(L.n, 0.0);
     for (int i = 0; i < L.n; i++)
-        for (int q = L.rowptr[i]; q < L.rowptr[i + 1]; q++)
-            if (L.col[q] == i) L.dinv[i] = kOmega / L.val[q];
+        for (int q = L.A.ptr[i]; q < L.A.ptr[i + 1]; q++)
+            if (L.A.col[q] == i) L.dinv[i] = kOmega / L.A.val[q];
 }
 
 // greedy aggregation on the matrix graph: each unassigned unknown opens an
@@ -56,43 +36,134 @@ int aggregate(const MgBuild::Level& L, std::vector<int>& agg) {
     for (int i = 0; i < L.n; i++) {
         if (agg[i] >= 0) continue;
         agg[i] = na;
-        for (int q = L.rowptr[i]; q < L.rowptr[i + 1]; q++)
-            if (agg[L.col[q]] < 0) agg[L.col[q]] = na;
+        for (int q = L.A.ptr[i]; q < L.A.ptr[i + 1]; q++)
+            if (agg[L.A.col[q]] < 0) agg[L.A.col[q]] = na;
         na++;
     }
     return na;
 }
 
-// dense inverse of an SPD matrix by Cholesky; false if not positive definite
+// rows built one after another from (column, value) contributions; columns
+// sorted, values summed in the order they come
+struct RowBuilder {
+    std::vector<int> at, cols;  // at[c]: 1 + place of column c in this row
+    std::vector<double> vals;
+    explicit RowBuilder(int ncols) : at(ncols, 0) {}
+    void add(int c, double v) {
+        if (at[c] == 0) {
+            cols.push_back(c);
+            vals.push_back(v);
+            at[c] = (int)cols.size();
+        } else {
+            vals[at[c] - 1] += v;
+        }
+    }
+    void finish(MgCsr& m) {
+        // insertion sort: rows are short
+        for (size_t i = 1; i < cols.size(); i++)
+            for (size_t j = i; j > 0 && cols[j - 1] > cols[j]; j--) {
+                std::swap(cols[j - 1], cols[j]);
+                std::swap(vals[j - 1], vals[j]);
+            }
+        for (size_t i = 0; i < cols.size(); i++) {
+            at[cols[i]] = 0;
+            m.col.push_back(cols[i]);
+            m.val.push_back(vals[i]);
+        }
+        m.ptr.push_back((int)m.col.size());
+        cols.clear();
+        vals.clear();
+    }
+};
+
+MgCsr transpose(const MgCsr& a, int rows, int cols) {
+    MgCsr t;
+    t.ptr.assign(cols + 1, 0);
+    for (int c : a.col) t.ptr[c + 1]++;
+    for (int c = 0; c < cols; c++) t.ptr[c + 1] += t.ptr[c];
+    t.col.resize(a.col.size());
+    t.val.resize(a.col.size());
+    std::vector<int> fill(t.ptr.begin(), t.ptr.end() - 1);
+    for (int i = 0; i < rows; i++)
+        for (int q = a.ptr[i]; q < a.ptr[i + 1]; q++) {
+            const int p = fill[a.col[q]]++;
+            t.col[p] = i;
+            t.val[p] = a.val[q];
+        }
+    return t;
+}
+
+// B^T = (I - D A) P, its transpose B, and M = 2 D - D A D of a level
+void cycle_matrices(MgBuild::Level& F, int nc) {
+    F.Bt = MgCsr();
+    F.Bt.ptr.reserve(F.n + 1);
+    F.Bt.ptr.push_back(0);
+    RowBuilder rb(nc);
+    for (int i = 0; i < F.n; i++) {
+        rb.add(F.agg[i], 1.0);
+        for (int q = F.A.ptr[i]; q < F.A.ptr[i + 1]; q++) rb.add(F.agg[F.A.col[q]], -F.dinv[i] * F.A.val[q]);
+        rb.finish(F.Bt);
+    }
+    F.B = transpose(F.Bt, F.n, nc);
+    F.M.ptr = F.A.ptr;
+    F.M.col = F.A.col;
+    F.M.val.resize(F.A.val.size());
+    for (int i = 0; i < F.n; i++)
+        for (int q = F.A.ptr[i]; q < F.A.ptr[i + 1]; q++) {
+            const int j = F.A.col[q];
+            F.M.val[q] = (i == j ? 2.0 * F.dinv[i] : 0.0) - F.dinv[i] * F.A.val[q] * F.dinv[j];
+        }
+}
+
+// dense inverse of an SPD matrix in place (Gauss-Jordan without pivoting: the
+// pivots are the Cholesky ones); false if not positive definite
 bool spd_inverse(int n, std::vector<double>& A) {
-    std::vector<double> Lm(A);
-    for (int j = 0; j < n; j++) {
-        double d = Lm[(size_t)j * n + j];
-        for (int k = 0; k < j; k++) d -= Lm[(size_t)j * n + k] * Lm[(size_t)j * n + k];
+    for (int k = 0; k < n; k++) {
+        double* rk = &A[(size_t)k * n];
+        const double d = rk[k];
         if (!(d > 0)) return false;
-        d = std::sqrt(d);
-        Lm[(size_t)j * n + j] = d;
-        for (int i = j + 1; i < n; i++) {
-            double s = Lm[(size_t)i * n + j];
-            for (int k = 0; k < j; k++) s -= Lm[(size_t)i * n + k] * Lm[(size_t)j * n + k];
-            Lm[(size_t)i * n + j] = s / d;
-        }
-    }
-    // inverse column by column: L y = e_c, L^T x = y
-    std::vector<double> y(n);
-    for (int c = 0; c < n; c++) {
+        const double inv = 1.0 / d;
+        rk[k] = 1.0;
+        for (int j = 0; j < n; j++) rk[j] *= inv;
         for (int i = 0; i < n; i++) {
-            double s = (i == c) ? 1.0 : 0.0;
-            for (int k = 0; k < i; k++) s -= Lm[(size_t)i * n + k] * y[k];
-            y[i] = s / Lm[(size_t)i * n + i];
-        }
-        for (int i = n - 1; i >= 0; i--) {
-            double s = y[i];
-            for (int k = i + 1; k < n; k++) s -= Lm[(size_t)k * n + i] * A[(size_t)k * n + c];
-            A[(size_t)i * n + c] = s / Lm[(size_t)i * n + i];
+            if (i == k) continue;
+            double* ri = &A[(size_t)i * n];
+            const double f = ri[k];
+            if (f == 0.0) continue;
+            ri[k] = 0.0;
+            for (int j = 0; j < n; j++) ri[j] -= f * rk[j];
         }
     }
+    for (int i = 0; i < n; i++)  // the preconditioner has to be symmetric
+        for (int j = 0; j < i; j++) A[(size_t)i * n + j] = A[(size_t)j * n + i] = 0.5 * (A[(size_t)i * n + j] + A[(size_t)j * n + i]);
     return true;
+}
+
+// dense cycle operator of a level from the next one's: V = M + B^T Vc B
+std::vector<double> dense_cycle(const MgBuild::Level& F, int nc, const std::vector<double>& Vc) {
+    const int n = F.n;
+    std::vector<double> T((size_t)nc * n, 0.0), V((size_t)n * n, 0.0);  // T = Vc B
+    for (int c = 0; c < nc; c++) {
+        double* t = &T[(size_t)c * n];
+        const double* v = &Vc[(size_t)c * nc];
+        for (int i = 0; i < n; i++) {
+            double s = 0;
+            for (int q = F.Bt.ptr[i]; q < F.Bt.ptr[i + 1]; q++) s += F.Bt.val[q] * v[F.Bt.col[q]];
+            t[i] = s;
+        }
+    }
+    for (int i = 0; i < n; i++) {
+        double* v = &V[(size_t)i * n];
+        for (int q = F.Bt.ptr[i]; q < F.Bt.ptr[i + 1]; q++) {
+            const double f = F.Bt.val[q];
+            const double* t = &T[(size_t)F.Bt.col[q] * n];
+            for (int j = 0; j < n; j++) v[j] += f * t[j];
+        }
+        for (int q = F.M.ptr[i]; q < F.M.ptr[i + 1]; q++) v[F.M.col[q]] += F.M.val[q];
+    }
+    for (int i = 0; i < n; i++)
+        for (int j = 0; j < i; j++) V[(size_t)i * n + j] = V[(size_t)j * n + i] = 0.5 * (V[(size_t)i * n + j] + V[(size_t)j * n + i]);
+    return V;
 }
 
 }  // namespace
@@ -121,11 +192,8 @@ std::string mg_build(int K, int N, int Np, const int* etov, const double* geo, c
         std::vector<int> fill(out.vptr.begin(), out.vptr.end() - 1);
         for (int q = 0; q < 3 * K; q++) out.vinc[fill[etov[q]]++] = q;
     }
-    // level 0: P^T S P for continuous P1 functions
-    std::vector<long long> key;
-    std::vector<double> val;
-    key.reserve((size_t)9 * K + 64);
-    val.reserve((size_t)9 * K + 64);
+    // level 0: P^T S P for continuous P1 functions, element matrices first
+    std::vector<double> ea((size_t)9 * K);
     for (int k = 0; k < K; k++) {
         const double* g = geo + 4 * (size_t)k;
         const double rx = g[0], sx = g[1], ry = g[2], sy = g[3];
@@ -157,121 +225,170 @@ std::string mg_build(int K, int N, int Np, const int* etov, const double* geo, c
                 for (int d = 0; d < 3; d++) a[c][d] += tau * mf[c][d] - (dn[c] * m1[d] + m1[c] * dn[d]);
         }
         for (int c = 0; c < 3; c++)
-            for (int d = 0; d < 3; d++) {
-                key.push_back((long long)etov[3 * k + c] * nv + etov[3 * k + d]);
-                val.push_back(a[c][d]);
-            }
+            for (int d = 0; d < 3; d++) ea[(size_t)9 * k + 3 * c + d] = a[c][d];
     }
     out.levels.emplace_back();
-    to_csr(nv, key, val, out.levels.back());
-    jacobi_of(out.levels.back());
+    {
+        MgBuild::Level& L = out.levels.back();
+        L.n = nv;
+        L.A.ptr.reserve(nv + 1);
+        L.A.ptr.push_back(0);
+        L.A.col.reserve((size_t)8 * nv);
+        L.A.val.reserve((size_t)8 * nv);
+        RowBuilder rb(nv);
+        for (int v = 0; v < nv; v++) {
+            for (int q = out.vptr[v]; q < out.vptr[v + 1]; q++) {
+                const int k = out.vinc[q] / 3, c = out.vinc[q] - 3 * k;
+                for (int d = 0; d < 3; d++) rb.add(etov[3 * (size_t)k + d], ea[(size_t)9 * k + 3 * c + d]);
+            }
+            rb.finish(L.A);
+        }
+        jacobi_of(L);
+    }
     // aggregation levels
     while (out.levels.back().n > kCoarsest) {
         if ((int)out.levels.size() >= kMgMaxLevels) return "too many levels";
         MgBuild::Level& F = out.levels.back();
         const int na = aggregate(F, F.agg);
         if (na > F.n * 9 / 10) return "aggregation does not coarsen";
-        F.cptr.assign(na + 1, 0);
-        for (int i = 0; i < F.n; i++) F.cptr[F.agg[i] + 1]++;
-        for (int a = 0; a < na; a++) F.cptr[a + 1] += F.cptr[a];
-        F.cmem.assign(F.n, 0);
+        // Galerkin operator: rows of one aggregate after another
+        std::vector<int> cptr(na + 1, 0), cmem(F.n);
+        for (int i = 0; i < F.n; i++) cptr[F.agg[i] + 1]++;
+        for (int a = 0; a < na; a++) cptr[a + 1] += cptr[a];
         {
-            std::vector<int> fill(F.cptr.begin(), F.cptr.end() - 1);
-            for (int i = 0; i < F.n; i++) F.cmem[fill[F.agg[i]]++] = i;
+            std::vector<int> fill(cptr.begin(), cptr.end() - 1);
+            for (int i = 0; i < F.n; i++) cmem[fill[F.agg[i]]++] = i;
         }
-        key.clear();
-        val.clear();
-        for (int i = 0; i < F.n; i++)
-            for (int q = F.rowptr[i]; q < F.rowptr[i + 1]; q++) {
-                key.push_back((long long)F.agg[i] * na + F.agg[F.col[q]]);
-                val.push_back(F.val[q]);
-            }
         MgBuild::Level C;
-        to_csr(na, key, val, C);
+        C.n = na;
+        C.A.ptr.push_back(0);
+        RowBuilder rb(na);
+        for (int a = 0; a < na; a++) {
+            for (int p = cptr[a]; p < cptr[a + 1]; p++)
+                for (int q = F.A.ptr[cmem[p]]; q < F.A.ptr[cmem[p] + 1]; q++) rb.add(F.agg[F.A.col[q]], F.A.val[q]);
+            rb.finish(C.A);
+        }
         jacobi_of(C);
+        cycle_matrices(F, na);
         out.levels.push_back(std::move(C));
     }
-    // coarsest: dense inverse
-    const MgBuild::Level& C = out.levels.back();
-    out.nc = C.n;
-    out.Cinv.assign((size_t)C.n * C.n, 0.0);
-    for (int i = 0; i < C.n; i++)
-        for (int q = C.rowptr[i]; q < C.rowptr[i + 1]; q++) out.Cinv[(size_t)i * C.n + C.col[q]] = C.val[q];
-    if (!spd_inverse(C.n, out.Cinv)) return "coarse operator is not positive definite";
+    // coarsest: dense inverse; then the dense cycle operators of the levels above it
+    out.nd = (int)out.levels.size() - 1;
+    {
+        const MgBuild::Level& C = out.levels.back();
+        out.V.assign((size_t)C.n * C.n, 0.0);
+        for (int i = 0; i < C.n; i++)
+            for (int q = C.A.ptr[i]; q < C.A.ptr[i + 1]; q++) out.V[(size_t)i * C.n + C.A.col[q]] = C.A.val[q];
+        if (!spd_inverse(C.n, out.V)) return "coarse operator is not positive definite";
+    }
+    while (out.nd > 0 && out.levels[out.nd - 1].n <= kDense) {
+        out.V = dense_cycle(out.levels[out.nd - 1], out.levels[out.nd].n, out.V);
+        out.nd--;
+    }
     (void)N;
     return "";
 }
 
 // ---------------------------------------------------------------------------
-// device cycle
+// device cycle: the DG-to-P1 restriction, one launch per sparse level down,
+// one dense product, one launch per level up, and the collect kernel.  Every
+// launch is a few microseconds of dependent L2 reads on vectors that fit L2, so
+// their number is what the cycle costs (three a level down and two up, before
+// the level's matrices were multiplied out).  Measured per application, kernel
+// times with cold caches: K = 32768 (16,641 vertices) 16 launches, 83 us ->
+// 6 launches, 38 us; K = 101,246 (51,000 vertices) 61 us now.  One cluster of
+// 16 blocks for the whole cycle took 41 and 111 us (too few SMs for the first
+// level) and was left out.  Solves: K = 101,246, N = 4, mixed 38.8 -> 31.3 ms;
+// building the levels 95 -> 30 ms there (rows merged in place instead of
+// sorted triplets, a vectorised inverse, one upload).
 
-__global__ void mg_restrict_dg_kernel(MgLevels m, const double* __restrict__ r, double* __restrict__ r1) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= m.lv[0].n) return;
+// r1 = P^T r; eight lanes per vertex, one incident element corner each,
+// summed in a fixed order
+__global__ void __launch_bounds__(256) mg_restrict_dg_kernel(MgLevels m, const double* __restrict__ r,
+                                                             double* __restrict__ r1, const int* __restrict__ done) {
+    if (done && *done) return;
+    __shared__ double lam[36 * 3];
+    for (int i = threadIdx.x; i < 3 * m.Np; i += blockDim.x) lam[i] = m.lam[i];
+    __syncthreads();
+    const int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, l8 = threadIdx.x & 7;
+    const bool ok = v < m.lv[0].n;
     double s = 0;
-    for (int q = m.vptr[v]; q < m.vptr[v + 1]; q++) {
-        const int c = m.vinc[q], k = c / 3, lv = c - 3 * k;
-        const double* rk = r + (size_t)k * m.Np;
-        for (int i = 0; i < m.Np; i++) s += m.lam[i * 3 + lv] * rk[i];
+    if (ok) {
+        const int q1 = m.vptr[v + 1];
+        for (int q = m.vptr[v] + l8; q < q1; q += 8) {
+            const int c = m.vinc[q], k = c / 3, lv = c - 3 * k;
+            const double* rk = r + (size_t)k * m.Np;
+#pragma unroll 6
+            for (int i = 0; i < m.Np; i++) s += lam[i * 3 + lv] * rk[i];
+        }
     }
-    r1[v] = s;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, 8);
+    if (ok && l8 == 0) r1[v] = s;
 }
 
-// x = dinv r
-__global__ void mg_jacobi0_kernel(int n, const double* __restrict__ dinv, const double* __restrict__ r,
-                                  double* __restrict__ x) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) x[i] = dinv[i] * r[i];
-}
-
-// t = r - A x
-__global__ void mg_residual_kernel(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
-                                   const double* __restrict__ val, const double* __restrict__ r,
-                                   const double* __restrict__ x, double* __restrict__ t) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = r[i];
-    for (int q = rowptr[i]; q < rowptr[i + 1]; q++) s -= val[q] * x[col[q]];
-    t[i] = s;
-}
-
-// x += dinv (r - A x), the residual computed in the same pass into t
-__global__ void mg_smooth_kernel(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
-                                 const double* __restrict__ val, const double* __restrict__ dinv,
-                                 const double* __restrict__ r, const double* __restrict__ x,
-                                 double* __restrict__ xo) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = r[i];
-    for (int q = rowptr[i]; q < rowptr[i + 1]; q++) s -= val[q] * x[col[q]];
-    xo[i] = x[i] + dinv[i] * s;
-}
-
-__global__ void mg_restrict_agg_kernel(int nc, const int* __restrict__ cptr, const int* __restrict__ cmem,
-                                       const double* __restrict__ t, double* __restrict__ rc) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= nc) return;
+// sum of a CSR row over LANES lanes (all of a warp's lanes call it); valid in lane 0 of the row's group
+template <int LANES>
+__device__ __forceinline__ double row_dot(const int* __restrict__ ptr, const int* __restrict__ col,
+                                          const double* __restrict__ val, const double* __restrict__ x, int row, bool ok,
+                                          int l) {
     double s = 0;
-    for (int q = cptr[a]; q < cptr[a + 1]; q++) s += t[cmem[q]];
-    rc[a] = s;
+    if (ok) {
+        const int q1 = ptr[row + 1];
+        for (int q = ptr[row] + l; q < q1; q += LANES) s += val[q] * x[col[q]];
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, LANES);
+    return s;
 }
 
-__global__ void mg_prolong_agg_kernel(int n, const int* __restrict__ agg, const double* __restrict__ xc,
-                                      double* __restrict__ x) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) x[i] += xc[agg[i]];
+constexpr int kDownLanes = 16, kMLanes = 4, kUpLanes = 4;  // lanes per row: about a third of its entries each
+
+// r_c = B r (blocks [0, bblocks)) and w = M r (the others)
+__global__ void __launch_bounds__(256) mg_down_kernel(MgLevel a, int nc, int bblocks, const double* __restrict__ r,
+                                                      double* __restrict__ rc, const int* __restrict__ done) {
+    if (done && *done) return;
+    if ((int)blockIdx.x < bblocks) {
+        const int t = blockIdx.x * blockDim.x + threadIdx.x, row = t / kDownLanes, l = t % kDownLanes;
+        const double s = row_dot<kDownLanes>(a.bptr, a.bcol, a.bval, r, row, row < nc, l);
+        if (row < nc && l == 0) rc[row] = s;
+    } else {
+        const int t = (blockIdx.x - bblocks) * blockDim.x + threadIdx.x, row = t / kMLanes, l = t % kMLanes;
+        const double s = row_dot<kMLanes>(a.mptr, a.mcol, a.mval, r, row, row < a.n, l);
+        if (row < a.n && l == 0) a.w[row] = s;
+    }
 }
 
-// x = Cinv r, one warp per row
-__global__ void mg_dense_kernel(int n, const double* __restrict__ Cinv, const double* __restrict__ r,
-                                double* __restrict__ x) {
+// x = w + B^T x_c
+__global__ void __launch_bounds__(256) mg_up_kernel(MgLevel a, const double* __restrict__ xc, const int* __restrict__ done) {
+    if (done && *done) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, row = t / kUpLanes, l = t % kUpLanes;
+    const double s = row_dot<kUpLanes>(a.tptr, a.tcol, a.tval, xc, row, row < a.n, l);
+    if (row < a.n && l == 0) a.x[row] = a.w[row] + s;
+}
+
+// x = V r, one warp per row, r staged in shared memory
+__global__ void __launch_bounds__(256) mg_dense_kernel(int n, const double* __restrict__ V, const double* __restrict__ r,
+                                                       double* __restrict__ x, const int* __restrict__ done) {
+    __shared__ double rs[kDense];
+    if (done && *done) return;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) rs[j] = r[j];
+    __syncthreads();
     const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (row >= n) return;
-    double s = 0;
-    for (int j = lane; j < n; j += 32) s += Cinv[(size_t)row * n + j] * r[j];
+    const double* v = V + (size_t)row * n;
+    double s0 = 0, s1 = 0;
+    int j = lane;
+#pragma unroll 4
+    for (; j + 32 < n; j += 64) {
+        s0 += v[j] * rs[j];
+        s1 += v[j + 32] * rs[j + 32];
+    }
+    if (j < n) s0 += v[j] * rs[j];
+    s0 += s1;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) x[row] = s;
+    for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    if (lane == 0) x[row] = s0;
 }
 
 // z = zb + P x1; r.z; dz mirror; finish like the learned preconditioner's collect
@@ -317,34 +434,21 @@ __global__ void mg_collect_kernel(MgLevels m, const double* __restrict__ zb, con
 static unsigned nb256(int n) { return (unsigned)((n + 255) / 256); }
 
 cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const double* zb, double* z, float* dz,
-                                 int mode, PcgScalars* S, double* part, int grid, const int* done,
-                                 cudaStream_t s) {
-    (void)done;
+                                 int mode, PcgScalars* S, double* part, int grid, cudaStream_t s) {
     const int L = m.nl;
-    mg_restrict_dg_kernel<<<nb256(m.lv[0].n), 256, 0, s>>>(m, r, m.lv[0].r);
-    // down: pre-smooth, restrict the residual
+    const int* done = mode == 3 ? &S->done : nullptr;  // a stopped iteration leaves every vector as it is
+    mg_restrict_dg_kernel<<<nb256(8 * m.lv[0].n), 256, 0, s>>>(m, r, m.lv[0].r, done);
     for (int l = 0; l + 1 < L; l++) {
-        const MgLevel& a = m.lv[l];
-        mg_jacobi0_kernel<<<nb256(a.n), 256, 0, s>>>(a.n, a.dinv, a.r, a.x);
-        mg_residual_kernel<<<nb256(a.n), 256, 0, s>>>(a.n, a.rowptr, a.col, a.val, a.r, a.x, a.t);
-        mg_restrict_agg_kernel<<<nb256(m.lv[l + 1].n), 256, 0, s>>>(m.lv[l + 1].n, a.cptr, a.cmem, a.t, m.lv[l + 1].r);
+        const int nc = m.lv[l + 1].n, bblocks = (int)nb256(kDownLanes * nc);
+        mg_down_kernel<<<bblocks + nb256(kMLanes * m.lv[l].n), 256, 0, s>>>(m.lv[l], nc, bblocks, m.lv[l].r, m.lv[l + 1].r,
+                                                                            done);
     }
-    {
-        const MgLevel& c = m.lv[L - 1];
-        mg_dense_kernel<<<(c.n + 7) / 8, 256, 0, s>>>(c.n, m.Cinv, c.r, c.x);
-    }
-    // up: prolong the correction, post-smooth into t (the level's result: t
-    // below the coarsest, x on the coarsest)
-    for (int l = L - 2; l >= 0; l--) {
-        const MgLevel& a = m.lv[l];
-        const double* xc = (l + 1 == L - 1) ? m.lv[l + 1].x : m.lv[l + 1].t;
-        mg_prolong_agg_kernel<<<nb256(a.n), 256, 0, s>>>(a.n, a.agg, xc, a.x);
-        mg_smooth_kernel<<<nb256(a.n), 256, 0, s>>>(a.n, a.rowptr, a.col, a.val, a.dinv, a.r, a.x, a.t);
-    }
-    const double* x1 = (L == 1) ? m.lv[0].x : m.lv[0].t;
+    const MgLevel& c = m.lv[L - 1];
+    mg_dense_kernel<<<(c.n + 7) / 8, 256, 0, s>>>(c.n, m.V, c.r, c.x, done);
+    for (int l = L - 2; l >= 0; l--) mg_up_kernel<<<nb256(kUpLanes * m.lv[l].n), 256, 0, s>>>(m.lv[l], m.lv[l + 1].x, done);
     const int EB = 256 / m.Np;
     const int ngroups = (m.K + EB - 1) / EB;
-    mg_collect_kernel<<<std::min(ngroups, grid), 256, 0, s>>>(m, zb, x1, r, z, dz, mode, S, part);
+    mg_collect_kernel<<<std::min(ngroups, grid), 256, 0, s>>>(m, zb, m.lv[0].x, r, z, dz, mode, S, part);
     return cudaGetLastError();
 }
 

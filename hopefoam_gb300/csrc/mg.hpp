@@ -7,8 +7,8 @@
 // continuous P1 functions the interior-face terms of SIPG vanish, leaving the
 // P1 stiffness, the Nitsche terms of the fixed-value boundary faces and the
 // Helmholtz mass term), weighted-Jacobi smoothing, coarser levels by greedy
-// vertex aggregation with piecewise-constant transfer, the coarsest solved by
-// a dense inverse.  Everything is linear and symmetric, so plain PCG applies.
+// vertex aggregation with piecewise-constant transfer, the coarsest (at most
+// 500 unknowns) solved by a dense inverse.  Everything is linear and symmetric, so plain PCG applies.
 #pragma once
 
 #include <string>
@@ -23,25 +23,31 @@ namespace dgk {
 
 constexpr int kMgMaxLevels = 10;
 
+// A level as its cycle uses it.  The sweep down starts from x = D r (D =
+// omega / diag A) and the sweep up ends with one Jacobi step, so with R the
+// sum over aggregates and P = R^T its transpose the level's work is linear in
+// r and in the coarse result:
+//   r_c = B r,            B = R (I - A D)
+//   x   = w + B^T x_c,    w = M r,  M = 2 D - D A D
+// (B^T = (I - D A) P).  The sparse matrices B, B^T and M are formed once, so
+// a level is one launch down (B r and M r) and one up.
 struct MgLevel {
     int n = 0;
-    const int* rowptr = nullptr;  // A_l in CSR
-    const int* col = nullptr;
-    const double* val = nullptr;
-    const double* dinv = nullptr;  // omega / diag(A_l)
-    // transfer to level l + 1 (null on the coarsest level)
-    const int* agg = nullptr;      // [n] coarse index of each unknown
-    const int* cptr = nullptr;     // coarse -> members (CSR), deterministic restriction
-    const int* cmem = nullptr;
-    double* r = nullptr;           // work vectors of the cycle
+    const int *bptr = nullptr, *bcol = nullptr;  // B in CSR, nc rows
+    const double* bval = nullptr;
+    const int *tptr = nullptr, *tcol = nullptr;  // B^T in CSR, n rows
+    const double* tval = nullptr;
+    const int *mptr = nullptr, *mcol = nullptr;  // M in CSR, n rows
+    const double* mval = nullptr;
+    double* r = nullptr;  // work vectors of the cycle
     double* x = nullptr;
-    double* t = nullptr;
+    double* w = nullptr;
 };
 
 struct MgLevels {
-    int nl = 0;                    // levels lv[0] (P1 on the vertices) .. lv[nl-1] (the coarsest)
+    int nl = 0;                    // lv[0] (P1 on the vertices) .. lv[nl-1], the level held as a dense matrix
     MgLevel lv[kMgMaxLevels];
-    const double* Cinv = nullptr;  // dense inverse of the coarsest operator (row-major)
+    const double* V = nullptr;     // dense cycle operator of lv[nl-1] (row-major, symmetric)
     int K = 0, Np = 0;
     const int* etov = nullptr;     // [K][3] vertex ids
     const double* lam = nullptr;   // [Np][3] barycentric coordinates of the nodes (ring order)
@@ -50,17 +56,24 @@ struct MgLevels {
 };
 
 // host-side levels
+struct MgCsr {
+    std::vector<int> ptr, col;
+    std::vector<double> val;
+};
+
 struct MgBuild {
     struct Level {
         int n = 0;
-        std::vector<int> rowptr, col, agg, cptr, cmem;
-        std::vector<double> val, dinv;
+        MgCsr A;
+        std::vector<double> dinv;  // omega / diag A
+        std::vector<int> agg;      // coarse index of each unknown (empty on the coarsest level)
+        MgCsr B, Bt, M;
     };
     std::vector<int> vptr, vinc;
     std::vector<double> lam;
     std::vector<Level> levels;  // levels[0]: P1 on the vertices
-    std::vector<double> Cinv;
-    int nc = 0;
+    int nd = 0;                 // levels kept: levels[nd] is the dense one
+    std::vector<double> V;      // its cycle operator, levels[nd].n^2
 };
 
 // Builds the levels; "" on success.  etov: [K][3] vertex ids, geo: [K][4]
@@ -76,7 +89,6 @@ std::string mg_build(int K, int N, int Np, const int* etov, const double* geo, c
 // collect step (mode: 1 init -> S->rz, 2 refresh -> S->rz, 3 iteration ->
 // pcg_finish); dz (mixed precision) is completed as an offset mirror
 cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const double* zb, double* z, float* dz,
-                                 int mode, PcgScalars* S, double* part, int grid, const int* done,
-                                 cudaStream_t s);
+                                 int mode, PcgScalars* S, double* part, int grid, cudaStream_t s);
 
 }  // namespace dgk

@@ -48,3 +48,69 @@ def test_multilevel_iterations_do_not_grow(gpu_lib):
         its.append(st["iterations"])
     print("multilevel iterations at 2k / 8k / 32k interior points:", its)
     assert max(its) < 1.6 * min(its)
+
+
+def _cycle(A, r, omega=0.6, coarsest=500):
+    """One V(1,1) cycle as mg.hpp defines it, on scipy matrices."""
+    import scipy.sparse as sp
+
+    n = A.shape[0]
+    if n <= coarsest:
+        return np.linalg.solve(A.toarray(), r)
+    agg = -np.ones(n, np.int64)
+    na = 0
+    for i in range(n):
+        if agg[i] >= 0:
+            continue
+        agg[i] = na
+        nb = A.indices[A.indptr[i]:A.indptr[i + 1]]
+        agg[nb[agg[nb] < 0]] = na
+        na += 1
+    P = sp.csr_matrix((np.ones(n), (np.arange(n), agg)), shape=(n, na))
+    d = omega / A.diagonal()
+    x = d * r
+    x = x + P @ _cycle((P.T @ A @ P).tocsr(), P.T @ (r - A @ x), omega, coarsest)
+    return x + d * (r - A @ x)
+
+
+@pytest.mark.parametrize("n_interior", [300, 1200, 3000, 12000])
+def test_one_application_against_its_definition(gpu_lib, n_interior):
+    """z = B r + P V(P^T r) of the first iteration (its solution is a multiple of z) against the cycle written out
+    level by level: only the dense inverse; the cycle as one dense matrix; one and two sparse levels above it.
+    Tolerance: round-off (1e-15) times the condition number of the P1 operator (about 1e5 at 12000 vertices), with a
+    factor of 100 for the differently formed coarse operators."""
+    import scipy.sparse as sp
+
+    from hopefoam_gb300 import _lib as L
+    from hopefoam_gb300.euler import reference_operators
+    from hopefoam_gb300.mesh import delaunay_square, load_cubature
+    from hopefoam_gb300.poisson import PressureSolver, poisson_rhs
+    from oracle.oracle import Oracle
+
+    N = 2
+    m = delaunay_square(n_interior, seed=1)
+    ps = PressureSolver(m, N, tau_coef=1.0)
+    b, _ = poisson_rhs(m, N, seed=3)
+    x, st = ps.solve(b, rtol=1e-14, maxit=1, pc=L.DG_PC_MULTILEVEL, precision=L.DG_PREC_FP64, raise_on_fail=False)
+    assert st["status"] == L.DG_ERR_NOT_CONVERGED and st["iterations"] == 1
+    ops = reference_operators(N)
+    orc = Oracle(m, N, load_cubature(3 * (N + 1)))
+    diag, off, _ = orc.ipdg_blocks(tau_coef=1.0)
+    K, Np = m.K, ps.Np
+    lam = np.stack([-(ops["r"] + ops["s"]) / 2, (1 + ops["r"]) / 2, (1 + ops["s"]) / 2], 1)
+    rows = np.repeat(np.arange(K * Np), 3)
+    nv = int(m.EToV.max()) + 1
+    P = sp.csr_matrix((np.tile(lam, (K, 1)).reshape(-1), (rows, np.repeat(m.EToV, Np, axis=0).reshape(-1))), shape=(K * Np, nv))
+    i, j = np.meshgrid(np.arange(Np), np.arange(Np), indexing="ij")
+    k = np.arange(K)
+    blocks = [(k, k, -diag)] + [(k[m.EToE[:, f] >= 0], m.EToE[m.EToE[:, f] >= 0, f], -off[m.EToE[:, f] >= 0, f])
+                                for f in range(3)]
+    S = sum(sp.csr_matrix((v.reshape(-1), ((kr[:, None, None] * Np + i).reshape(-1), (kc[:, None, None] * Np + j).reshape(-1))),
+                          shape=(K * Np, K * Np)) for kr, kc, v in blocks)
+    pattern = sp.csr_matrix((np.ones(9 * K), (np.repeat(m.EToV, 3, axis=1).reshape(-1), np.tile(m.EToV, (1, 3)).reshape(-1))),
+                            shape=(nv, nv))
+    A1 = (P.T @ S @ P).multiply(pattern > 0).tocsr()
+    A1.sort_indices()
+    z = np.linalg.solve(-diag, b.reshape(K, Np, 1)).reshape(-1) + P @ _cycle(A1, P.T @ b)
+    alpha = (b @ z) / (z @ (S @ z))
+    assert rel_l2(x, alpha * z) < 1e-8
