@@ -36,6 +36,7 @@
 #include "dg_ctx.hpp"
 #include "euler_flux.cuh"
 #include "ipdg.hpp"
+#include "ipdg_rows.cuh"
 #include "lpc.hpp"
 #include "mg.hpp"
 #include "pcg_reduce.cuh"
@@ -82,19 +83,6 @@ __device__ __forceinline__ const IpdgOps<float>& ops_of<float>(const IpdgArgs& a
 // Persistent CTAs (a few per SM) stride over the tiles; in the PCG each CTA's
 // share of p.Ap enters one deterministic grid-wide sum whose last CTA also
 // forms alpha (one arrival per CTA, not per tile).
-struct ApplyPcg {
-    const double* p_old;  // previous search direction (read when beta != 0)
-    double* p_new;        // this direction, written for each element's rows
-    PcgScalars* S;        // beta in, pap / alpha out; null outside the PCG
-    double* part;
-    // FP32 offset mirrors (element value minus the element's first-node
-    // value) of z and of the search directions; used by the FP32 apply in the
-    // PCG so that staging needs no FP64 arithmetic per node
-    const float* dz;
-    const float* dp_old;
-    float* dp_new;
-};
-
 template <int N, typename T>
 __global__ void __launch_bounds__(256, 4) ipdg_apply_kernel(IpdgArgs a, const double* __restrict__ u,
                                                          double* __restrict__ y, ApplyPcg pc) {
@@ -605,51 +593,6 @@ __global__ void __launch_bounds__(256, N <= 4 ? 3 : 2) ipdg_lane_face_apply_kern
     }
 }
 
-// diagonal blocks S_kk (column j = S_kk e_j with neighbours zero), FP64
-template <int N>
-__global__ void ipdg_diag_kernel(IpdgArgs a, double* __restrict__ blocks) {
-    using D = IpDims<N>;
-    constexpr int Np = D::Np, Nfp = D::Nfp, Nfq = D::Nfq, NB = 3 * N;
-    const IpdgOps<double>& o = a.o64;
-    const int k = blockIdx.x;
-    const int j = threadIdx.x;  // column
-    if (k >= a.K || j >= Np) return;
-    const double vrr = o.vc[(size_t)k * 3], vrs = o.vc[(size_t)k * 3 + 1], vss = o.vc[(size_t)k * 3 + 2];
-    double col[Np];
-    const double mc = a.mass_coef * a.J[k];
-    for (int i = 0; i < Np; i++)
-        col[i] = vrr * o.Srr[i * Np + j] + vrs * o.Srs2[i * Np + j] + vss * o.Sss[i * Np + j] + mc * o.Mr[i * Np + j];
-    for (int f = 0; f < 3; f++) {
-        const double* fc = o.fc + ((size_t)k * 3 + f) * kFaceCoef;
-        const double arr = fc[0], ass = fc[1];
-        const int c = a.conn[(size_t)k * 3 + f];
-        // u = e_j: own trace / normal derivative at each Gauss point
-        int jf = -1;
-        if (j < NB) {
-            const int d = (j - f * N + NB) % NB;
-            if (d <= N) jf = d;
-        }
-        for (int g = 0; g < Nfq; g++) {
-            const double um = jf >= 0 ? o.If[g * Nfp + jf] : 0.0;
-            const double dm = arr * o.Drf[(f * Nfq + g) * Np + j] + ass * o.Dsf[(f * Nfq + g) * Np + j];
-            const double up = (c >= 0) ? 0.0 : -um;
-            const double dp = (c >= 0) ? 0.0 : dm;
-            const double wJ = fc[5] * o.fw[g];
-            const double jump = um - up, sigma = 0.5 * (dm + dp);
-            const double cc1 = wJ * (fc[4] * jump - sigma), cc2 = -0.5 * wJ * jump;
-            for (int i = 0; i < Np; i++) {
-                double t = cc2 * (arr * o.Drf[(f * Nfq + g) * Np + i] + ass * o.Dsf[(f * Nfq + g) * Np + i]);
-                if (i < NB) {
-                    const int d = (i - f * N + NB) % NB;
-                    if (d <= N) t += cc1 * o.If[g * Nfp + d];
-                }
-                col[i] += t;
-            }
-        }
-    }
-    for (int i = 0; i < Np; i++) blocks[(size_t)k * Np * Np + (size_t)i * Np + j] = col[i];
-}
-
 // in-place inverse of each Np x Np block (Gauss-Jordan, partial pivoting); FP64
 // result plus an FP32 copy
 __global__ void invert_blocks_kernel(double* __restrict__ blocks, float* __restrict__ blocks32, int K, int Np,
@@ -706,41 +649,6 @@ __device__ __forceinline__ void block_sum1(double a, double* oa) {
         double sa = 0;
         for (int w = 0; w < (int)((blockDim.x + 31) >> 5); w++) sa += ra[w];
         *oa = sa;
-    }
-}
-
-// Element-aligned kernels: a group of EB = 256 / Np whole elements, one
-// thread per (element, row), Np a compile-time constant so that the block
-// products unroll (Np independent loads in flight per thread).  Persistent
-// CTAs (a few per SM) stride over the groups, so each grid-wide sum has one
-// arrival per CTA.  The inverse diagonal blocks are stored grouped: for group
-// g and column j the EB x Np entries (element, row) are contiguous,
-//   Pg[((g Np + j) EB + e) Np + i] = P_{g EB + e}[i][j],
-// so the CTA's loads for one column form a single contiguous read.
-//
-// Up to Np = 32 (N <= 6) an element's rows never straddle a warp: each warp
-// holds EW = 32 / Np whole elements (WA), so the rows of an element exchange
-// their values by warp shuffles and the kernels need no CTA barrier per
-// group.  N = 7 (Np = 36) keeps one shared-memory exchange per group.
-template <int NP>
-struct RowDims {
-    static constexpr bool WA = NP <= 32;
-    static constexpr int EW = WA ? 32 / NP : 0;  // elements per warp
-    static constexpr int EB = WA ? 8 * EW : 256 / NP;
-    static constexpr int THREADS = WA ? 256 : (EB * NP + 31) / 32 * 32;  // extra lanes idle but join the reductions
-};
-
-// this thread's (element in the group, row) and its slot in the grouped layout
-template <int NP>
-__device__ __forceinline__ void row_of(int& e, int& i) {
-    if constexpr (RowDims<NP>::WA) {
-        const int lane = threadIdx.x & 31;
-        e = (threadIdx.x >> 5) * RowDims<NP>::EW + lane / NP;
-        i = lane % NP;
-        if (lane >= RowDims<NP>::EW * NP) e = RowDims<NP>::EB;  // idle lane
-    } else {
-        e = threadIdx.x / NP;
-        i = threadIdx.x - e * NP;
     }
 }
 
@@ -1115,6 +1023,7 @@ static cudaError_t apply_n(const IpdgArgs& a, bool fp32, const double* u, double
             return cudaGetLastError();
         }
     }
+    if (!fp32 && a.sblocks) return launch_block_apply(a, u, y, pc, s);
     const int grid = apply_grid<N>(a);
     if (fp32) ipdg_apply_kernel<N, float><<<grid, D::THREADS, 0, s>>>(a, u, y, pc);
     else ipdg_apply_kernel<N, double><<<grid, D::THREADS, 0, s>>>(a, u, y, pc);
@@ -1144,17 +1053,6 @@ int pcg_max_grid(int K, int N, int sms) {
     (void)K;
     (void)N;
     return std::max(8 * sms, 1024);  // element kernels: up to 8 CTAs per SM; apply: 4; learned kernel: 608
-}
-
-cudaError_t launch_ipdg_diag(const IpdgArgs& a, double* blocks, cudaStream_t s) {
-    switch (a.N) {
-#define DIAG_CASE(n) \
-    case n: ipdg_diag_kernel<n><<<a.K, 64, 0, s>>>(a, blocks); break;
-        DIAG_CASE(1) DIAG_CASE(2) DIAG_CASE(3) DIAG_CASE(4) DIAG_CASE(5) DIAG_CASE(6) DIAG_CASE(7)
-#undef DIAG_CASE
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_invert_blocks(double* blocks, float* blocks32, int K, int Np, int* status, cudaStream_t s) {

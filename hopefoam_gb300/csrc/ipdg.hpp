@@ -43,6 +43,8 @@ struct IpdgArgs {
     const void* lane_tab;
     float* lane_ftr;
     float2* lane_p0;
+    // assembled rows for the FP64 iterations (ipdg_block.cu; null: matrix-free)
+    const double* sblocks;
 };
 
 constexpr int kFaceCoef = 6;
@@ -80,6 +82,19 @@ struct PcgScalars {
     unsigned int counter;  // arrival counter of the grid-wide sums
 };
 
+struct ApplyPcg {
+    const double* p_old;  // previous search direction (read when beta != 0)
+    double* p_new;        // this direction, written for each element's rows
+    PcgScalars* S;        // beta in, pap / alpha out; null outside the PCG
+    double* part;
+    // FP32 offset mirrors (element value minus the element's first-node
+    // value) of z and of the search directions; used by the FP32 apply in the
+    // PCG so that staging needs no FP64 arithmetic per node
+    const float* dz;
+    const float* dp_old;
+    float* dp_new;
+};
+
 struct MgLevels;
 
 struct PcgVecs {
@@ -110,7 +125,12 @@ cudaError_t launch_group_blocks(const IpdgArgs& a, const double* blocks, double*
 
 // y = S u (standalone)
 cudaError_t launch_ipdg_apply(const IpdgArgs& a, bool fp32, const double* u, double* y, cudaStream_t s);
+// diagonal blocks S_kk, row-major per element
 cudaError_t launch_ipdg_diag(const IpdgArgs& a, double* blocks, cudaStream_t s);
+// assembled rows of the FP64 iterations: doubles of storage, and their build
+size_t block_rows_size(int K, int Np);
+cudaError_t launch_block_rows(const IpdgArgs& a, double* sblocks, cudaStream_t s);
+cudaError_t launch_block_apply(const IpdgArgs& a, const double* u, double* y, const ApplyPcg& pc, cudaStream_t s);
 cudaError_t launch_invert_blocks(double* blocks, float* blocks32, int K, int Np, int* status, cudaStream_t s);
 struct LpcNet;
 struct LpcFeatArgs;

@@ -35,6 +35,8 @@ struct IpdgState {
     std::vector<unsigned char> lane_tab;  // IpLaneTab<N> of the two-pass FP32 apply (N <= 5)
     std::vector<int> btype;       // per boundary slot: 0 fixesValue, 1 fixesGradient, 2 neither
     double* d_blocks = nullptr;  // FP64 inverse diagonal blocks (row-major per element)
+    double* d_sblocks = nullptr;  // assembled rows of the FP64 iterations, built by the first FP64 solve
+    bool sb_ready = false, sb_none = false;  // current; no memory for them
     double* d_P64 = nullptr;     // the same, grouped layout of the element-aligned kernels
     float* d_P32 = nullptr;      // FP32 copy, grouped
     // solver vectors (ring order)
@@ -357,6 +359,7 @@ extern "C" {
 static int build_blocks(dg_ctx* c) {
     IpdgState* s = c->ipdg;
     const IpdgArgs& a = s->args;
+    s->sb_ready = false;
     IP_CUDA(c, cudaMemsetAsync(s->d_status, 0, sizeof(int), c->stream));
     IP_CUDA(c, launch_ipdg_diag(a, s->d_blocks, c->stream));
     IP_CUDA(c, launch_invert_blocks(s->d_blocks, nullptr, a.K, a.Np, s->d_status, c->stream));
@@ -367,6 +370,43 @@ static int build_blocks(dg_ctx* c) {
     if (st) return ifail(c, DG_ERR_NONFINITE, "singular diagonal block in the SIPG operator");
     return DG_OK;
 }
+
+// FP64 solves run on assembled block rows (ipdg_block.cu) up to this size, on
+// the matrix-free apply above it or where the allocation fails.  The rows win at
+// every order (K = 101,246, N = 4: 0.73 GB, 230 us against 665 us matrix-free),
+// so only the memory they hold draws the line: 8 GB, 3 % of the device, is
+// K = 1.1e6 at N = 4.
+constexpr size_t kBlockRowsMax = (size_t)8 << 30;
+
+// points the FP64 applies of a solve at the block rows while it lives; every
+// other apply stays matrix-free
+struct BlockRows {
+    IpdgState* s;
+    int rc = DG_OK;
+    BlockRows(dg_ctx* c, bool fp64) : s(c->ipdg) {
+        if (!fp64 || s->sb_none) return;
+        const size_t n = block_rows_size(c->K, c->Np);
+        if (!s->d_sblocks) {
+            if (n * sizeof(double) > kBlockRowsMax || cudaMalloc((void**)&s->d_sblocks, n * sizeof(double)) != cudaSuccess) {
+                (void)cudaGetLastError();
+                s->d_sblocks = nullptr;
+                s->sb_none = true;
+                return;
+            }
+            s->allocs.push_back(s->d_sblocks);
+        }
+        if (!s->sb_ready) {
+            const cudaError_t e = launch_block_rows(s->args, s->d_sblocks, c->stream);
+            if (e != cudaSuccess) {
+                rc = ifail(c, DG_ERR_CUDA, std::string("block rows: ") + cudaGetErrorString(e));
+                return;
+            }
+            s->sb_ready = true;
+        }
+        s->args.sblocks = s->d_sblocks;
+    }
+    ~BlockRows() { s->args.sblocks = nullptr; }
+};
 
 // (re)builds the multilevel preconditioner of the current operator
 static int mg_setup(dg_ctx* c) {
@@ -624,6 +664,7 @@ int dg_ipdg_setup(dg_ctx* c, double tau_coef) {
     a.lane_tab = s->lane_tab.empty() ? nullptr : s->lane_tab.data();
     a.lane_ftr = s->d_lane_ftr;
     a.lane_p0 = s->d_lane_p0;
+    a.sblocks = nullptr;
     rc = build_blocks(c);
     if (rc) return rc;
     s->ready = true;
@@ -711,6 +752,8 @@ static int pcg_solve_impl(dg_ctx* c, const double* b_host, double* x_host, doubl
     if (precision != DG_PREC_FP64 && precision != DG_PREC_SPLIT) return ifail(c, DG_ERR_ARG, "unknown precision");
     IpdgState* s = c->ipdg;
     const size_t n = (size_t)c->K * c->Np;
+    const BlockRows rows(c, precision == DG_PREC_FP64);
+    if (rows.rc) return rows.rc;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -849,6 +892,8 @@ int ipdg_solve_device(dg_ctx* c, const double* b_dev, double* x_dev, double rtol
         if (rcm) return rcm;
     }
     const size_t n = (size_t)c->K * c->Np;
+    const BlockRows rows(c, precision == DG_PREC_FP64);
+    if (rows.rc) return rows.rc;
     IP_CUDA(c, cudaMemcpyAsync(s->d_b, b_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     IP_CUDA(c, cudaMemcpyAsync(s->d_x, x_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     double bb = 0;

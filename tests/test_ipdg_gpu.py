@@ -115,3 +115,51 @@ def test_pcg_errors(gpu_lib):
     assert st["status"] == L.DG_ERR_NOT_CONVERGED
     with pytest.raises(L.DGError):
         ps.solve(b, pc=L.DG_PC_LEARNED + 5)
+
+
+@pytest.mark.parametrize("N", range(1, 8))
+@pytest.mark.parametrize("n,mass", [(6, 0.0), (150, 3.0)])
+def test_fp64_iterations_on_block_rows(gpu_lib, N, n, mass):
+    """Three FP64 block-Jacobi iterations (their operator is the assembled block rows) against the same iterations on
+    the oracle's assembled blocks: every order, less than one group of elements and a ragged last group, with the
+    Helmholtz term and with boundary faces without a fixed value.  Round-off times the growth over three iterations
+    of the operator's condition (below 1e6 here): 1e-10."""
+    from hopefoam_gb300 import _lib as L
+    from hopefoam_gb300 import euler
+    from hopefoam_gb300.mesh import delaunay_square, load_cubature
+    from hopefoam_gb300.poisson import PressureSolver
+    from oracle.oracle import Oracle
+
+    m = delaunay_square(n, seed=N)
+    ps = PressureSolver(m, N, tau_coef=1.0)
+    kk, ff = euler.boundary_faces(m)
+    bt = (np.arange(len(kk)) % 3 == 0).astype(np.int32)  # every third face natural
+    assert ps.ctx.lib.dg_ipdg_set_boundary_types(ps.ctx.h, L.iptr(bt)) == L.DG_OK
+    assert ps.ctx.lib.dg_ipdg_set_mass(ps.ctx.h, mass) == L.DG_OK
+    full = np.zeros((m.K, 3), np.int32)
+    full[kk, ff] = np.where(bt == 1, 2, 0)
+    orc = Oracle(m, N, load_cubature(3 * (N + 1)))
+    diag, off, _ = orc.ipdg_blocks_bc(full, tau_coef=1.0)
+    v = m.VXY
+    J = 0.25 * ((v[:, 1, 0] - v[:, 0, 0]) * (v[:, 2, 1] - v[:, 0, 1]) - (v[:, 2, 0] - v[:, 0, 0]) * (v[:, 1, 1] - v[:, 0, 1]))
+    D = -diag + mass * J[:, None, None] * euler.reference_operators(N)["Mref"]
+
+    def S(u):
+        return -orc.blk_apply(-D, off, u)
+
+    rng = np.random.default_rng(N)
+    b = rng.standard_normal(m.K * ps.Np)
+    x, st = ps.solve(b, rtol=1e-14, maxit=3, pc=L.DG_PC_BLOCK_JACOBI, precision=L.DG_PREC_FP64, raise_on_fail=False)
+    assert st["iterations"] == 3
+    xr, r = np.zeros_like(b), b.copy()
+    prec = lambda w: np.linalg.solve(D, w.reshape(m.K, ps.Np, 1)).reshape(-1)
+    z = prec(r)
+    p, rz = z.copy(), r @ z
+    for _ in range(3):
+        Sp = S(p)
+        al = rz / (p @ Sp)
+        xr, r = xr + al * p, r - al * Sp
+        z = prec(r)
+        p, rz = z + (r @ z) / rz * p, r @ z
+    assert rel_l2(x, xr) < 1e-10
+    ps.ctx.close()
