@@ -80,6 +80,7 @@ struct PcgScalars {
     int done;       // 1 converged, 2 breakdown / non-finite
     int it;         // iterations taken
     unsigned int counter;  // arrival counter of the grid-wide sums
+    int gaveup;            // a bounded wait of the cooperative iterations gave up (ipdg_persist.cu)
 };
 
 struct ApplyPcg {
@@ -130,6 +131,7 @@ cudaError_t launch_ipdg_diag(const IpdgArgs& a, double* blocks, cudaStream_t s);
 // assembled rows of the FP64 iterations: doubles of storage, and their build
 size_t block_rows_size(int K, int Np);
 cudaError_t launch_block_rows(const IpdgArgs& a, double* sblocks, cudaStream_t s);
+cudaError_t launch_block_rows(const IpdgArgs& a, float* sblocks, cudaStream_t s);
 cudaError_t launch_block_apply(const IpdgArgs& a, const double* u, double* y, const ApplyPcg& pc, cudaStream_t s);
 cudaError_t launch_invert_blocks(double* blocks, float* blocks32, int K, int Np, int* status, cudaStream_t s);
 struct LpcNet;
@@ -141,6 +143,14 @@ cudaError_t launch_pcg_init(const IpdgArgs& a, const PcgVecs& v, const LpcNet* l
 // device), then x, r, z updates with beta and the stop test on the device
 cudaError_t launch_pcg_iteration(const IpdgArgs& a, const PcgVecs& v, bool fp32, int parity, const LpcNet* lpc,
                                  const LpcFeatArgs* fa, cudaStream_t s);
+// whether one cooperative launch can hold these iterations (ipdg_persist.cu);
+// up to `count` of them from the state in v: rows are the block rows in the
+// arithmetic type, corner [K][3] work space, slots persist_slots() bytes (zero before the
+// first launch) and exchanges the count that goes with them
+bool persist_fits(const IpdgArgs& a, const PcgVecs& v, bool fp32);
+size_t persist_slots();
+cudaError_t launch_pcg_persistent(const IpdgArgs& a, const PcgVecs& v, bool fp32, const void* rows, double* corner,
+                                  void* slots, unsigned long long* exchanges, int parity, int count, cudaStream_t s);
 // residual replacement: z = M r, S->rz (and S->rr) from the current r; beta kept
 cudaError_t launch_pcg_refresh(const IpdgArgs& a, const PcgVecs& v, const LpcNet* lpc, const LpcFeatArgs* fa,
                                cudaStream_t s);

@@ -37,6 +37,11 @@ struct IpdgState {
     double* d_blocks = nullptr;  // FP64 inverse diagonal blocks (row-major per element)
     double* d_sblocks = nullptr;  // assembled rows of the FP64 iterations, built by the first FP64 solve
     bool sb_ready = false, sb_none = false;  // current; no memory for them
+    float* d_sblocks32 = nullptr;  // FP32 rows of the cooperative iterations of small problems
+    bool sb32_ready = false;
+    double* d_corner = nullptr;
+    unsigned char* d_slots = nullptr;
+    unsigned long long exchanges = 0;
     double* d_P64 = nullptr;     // the same, grouped layout of the element-aligned kernels
     float* d_P32 = nullptr;      // FP32 copy, grouped
     // solver vectors (ring order)
@@ -158,6 +163,35 @@ void lpc_descr(dg_ctx* c, LpcNet& net, LpcFeatArgs& fa) {
     fa.perm = s->d_perm;
 }
 
+// the block rows of the cooperative iterations: the FP64 ones of this solve
+// (none if they did not fit), or FP32 ones formed here; *rows stays null when
+// there is no memory for them, and the iterations go by the general path
+int persist_rows(dg_ctx* c, const PcgVecs& v, bool fp32, const void** rows) {
+    IpdgState* s = c->ipdg;
+    *rows = nullptr;
+    auto room = [&](auto** p, size_t n) {
+        if (*p || ialloc(c, s, p, n) == DG_OK) return true;
+        (void)cudaGetLastError();
+        return false;
+    };
+    if (!s->d_slots) {
+        if (!room(&s->d_slots, persist_slots())) return DG_OK;
+        IP_CUDA(c, cudaMemsetAsync(s->d_slots, 0, persist_slots(), c->stream));
+    }
+    if (v.mg && !room(&s->d_corner, (size_t)c->K * 3)) return DG_OK;
+    if (!fp32) {
+        *rows = s->args.sblocks;
+        return DG_OK;
+    }
+    if (!room(&s->d_sblocks32, block_rows_size(c->K, c->Np))) return DG_OK;
+    if (!s->sb32_ready) {
+        IP_CUDA(c, launch_block_rows(s->args, s->d_sblocks32, c->stream));
+        s->sb32_ready = true;
+    }
+    *rows = s->d_sblocks32;
+    return DG_OK;
+}
+
 // PCG iterations on S x = b (vectors in v, r = b - S x given) until S->done
 // or `limit` iterations.  Every `refresh` host checks (0: never) the
 // recurrence residual is replaced by the true FP64 residual b - S x (residual
@@ -182,7 +216,16 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
     }
     IP_CUDA(c, cudaMemcpyAsync(s->d_S, &h, sizeof(h), cudaMemcpyHostToDevice, c->stream));
     IP_CUDA(c, launch_pcg_init(s->args, v, pnet, pfa, c->stream));
-    const int CHECK = 16;
+    // small problems: cooperative launches of many iterations (in FP32 arithmetic
+    // as many as between two residual replacements)
+    const void* prows = nullptr;
+    if (persist_fits(s->args, v, fp32)) {
+        const int rcp = persist_rows(c, v, fp32, &prows);
+        if (rcp) return rcp;
+    }
+    const bool persist = prows != nullptr;
+    const int CHECK = persist ? (refresh > 0 ? 16 * refresh : 256) : 16;
+    if (persist && refresh > 0) refresh = 1;
     int checks = 0;
     *stop = 0;
     *iters = 0;
@@ -244,10 +287,15 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
     };
     while (h.it < limit) {
         const int batch = std::min(CHECK, limit - h.it);
-        IP_CUDA(c, launch_batch(h.it, batch));
+        if (persist)
+            IP_CUDA(c, launch_pcg_persistent(s->args, v, fp32, prows, s->d_corner, s->d_slots, &s->exchanges, h.it & 1,
+                                             batch, c->stream));
+        else
+            IP_CUDA(c, launch_batch(h.it, batch));
         IP_CUDA(c, cudaMemcpyAsync(&h, s->d_S, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
         IP_CUDA(c, cudaStreamSynchronize(c->stream));
         checks++;
+        if (h.gaveup) return ifail(c, DG_ERR_TIMEOUT, "PCG: a grid-wide barrier timed out");
         if (h.done == 2) break;
         if (v.zb && !v.mg && h.done == 0) {
             if (best_rr < 0 || h.rr < 0.5 * best_rr) {
@@ -359,7 +407,7 @@ extern "C" {
 static int build_blocks(dg_ctx* c) {
     IpdgState* s = c->ipdg;
     const IpdgArgs& a = s->args;
-    s->sb_ready = false;
+    s->sb_ready = s->sb32_ready = false;
     IP_CUDA(c, cudaMemsetAsync(s->d_status, 0, sizeof(int), c->stream));
     IP_CUDA(c, launch_ipdg_diag(a, s->d_blocks, c->stream));
     IP_CUDA(c, launch_invert_blocks(s->d_blocks, nullptr, a.K, a.Np, s->d_status, c->stream));

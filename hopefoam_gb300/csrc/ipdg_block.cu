@@ -43,12 +43,12 @@ constexpr int kRowCols = 4 * NP + 4;
 
 // blocks of one element, one CTA; D row-major to `diag` (when set), everything
 // to the grouped storage `sb` (when set)
-template <int N>
-__global__ void __launch_bounds__(128) ipdg_blocks_kernel(IpdgArgs a, double* __restrict__ diag, double* __restrict__ sb) {
+template <int N, typename T>
+__global__ void __launch_bounds__(128) ipdg_blocks_kernel(IpdgArgs a, double* __restrict__ diag, T* __restrict__ sb) {
     constexpr int Np = Dims<N>::Np, Nfp = Dims<N>::Nfp, Nfq = Dims<N>::Nfq, NF = 3 * Nfq, NB = 3 * N;
     using R = RowDims<Np>;
     const IpdgOps<double>& o = a.o64;
-    __shared__ double T[NF][Np];   // trace of the basis (zero off the face)
+    __shared__ double tr[NF][Np];  // trace of the basis (zero off the face)
     __shared__ double dm[NF][Np];  // own normal derivative
     __shared__ double up[NF][Np];  // neighbour's trace and derivative at the same points
     __shared__ double dp[NF][Np];
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(128) ipdg_blocks_kernel(IpdgArgs a, double* __
                 const int d = (p - face * N + NB) % NB;
                 return d <= N ? o.If[gq * Nfp + d] : 0.0;
             };
-            T[fg][p] = trace(f, g);
+            tr[fg][p] = trace(f, g);
             dm[fg][p] = fc[0] * o.Drf[(size_t)fg * Np + p] + fc[1] * o.Dsf[(size_t)fg * Np + p];
             double u = 0.0, d = 0.0;
             if (cn[f] >= 0) {
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128) ipdg_blocks_kernel(IpdgArgs a, double* __
         const double vrr = o.vc[(size_t)k * 3], vrs = o.vc[(size_t)k * 3 + 1], vss = o.vc[(size_t)k * 3 + 2];
         const double mc = a.mass_coef * a.J[k];
         const int grp = k / R::EB, e = k - grp * R::EB;
-        double* col0 = sb ? sb + (size_t)grp * kRowCols<Np> * R::EB * Np + e * Np : nullptr;
+        T* col0 = sb ? sb + (size_t)grp * kRowCols<Np> * R::EB * Np + e * Np : nullptr;
         constexpr size_t CS = (size_t)R::EB * Np;  // column stride
         for (int t = threadIdx.x; t < Np * Np; t += blockDim.x) {
             const int j = t / Np, i = t - j * Np;
@@ -97,13 +97,13 @@ __global__ void __launch_bounds__(128) ipdg_blocks_kernel(IpdgArgs a, double* __
 #pragma unroll
                 for (int g = 0; g < Nfq; g++) {
                     const int fg = f * Nfq + g;
-                    const double ti = wJ[fg] * T[fg][i], di = wJ[fg] * dm[fg][i];
-                    v += ti * (2.0 * h * tau2[f] * T[fg][j] - h * dm[fg][j]) - h * di * T[fg][j];
+                    const double ti = wJ[fg] * tr[fg][i], di = wJ[fg] * dm[fg][i];
+                    v += ti * (2.0 * h * tau2[f] * tr[fg][j] - h * dm[fg][j]) - h * di * tr[fg][j];
                     vo += 0.5 * di * up[fg][j] - ti * (tau2[f] * up[fg][j] + 0.5 * dp[fg][j]);
                 }
-                if (col0) col0[((size_t)(f + 1) * Np + j) * CS + i] = vo;
+                if (col0) col0[((size_t)(f + 1) * Np + j) * CS + i] = (T)vo;
             }
-            if (col0) col0[(size_t)j * CS + i] = v;
+            if (col0) col0[(size_t)j * CS + i] = (T)v;
             if (diag) diag[((size_t)k * Np + i) * Np + j] = v;
         }
         if (col0)
@@ -115,13 +115,13 @@ __global__ void __launch_bounds__(128) ipdg_blocks_kernel(IpdgArgs a, double* __
 #pragma unroll
                     for (int g = 0; g < Nfq; g++) {
                         const int fg = f * Nfq + g;
-                        s += wJ[fg] * (tau2[f] * T[fg][i] - 0.5 * dm[fg][i]);
+                        s += wJ[fg] * (tau2[f] * tr[fg][i] - 0.5 * dm[fg][i]);
                     }
                     // inside: row sums of the neighbour block; Dirichlet: twice the term, on u_0
-                    col0[((size_t)4 * Np + f) * CS + i] = cn[f] >= 0 ? -s : 0.0;
+                    col0[((size_t)4 * Np + f) * CS + i] = cn[f] >= 0 ? (T)-s : (T)0;
                     if (cn[f] < 0) wb += 2.0 * s;
                 }
-                col0[((size_t)4 * Np + 3) * CS + i] = wb;
+                col0[((size_t)4 * Np + 3) * CS + i] = (T)wb;
             }
         __syncthreads();
     }
@@ -225,29 +225,31 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS, 3) block_apply_kernel(Ip
     }
 }
 
-template <int N>
-cudaError_t blocks_n(const IpdgArgs& a, double* diag, double* sb, cudaStream_t s) {
-    ipdg_blocks_kernel<N><<<std::min(a.K, 16 * a.sms), 128, 0, s>>>(a, diag, sb);
+template <int N, typename T>
+cudaError_t blocks_n(const IpdgArgs& a, double* diag, T* sb, cudaStream_t s) {
+    ipdg_blocks_kernel<N, T><<<std::min(a.K, 16 * a.sms), 128, 0, s>>>(a, diag, sb);
     return cudaGetLastError();
 }
 
-cudaError_t blocks_dispatch(const IpdgArgs& a, double* diag, double* sb, cudaStream_t s) {
+template <typename T>
+cudaError_t blocks_dispatch(const IpdgArgs& a, double* diag, T* sb, cudaStream_t s) {
     switch (a.N) {
-        case 1: return blocks_n<1>(a, diag, sb, s);
-        case 2: return blocks_n<2>(a, diag, sb, s);
-        case 3: return blocks_n<3>(a, diag, sb, s);
-        case 4: return blocks_n<4>(a, diag, sb, s);
-        case 5: return blocks_n<5>(a, diag, sb, s);
-        case 6: return blocks_n<6>(a, diag, sb, s);
-        case 7: return blocks_n<7>(a, diag, sb, s);
+        case 1: return blocks_n<1, T>(a, diag, sb, s);
+        case 2: return blocks_n<2, T>(a, diag, sb, s);
+        case 3: return blocks_n<3, T>(a, diag, sb, s);
+        case 4: return blocks_n<4, T>(a, diag, sb, s);
+        case 5: return blocks_n<5, T>(a, diag, sb, s);
+        case 6: return blocks_n<6, T>(a, diag, sb, s);
+        case 7: return blocks_n<7, T>(a, diag, sb, s);
         default: return cudaErrorInvalidValue;
     }
 }
 
 }  // namespace
 
-cudaError_t launch_ipdg_diag(const IpdgArgs& a, double* blocks, cudaStream_t s) { return blocks_dispatch(a, blocks, nullptr, s); }
-cudaError_t launch_block_rows(const IpdgArgs& a, double* sblocks, cudaStream_t s) { return blocks_dispatch(a, nullptr, sblocks, s); }
+cudaError_t launch_ipdg_diag(const IpdgArgs& a, double* blocks, cudaStream_t s) { return blocks_dispatch<double>(a, blocks, nullptr, s); }
+cudaError_t launch_block_rows(const IpdgArgs& a, double* sblocks, cudaStream_t s) { return blocks_dispatch<double>(a, nullptr, sblocks, s); }
+cudaError_t launch_block_rows(const IpdgArgs& a, float* sblocks, cudaStream_t s) { return blocks_dispatch<float>(a, nullptr, sblocks, s); }
 
 size_t block_rows_size(int K, int Np) {
     auto n = [&](auto tag) {

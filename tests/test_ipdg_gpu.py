@@ -163,3 +163,29 @@ def test_fp64_iterations_on_block_rows(gpu_lib, N, n, mass):
         p, rz = z + (r @ z) / rz * p, r @ z
     assert rel_l2(x, xr) < 1e-10
     ps.ctx.close()
+
+
+@pytest.mark.parametrize("N,n,pc,precision", [
+    (1, 4, "BLOCK_JACOBI", 0), (1, 400, "MULTILEVEL", 0), (1, 400, "BLOCK_JACOBI", 1),  # one block; a few
+    (2, 4, "MULTILEVEL", 1), (2, 400, "MULTILEVEL", 0), (3, 400, "BLOCK_JACOBI", 0), (3, 400, "MULTILEVEL", 1),
+    (3, 1700, "MULTILEVEL", 0), (3, 1800, "MULTILEVEL", 0),  # just below what one launch holds, and above
+    (4, 100, "MULTILEVEL", 0), (4, 2300, "BLOCK_JACOBI", 1), (4, 2400, "BLOCK_JACOBI", 1),  # likewise
+    (5, 400, "MULTILEVEL", 1), (5, 4, "BLOCK_JACOBI", 1), (5, 100, "BLOCK_JACOBI", 0)])
+def test_iterations_of_small_problems(gpu_lib, N, n, pc, precision):
+    """Solves whose iterations one launch holds, and their neighbours above the limit: every order, ragged last warps
+    and blocks, both arithmetic types and preconditioners.  The solve stops on ||b - S x|| <= 1e-10 ||b|| with its own
+    operator; on the oracle's assembled blocks the same residual differs by round-off of S x, below 1e-10 ||b|| at these
+    conditions (1e-16 * |S| |x| / ||b||, condition below 1e6): 2e-10.  A second solve gives the same bits."""
+    from hopefoam_gb300 import _lib as L
+    from hopefoam_gb300.mesh import delaunay_square
+
+    m = delaunay_square(n, seed=3)
+    ps, orc, diag, off = _setup(m, N)
+    b = np.random.default_rng(N).standard_normal(m.K * ps.Np)
+    kw = dict(rtol=1e-10, maxit=20000, pc=getattr(L, "DG_PC_" + pc), precision=precision)
+    x, st = ps.solve(b, **kw)
+    r = b + orc.blk_apply(diag, off, x)
+    assert st["rel_residual"] <= 1e-10 and np.linalg.norm(r) < 2e-10 * np.linalg.norm(b)
+    x2, st2 = ps.solve(b, **kw)
+    assert st2["iterations"] == st["iterations"] and np.array_equal(x, x2)
+    ps.ctx.close()
