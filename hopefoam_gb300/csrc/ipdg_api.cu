@@ -491,25 +491,36 @@ static int mg_setup(dg_ctx* c) {
     up((double**)&m.lam, b.lam);
     up((int**)&m.vptr, b.vptr);
     up((int**)&m.vinc, b.vinc);
-    up((double**)&m.V, b.V);
     size_t work = 0;
+    auto up_csr = [&](const int** ptr, const int** col, const double** val, const MgCsr& h) {
+        up((int**)ptr, h.ptr);
+        up((int**)col, h.col);
+        up((double**)val, h.val);
+    };
+    // the dense levels, from the one the cycle ends on to the coarsest
+    const int nd = (int)b.levels.size() - b.nd;
+    MgDenseLevel dense[kMgMaxLevels];
+    int dn[kMgMaxLevels];
+    for (int l = 0; l < nd; l++) {
+        const MgBuild::Level& L = b.levels[b.nd + l];
+        dense[l].n = dn[l] = L.n;
+        if (l + 1 < nd) up_csr(&dense[l].tptr, &dense[l].tcol, &dense[l].tval, L.Bt);
+        up_csr(&dense[l].mptr, &dense[l].mcol, &dense[l].mval, l + 1 < nd ? L.M : L.A);
+    }
+    const std::vector<int> zero(1, 0);
+    int* d_status = nullptr;
+    up(&d_status, zero);
     for (int l = 0; l < m.nl; l++) {
         const MgBuild::Level& L = b.levels[l];
         MgLevel& d = m.lv[l];
         d.n = L.n;
         work += 3 * ((size_t)L.n + 31) / 32 * 32;
         if (l + 1 == m.nl) continue;
-        up((int**)&d.bptr, L.B.ptr);
-        up((int**)&d.bcol, L.B.col);
-        up((double**)&d.bval, L.B.val);
-        up((int**)&d.tptr, L.Bt.ptr);
-        up((int**)&d.tcol, L.Bt.col);
-        up((double**)&d.tval, L.Bt.val);
-        up((int**)&d.mptr, L.M.ptr);
-        up((int**)&d.mcol, L.M.col);
-        up((double**)&d.mval, L.M.val);
+        up_csr(&d.bptr, &d.bcol, &d.bval, L.B);
+        up_csr(&d.tptr, &d.tcol, &d.tval, L.Bt);
+        up_csr(&d.mptr, &d.mcol, &d.mval, L.M);
     }
-    const size_t need = blob.size() + (work + 96 * m.nl) * sizeof(double);
+    const size_t need = blob.size() + (work + 96 * m.nl + mg_dense_work(dn, nd)) * sizeof(double);
     if (need > s->mg_bytes) {
         if (s->d_mg) cudaFree(s->d_mg);
         s->d_mg = nullptr;
@@ -530,6 +541,16 @@ static int mg_setup(dg_ctx* c) {
                 *p = w;
                 w += ((size_t)m.lv[l].n + 31) / 32 * 32;
             }
+        m.V = w;
+        int bad = 0;
+        if (!rc && (launch_mg_dense(dense, nd, w, d_status, c->stream) != cudaSuccess ||
+                    cudaMemcpyAsync(&bad, d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
+                    cudaStreamSynchronize(c->stream) != cudaSuccess))
+            return ifail(c, DG_ERR_CUDA, "multilevel preconditioner: dense cycle operator");
+        if (bad) {
+            s->mg_err = "multilevel preconditioner: coarse operator is not positive definite";
+            return ifail(c, DG_ERR_UNSUPPORTED, s->mg_err);
+        }
     }
     if (!s->d_zb) rc |= ialloc(c, s, &s->d_zb, (size_t)c->K * c->Np);
     if (rc) return ifail(c, DG_ERR_NOMEM, "multilevel preconditioner: device allocation failed");
@@ -793,15 +814,15 @@ static int pcg_solve_impl(dg_ctx* c, const double* b_host, double* x_host, doubl
     if (learned && !c->ipdg->lpc_ready) return ifail(c, DG_ERR_ARG, "dg_lpc_setup not called");
     if (pc == DG_PC_LEARNED_MULTILEVEL && c->ipdg->lpc_form != DG_LPC_SCHWARZ)
         return ifail(c, DG_ERR_ARG, "learned + multilevel needs the linear learned Schwarz form");
+    if (precision != DG_PREC_FP64 && precision != DG_PREC_SPLIT) return ifail(c, DG_ERR_ARG, "unknown precision");
+    const BlockRows rows(c, precision == DG_PREC_FP64);  // formed while the host builds the levels
+    if (rows.rc) return rows.rc;
     if (mgm && !c->ipdg->mg_ready) {
         const int rcm = mg_setup(c);
         if (rcm) return rcm;
     }
-    if (precision != DG_PREC_FP64 && precision != DG_PREC_SPLIT) return ifail(c, DG_ERR_ARG, "unknown precision");
     IpdgState* s = c->ipdg;
     const size_t n = (size_t)c->K * c->Np;
-    const BlockRows rows(c, precision == DG_PREC_FP64);
-    if (rows.rc) return rows.rc;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -935,13 +956,13 @@ int ipdg_solve_device(dg_ctx* c, const double* b_dev, double* x_dev, double rtol
     if (!c->ipdg || !c->ipdg->ready) return ifail(c, DG_ERR_ARG, "dg_ipdg_setup not called");
     IpdgState* s = c->ipdg;
     const bool mgm = pc == DG_PC_MULTILEVEL;
+    const BlockRows rows(c, precision == DG_PREC_FP64);  // formed while the host builds the levels
+    if (rows.rc) return rows.rc;
     if (mgm && !s->mg_ready) {
         const int rcm = mg_setup(c);
         if (rcm) return rcm;
     }
     const size_t n = (size_t)c->K * c->Np;
-    const BlockRows rows(c, precision == DG_PREC_FP64);
-    if (rows.rc) return rows.rc;
     IP_CUDA(c, cudaMemcpyAsync(s->d_b, b_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     IP_CUDA(c, cudaMemcpyAsync(s->d_x, x_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     double bb = 0;

@@ -67,13 +67,12 @@ struct MgBuild {
         MgCsr A;
         std::vector<double> dinv;  // omega / diag A
         std::vector<int> agg;      // coarse index of each unknown (empty on the coarsest level)
-        MgCsr B, Bt, M;
+        MgCsr B, Bt, M;            // B of the sparse levels only
     };
     std::vector<int> vptr, vinc;
     std::vector<double> lam;
     std::vector<Level> levels;  // levels[0]: P1 on the vertices
-    int nd = 0;                 // levels kept: levels[nd] is the dense one
-    std::vector<double> V;      // its cycle operator, levels[nd].n^2
+    int nd = 0;                 // levels[nd] is held as its dense cycle operator, those below go into it
 };
 
 // Builds the levels; "" on success.  etov: [K][3] vertex ids, geo: [K][4]
@@ -84,6 +83,21 @@ struct MgBuild {
 std::string mg_build(int K, int N, int Np, const int* etov, const double* geo, const int* conn,
                      const std::vector<double>& fc, const std::vector<int>& btype, double mass_coef,
                      const dgb::RefOps& ops, MgBuild& out);
+
+// The dense cycle operator of levels[nd] from the levels nd .. coarsest
+// (count of them, lv[0] = levels[nd]): B^T and M of each in CSR, for the coarsest
+// its operator A in place of M.  work holds mg_dense_work doubles (sizes n[0..count-1]);
+// the n[0]^2 result is at its start.  *status (0 before) becomes 1 where the
+// coarsest operator is not positive definite.
+struct MgDenseLevel {
+    int n = 0;
+    const int *tptr = nullptr, *tcol = nullptr;
+    const double* tval = nullptr;
+    const int *mptr = nullptr, *mcol = nullptr;
+    const double* mval = nullptr;
+};
+size_t mg_dense_work(const int* n, int count);
+cudaError_t launch_mg_dense(const MgDenseLevel* lv, int count, double* work, int* status, cudaStream_t s);
 
 // z = zb + P V(P^T r) with r.z reduced like the learned preconditioner's
 // collect step (mode: 1 init -> S->rz, 2 refresh -> S->rz, 3 iteration ->

@@ -73,10 +73,11 @@ def _cycle(A, r, omega=0.6, coarsest=500):
     return x + d * (r - A @ x)
 
 
-@pytest.mark.parametrize("n_interior", [300, 1200, 3000, 12000])
+@pytest.mark.parametrize("n_interior", [4, 60, 300, 450, 1200, 3000, 12000])
 def test_one_application_against_its_definition(gpu_lib, n_interior):
     """z = B r + P V(P^T r) of the first iteration (its solution is a multiple of z) against the cycle written out
-    level by level: only the dense inverse; the cycle as one dense matrix; one and two sparse levels above it.
+    level by level: only the dense inverse (20, 96 and some 300 unknowns: part of a block, whole blocks, a remainder);
+    the cycle as one dense matrix; one and two sparse levels above it.
     Tolerance: round-off (1e-15) times the condition number of the P1 operator (about 1e5 at 12000 vertices), with a
     factor of 100 for the differently formed coarse operators."""
     import scipy.sparse as sp
