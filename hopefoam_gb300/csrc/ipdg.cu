@@ -699,7 +699,7 @@ __device__ __forceinline__ double bj_rowg(const PT* __restrict__ P, const RT* rs
 
 // mode 0 (init):    z = P r; S->rz = r.z, S->rr = r.r, beta = 0 (first p = z)
 // mode 1 (refresh): the same, beta kept (residual replacement)
-// Learned mode (v.zb): zb = P r and S->rr only; the learned kernel forms z, r.z.
+// Learned and multilevel modes (v.zb): zb = P r, S->rr and (multilevel) S->rzb; the kernels after it form z and r.z.
 template <int NP>
 __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_init_kernel(PcgVecs v, int K, int mode) {
     constexpr int EB = RowDims<NP>::EB;
@@ -741,10 +741,8 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_init_kernel(PcgVecs 
             const float dzi = mirror_offset(v.dz != nullptr, v.P64 != nullptr, z, zf, lb);
             if (act) {
                 if (v.zb) v.zb[idx] = z;
-                else {
-                    v.z[idx] = z;
-                    rz += ri * z;
-                }
+                else v.z[idx] = z;
+                if (!v.zb || v.mg) rz += ri * z;
                 if (v.r32) v.r32[idx] = r32;
                 if (v.dz) v.dz[idx] = dzi;  // learned mode: the mirror of P r
                 rr += ri * ri;
@@ -768,10 +766,8 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_init_kernel(PcgVecs 
             if (act) {
                 z = v.P64 ? bj_rowg<NP>(v.P64, rs[e], grp) : bj_rowg<NP>(v.P32, rs32[e], grp);
                 if (v.zb) v.zb[idx] = z;
-                else {
-                    v.z[idx] = z;
-                    rz += ri * z;
-                }
+                else v.z[idx] = z;
+                if (!v.zb || v.mg) rz += ri * z;
                 if (i == 0) zs0[e] = z;
                 if (v.r32) v.r32[idx] = rs32[e][i];
                 rr += ri * ri;
@@ -787,6 +783,7 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_init_kernel(PcgVecs 
     if (grid_sum<2>(val, v.part, gridDim.x, &v.S->counter, tot) && threadIdx.x == 0) {
         v.S->rr = tot[1];
         if (!v.zb) v.S->rz = tot[0];
+        else v.S->rzb = tot[0];
         if (mode == 0) {
             v.S->beta = 0.0;
             if (tot[1] <= v.S->tol2) v.S->done = 1;
@@ -844,7 +841,7 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_update_kernel(PcgVec
     int e, i;
     row_of<NP>(e, i);
     const int ngroups = (K + EB - 1) / EB;
-    double rz = 0, rr = 0, rzo = 0;
+    double rz = 0, rr = 0;
     if constexpr (RowDims<NP>::WA) {
         // no CTA barrier: the element's residual reaches its rows by shuffles
         const int lb = (threadIdx.x & 31) - i;
@@ -887,14 +884,12 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_update_kernel(PcgVec
             if (act) {
                 rr += ri * ri;
                 if (v.r32) v.r32[idx] = r32;
-                if (v.zb) {
-                    v.zb[idx] = z;  // the learned kernel forms z and finishes the iteration
-                } else {
-                    // block Jacobi is a fixed linear preconditioner: the standard
-                    // (Fletcher-Reeves) beta needs no r.z_old
-                    v.z[idx] = z;
-                    rz += ri * z;
-                }
+                // block Jacobi is a fixed linear preconditioner: the standard
+                // (Fletcher-Reeves) beta needs no r.z_old; with zb the learned kernel
+                // or the coarse-space correction forms z and finishes the iteration
+                if (v.zb) v.zb[idx] = z;
+                else v.z[idx] = z;
+                if (!v.zb || v.mg) rz += ri * z;
                 if (v.dz) v.dz[idx] = dzi;  // learned mode: the mirror of P r
             }
         }
@@ -922,10 +917,8 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_update_kernel(PcgVec
                 rr += ri * ri;
                 if (v.r32) v.r32[idx] = rs32[e][i];
                 if (v.zb) v.zb[idx] = z;
-                else {
-                    v.z[idx] = z;
-                    rz += ri * z;
-                }
+                else v.z[idx] = z;
+                if (!v.zb || v.mg) rz += ri * z;
                 if (i == 0) zs0[e] = z;
             }
             if (v.dz) {
@@ -935,10 +928,14 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_update_kernel(PcgVec
             __syncthreads();
         }
     }
-    double val[3] = {rz, rr, rzo}, tot[3];
-    if (grid_sum<3>(val, v.part, gridDim.x, &v.S->counter, tot) && threadIdx.x == 0) {
-        if (v.zb) v.S->rr = tot[1];
-        else pcg_finish(v.S, tot[0], tot[2], tot[1]);
+    double val[2] = {rz, rr}, tot[2];
+    if (grid_sum<2>(val, v.part, gridDim.x, &v.S->counter, tot) && threadIdx.x == 0) {
+        if (v.zb) {
+            v.S->rr = tot[1];
+            v.S->rzb = tot[0];
+        } else {
+            pcg_finish(v.S, tot[0], 0.0, tot[1]);
+        }
     }
 }
 
@@ -1116,9 +1113,9 @@ static cudaError_t pcg_precondition(const IpdgArgs& a, const PcgVecs& v, const L
         if (e == cudaSuccess)
             e = launch_schwarz_collect(*lpc->sw, v.zb, lpc->U, nullptr, v.zl, v.dz, LPC_APPLY, v.S, v.part, s);
         if (e != cudaSuccess) return e;
-        return launch_mg_correction(*v.mg, v.r, v.zl, v.z, v.dz, lmode, v.S, v.part, v.nmax, s);
+        return launch_mg_correction(*v.mg, v.r, v.zl, v.z, v.dz, lmode, false, v.S, v.part, v.nmax, s);
     }
-    if (v.mg) return launch_mg_correction(*v.mg, v.r, v.zb, v.z, v.dz, lmode, v.S, v.part, v.nmax, s);
+    if (v.mg) return launch_mg_correction(*v.mg, v.r, v.zb, v.z, v.dz, lmode, true, v.S, v.part, v.nmax, s);
     if (lpc->sw) {
         e = launch_schwarz_local(*lpc->sw, v.r, v.r32, lpc->U, nullptr, s);
         if (e != cudaSuccess) return e;
@@ -1150,9 +1147,9 @@ cudaError_t launch_pcg_iteration(const IpdgArgs& a, const PcgVecs& v, bool fp32,
         if (e == cudaSuccess)
             e = launch_schwarz_collect(*lpc->sw, v.zb, lpc->U, nullptr, v.zl, v.dz, LPC_APPLY, v.S, v.part, s);
         if (e == cudaSuccess)
-            e = launch_mg_correction(*v.mg, v.r, v.zl, v.z, v.dz, LPC_PCG_ITERATION, v.S, v.part, v.nmax, s);
+            e = launch_mg_correction(*v.mg, v.r, v.zl, v.z, v.dz, LPC_PCG_ITERATION, false, v.S, v.part, v.nmax, s);
     } else if (v.zb && v.mg) {
-        e = launch_mg_correction(*v.mg, v.r, v.zb, v.z, v.dz, LPC_PCG_ITERATION, v.S, v.part, v.nmax, s);
+        e = launch_mg_correction(*v.mg, v.r, v.zb, v.z, v.dz, LPC_PCG_ITERATION, true, v.S, v.part, v.nmax, s);
     } else if (v.zb) {
         if (lpc->sw) {
             e = launch_schwarz_local(*lpc->sw, v.r, v.r32, lpc->U, &v.S->done, s);

@@ -77,6 +77,7 @@ struct PcgScalars {
     double alpha;   // rz / pap
     double beta;    // next p = z + beta p (0: restart from z)
     double rr;      // recurrence residual r.r
+    double rzb;     // multilevel mode: r.zb, before the coarse-space correction
     int done;       // 1 converged, 2 breakdown / non-finite
     int it;         // iterations taken
     unsigned int counter;  // arrival counter of the grid-wide sums

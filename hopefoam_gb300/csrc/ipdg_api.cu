@@ -1064,7 +1064,7 @@ int lpc_forward_vec(dg_ctx* c, const double* r, bool with_bj_loss) {
         // the reference loss: block Jacobi, with the coarse-space correction when training under it
         const double* zref = s->d_zb;
         if (s->lpc_coarse) {
-            IP_CUDA(c, launch_mg_correction(s->mg, r, s->d_zb, s->d_zt, nullptr, LPC_PCG_INIT, s->d_S, s->d_ppart,
+            IP_CUDA(c, launch_mg_correction(s->mg, r, s->d_zb, s->d_zt, nullptr, LPC_PCG_INIT, false, s->d_S, s->d_ppart,
                                             s->nmax, c->stream));
             zref = s->d_zt;
         }
@@ -1077,7 +1077,7 @@ int lpc_forward_vec(dg_ctx* c, const double* r, bool with_bj_loss) {
         IP_CUDA(c, launch_schwarz_collect(s->sw, s->d_zb, s->d_U, nullptr, s->d_zt, nullptr, LPC_APPLY, nullptr,
                                           nullptr, c->stream));
         if (s->lpc_coarse)  // z = learned local stage + P V(P^T r), in place (the preconditioner it is trained for)
-            IP_CUDA(c, launch_mg_correction(s->mg, r, s->d_zt, s->d_zt, nullptr, LPC_PCG_INIT, s->d_S, s->d_ppart,
+            IP_CUDA(c, launch_mg_correction(s->mg, r, s->d_zt, s->d_zt, nullptr, LPC_PCG_INIT, false, s->d_S, s->d_ppart,
                                             s->nmax, c->stream));
     } else {
         IP_CUDA(c, launch_lpc_features(fa, s->d_X, s->d_sc, c->stream));

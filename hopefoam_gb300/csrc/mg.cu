@@ -8,6 +8,8 @@
 #include <vector>
 
 #include "euler_flux.cuh"
+#include "f64split.cuh"
+#include "ipdg_rows.cuh"
 #include "mg.hpp"
 #include "pcg_reduce.cuh"
 
@@ -457,82 +459,142 @@ __global__ void __launch_bounds__(256) mg_down_kernel(MgLevel a, int nc, int bbl
     }
 }
 
-// x = w + B^T x_c
-__global__ void __launch_bounds__(256) mg_up_kernel(MgLevel a, const double* __restrict__ xc, const int* __restrict__ done) {
-    if (done && *done) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, row = t / kUpLanes, l = t % kUpLanes;
-    const double s = row_dot<kUpLanes>(a.tptr, a.tcol, a.tval, xc, row, row < a.n, l);
-    if (row < a.n && l == 0) a.x[row] = a.w[row] + s;
+// Where the level on the vertices comes out of the cycle, r1.x1 with r1 = P^T r
+// and x1 its result is what the correction adds to r.z: the sum over vertices
+// replaces one over all rows, which would read r again.  Finishes the iteration
+// or leaves rz, from S->rzb = r.zb.
+__device__ __forceinline__ void finish_rz(double dot, int mode, PcgScalars* S, double* part) {
+    double val[1] = {dot}, tot[1];
+    if (grid_sum<1>(val, part, gridDim.x, &S->counter, tot) && threadIdx.x == 0) {
+        const double rz = S->rzb + tot[0];
+        if (mode == 3) pcg_finish(S, rz, 0.0, S->rr);
+        else S->rz = rz;
+    }
 }
 
-// x = V r, one warp per row, r staged in shared memory
+// x = w + B^T x_c; DOT: and x.r
+template <bool DOT>
+__global__ void __launch_bounds__(256) mg_up_kernel(MgLevel a, const double* __restrict__ xc, const int* __restrict__ done,
+                                                    int mode, PcgScalars* S, double* part) {
+    if (done && *done) return;
+    double dot = 0;
+    for (int row0 = blockIdx.x * (256 / kUpLanes); row0 < a.n; row0 += gridDim.x * (256 / kUpLanes)) {
+        const int row = row0 + threadIdx.x / kUpLanes, l = threadIdx.x % kUpLanes;
+        const double s = row_dot<kUpLanes>(a.tptr, a.tcol, a.tval, xc, row, row < a.n, l);
+        if (row < a.n && l == 0) {
+            const double x = a.w[row] + s;
+            a.x[row] = x;
+            if (DOT) dot += x * a.r[row];
+        }
+    }
+    if (DOT) finish_rz(dot, mode, S, part);
+}
+
+// x = V r, one warp per row, r staged in shared memory; DOT: and x.r
+template <bool DOT>
 __global__ void __launch_bounds__(256) mg_dense_kernel(int n, const double* __restrict__ V, const double* __restrict__ r,
-                                                       double* __restrict__ x, const int* __restrict__ done) {
+                                                       double* __restrict__ x, const int* __restrict__ done, int mode,
+                                                       PcgScalars* S, double* part) {
     __shared__ double rs[kDense];
     if (done && *done) return;
     for (int j = threadIdx.x; j < n; j += blockDim.x) rs[j] = r[j];
     __syncthreads();
     const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const double* v = V + (size_t)row * n;
-    double s0 = 0, s1 = 0;
-    int j = lane;
+    double dot = 0;
+    if (row < n) {
+        const double* v = V + (size_t)row * n;
+        double s0 = 0, s1 = 0;
+        int j = lane;
 #pragma unroll 4
-    for (; j + 32 < n; j += 64) {
-        s0 += v[j] * rs[j];
-        s1 += v[j + 32] * rs[j + 32];
-    }
-    if (j < n) s0 += v[j] * rs[j];
-    s0 += s1;
+        for (; j + 32 < n; j += 64) {
+            s0 += v[j] * rs[j];
+            s1 += v[j + 32] * rs[j + 32];
+        }
+        if (j < n) s0 += v[j] * rs[j];
+        s0 += s1;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    if (lane == 0) x[row] = s0;
+        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        if (lane == 0) {
+            x[row] = s0;
+            dot = s0 * rs[row];
+        }
+    }
+    if (DOT) finish_rz(dot, mode, S, part);
 }
 
-// z = zb + P x1; r.z; dz mirror; finish like the learned preconditioner's collect
-__global__ void mg_collect_kernel(MgLevels m, const double* __restrict__ zb, const double* __restrict__ x1,
-                                  const double* __restrict__ r, double* __restrict__ z, float* __restrict__ dz,
-                                  int mode, PcgScalars* S, double* part) {
-    __shared__ double c0s[256];
+// z = zb + P x1, and dz from the mirror of zb to that of z: z - z0 = (zb - zb0) +
+// (c - c0).  Bound by the FP64 pipe: three operations for c, one each for z and
+// c - c0, which is rounded to FP32 by integer operations.  DOT (the learned
+// forms, whose r.zb nobody has summed): r.z as well, finishing like the learned
+// preconditioner's collect.  K = 101,246, N = 4: 34 us with the sum over
+// all rows here, 22 us without (and 8 us more in the kernel that sums the vertices).
+template <int NP, bool DOT>
+__global__ void __launch_bounds__(RowDims<NP>::THREADS) mg_collect_kernel(MgLevels m, const double* __restrict__ zb,
+                                                                          const double* __restrict__ x1,
+                                                                          const double* __restrict__ r, double* __restrict__ z,
+                                                                          float* __restrict__ dz, int mode, PcgScalars* S,
+                                                                          double* part) {
+    using R = RowDims<NP>;
     if (mode == 3 && S->done) return;
-    const int Np = m.Np, EB = 256 / Np;
-    const int e = threadIdx.x / Np, q = threadIdx.x - e * Np;
-    const int ngroups = (m.K + EB - 1) / EB;
+    int e, i;
+    row_of<NP>(e, i);
+    const bool lane_ok = e < R::EB;
+    const double l0 = m.lam[3 * i], l1 = m.lam[3 * i + 1], l2 = m.lam[3 * i + 2];
+    __shared__ double c0s[R::WA ? 1 : R::EB];
     double rz = 0;
-    for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
-        const int k = grp * EB + e;
-        const bool act = e < EB && k < m.K;
-        double c = 0;
+    for (int grp = blockIdx.x; grp < row_groups<NP>(m.K); grp += gridDim.x) {
+        const int k = grp * R::EB + e;
+        const bool act = lane_ok && k < m.K;
+        const size_t t = (size_t)k * NP + i;
+        double c = 0, zv = 0;
+        float d = 0.f;
         if (act) {
-            const size_t t = (size_t)k * Np + q;
-            c = m.lam[q * 3 + 0] * x1[m.etov[3 * (size_t)k]] + m.lam[q * 3 + 1] * x1[m.etov[3 * (size_t)k + 1]] +
-                m.lam[q * 3 + 2] * x1[m.etov[3 * (size_t)k + 2]];
-            const double zv = zb[t] + c;
+            const int* ev = m.etov + 3 * (size_t)k;
+            zv = zb[t];
+            if (dz) d = dz[t];
+            c = l0 * x1[ev[0]] + l1 * x1[ev[1]] + l2 * x1[ev[2]];
+            zv += c;
             z[t] = zv;
-            rz += r[t] * zv;
-            if (q == 0) c0s[e] = c;
+            if (DOT) rz += r[t] * zv;
         }
         if (dz) {
-            // dz enters as the offset mirror of zb: z - z0 = (zb - zb0) + (c - c0)
-            __syncthreads();
-            if (act) {
-                const size_t t = (size_t)k * Np + q;
-                dz[t] = dz[t] + (float)(c - c0s[e]);
+            double c0;
+            if constexpr (R::WA) {
+                c0 = __shfl_sync(0xffffffffu, c, (threadIdx.x & 31) - i);
+            } else {
+                __syncthreads();
+                if (act && i == 0) c0s[e] = c;
+                __syncthreads();
+                c0 = act ? c0s[e] : 0.0;
             }
-            __syncthreads();
+            if (act) dz[t] = d + f64s::minus_f32(c - c0, 0.f);
         }
     }
-    double val[1] = {rz}, tot[1];
-    if (grid_sum<1>(val, part, gridDim.x, &S->counter, tot) && threadIdx.x == 0) {
-        if (mode == 3) pcg_finish(S, tot[0], 0.0, S->rr);
-        else S->rz = tot[0];
+    if (DOT) {
+        double val[1] = {rz}, tot[1];
+        if (grid_sum<1>(val, part, gridDim.x, &S->counter, tot) && threadIdx.x == 0) {
+            if (mode == 3) pcg_finish(S, tot[0], 0.0, S->rr);
+            else S->rz = tot[0];
+        }
     }
+}
+
+template <int NP>
+static cudaError_t launch_collect(const MgLevels& m, const double* zb, const double* r, double* z, float* dz, int mode,
+                                  bool zb_summed, PcgScalars* S, double* part, int grid, cudaStream_t s) {
+    const int groups = row_groups<NP>(m.K);
+    if (zb_summed)
+        mg_collect_kernel<NP, false><<<groups, RowDims<NP>::THREADS, 0, s>>>(m, zb, m.lv[0].x, r, z, dz, mode, S, part);
+    else
+        mg_collect_kernel<NP, true><<<std::min(groups, grid), RowDims<NP>::THREADS, 0, s>>>(m, zb, m.lv[0].x, r, z, dz, mode,
+                                                                                           S, part);
+    return cudaGetLastError();
 }
 
 static unsigned nb256(int n) { return (unsigned)((n + 255) / 256); }
 
-cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const double* zb, double* z, float* dz,
-                                 int mode, PcgScalars* S, double* part, int grid, cudaStream_t s) {
+cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const double* zb, double* z, float* dz, int mode,
+                                 bool zb_summed, PcgScalars* S, double* part, int grid, cudaStream_t s) {
     const int L = m.nl;
     const int* done = mode == 3 ? &S->done : nullptr;  // a stopped iteration leaves every vector as it is
     mg_restrict_dg_kernel<<<nb256(8 * m.lv[0].n), 256, 0, s>>>(m, r, m.lv[0].r, done);
@@ -542,12 +604,27 @@ cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const doubl
                                                                             done);
     }
     const MgLevel& c = m.lv[L - 1];
-    mg_dense_kernel<<<(c.n + 7) / 8, 256, 0, s>>>(c.n, m.V, c.r, c.x, done);
-    for (int l = L - 2; l >= 0; l--) mg_up_kernel<<<nb256(kUpLanes * m.lv[l].n), 256, 0, s>>>(m.lv[l], m.lv[l + 1].x, done);
-    const int EB = 256 / m.Np;
-    const int ngroups = (m.K + EB - 1) / EB;
-    mg_collect_kernel<<<std::min(ngroups, grid), 256, 0, s>>>(m, zb, m.lv[0].x, r, z, dz, mode, S, part);
-    return cudaGetLastError();
+    if (L == 1 && zb_summed)
+        mg_dense_kernel<true><<<(c.n + 7) / 8, 256, 0, s>>>(c.n, m.V, c.r, c.x, done, mode, S, part);
+    else
+        mg_dense_kernel<false><<<(c.n + 7) / 8, 256, 0, s>>>(c.n, m.V, c.r, c.x, done, mode, S, part);
+    for (int l = L - 2; l >= 0; l--) {
+        const int blocks = (int)nb256(kUpLanes * m.lv[l].n);
+        if (l == 0 && zb_summed)
+            mg_up_kernel<true><<<std::min(blocks, grid / 2), 256, 0, s>>>(m.lv[l], m.lv[l + 1].x, done, mode, S, part);
+        else
+            mg_up_kernel<false><<<blocks, 256, 0, s>>>(m.lv[l], m.lv[l + 1].x, done, mode, S, part);
+    }
+    switch (m.Np) {
+        case 3: return launch_collect<3>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
+        case 6: return launch_collect<6>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
+        case 10: return launch_collect<10>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
+        case 15: return launch_collect<15>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
+        case 21: return launch_collect<21>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
+        case 28: return launch_collect<28>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
+        case 36: return launch_collect<36>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace dgk

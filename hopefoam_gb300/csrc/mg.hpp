@@ -99,10 +99,11 @@ struct MgDenseLevel {
 size_t mg_dense_work(const int* n, int count);
 cudaError_t launch_mg_dense(const MgDenseLevel* lv, int count, double* work, int* status, cudaStream_t s);
 
-// z = zb + P V(P^T r) with r.z reduced like the learned preconditioner's
-// collect step (mode: 1 init -> S->rz, 2 refresh -> S->rz, 3 iteration ->
-// pcg_finish); dz (mixed precision) is completed as an offset mirror
-cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const double* zb, double* z, float* dz,
-                                 int mode, PcgScalars* S, double* part, int grid, cudaStream_t s);
+// z = zb + P V(P^T r) and r.z (mode: 1 init -> S->rz, 2 refresh -> S->rz, 3
+// iteration -> pcg_finish); dz (mixed precision) is completed as an offset
+// mirror.  zb_summed: S->rzb holds r.zb, so that r.z = rzb + (P^T r).V(P^T r)
+// comes out of the cycle; otherwise r.z is summed over the rows.
+cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const double* zb, double* z, float* dz, int mode,
+                                 bool zb_summed, PcgScalars* S, double* part, int grid, cudaStream_t s);
 
 }  // namespace dgk

@@ -115,3 +115,17 @@ def test_one_application_against_its_definition(gpu_lib, n_interior):
     z = np.linalg.solve(-diag, b.reshape(K, Np, 1)).reshape(-1) + P @ _cycle(A1, P.T @ b)
     alpha = (b @ z) / (z @ (S @ z))
     assert rel_l2(x, alpha * z) < 1e-8
+
+
+@pytest.mark.parametrize("N", [1, 3, 5, 6])
+def test_every_order_matches_block_jacobi(gpu_lib, N):
+    """The orders that test_multilevel_matches_block_jacobi leaves out (every order has its own layout of elements in
+    warps), with sparse levels above the dense one, both arithmetic modes: both solves to 1e-10, the solutions agree
+    to 1e-8 as there."""
+    from hopefoam_gb300 import _lib as L
+
+    ps, b = _solver(3000, N, 1.0)
+    x_bj, _ = ps.solve(b, rtol=1e-10, pc=L.DG_PC_BLOCK_JACOBI, precision=L.DG_PREC_FP64)
+    for precision in (L.DG_PREC_FP64, L.DG_PREC_SPLIT):
+        x, st = ps.solve(b, rtol=1e-10, pc=L.DG_PC_MULTILEVEL, precision=precision)
+        assert st["rel_residual"] <= 1e-10 and rel_l2(x, x_bj) < 1e-8
