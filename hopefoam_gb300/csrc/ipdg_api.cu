@@ -40,6 +40,9 @@ struct IpdgState {
     float* d_sblocks32 = nullptr;  // FP32 rows of the cooperative iterations of small problems
     bool sb32_ready = false;
     double* d_corner = nullptr;
+    // a batch of PCG iterations as a CUDA graph, and the arguments of its launches (run_cg)
+    cudaGraphExec_t cg_graph = nullptr;
+    std::vector<unsigned char> cg_key;
     unsigned char* d_slots = nullptr;
     unsigned long long exchanges = 0;
     double* d_P64 = nullptr;     // the same, grouped layout of the element-aligned kernels
@@ -238,27 +241,47 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
     int best_it = 0;
     // A batch of CHECK iterations is ~20 kernels per iteration; on small
     // operators each is a few microseconds of device work, less than the
-    // host's cost of launching it.  From the second full batch on, a batch is
-    // one CUDA graph (captured once per solve, parity of the first iteration
-    // as its key; the kernels read all vectors and scalars from device memory,
-    // so the graph stays valid while this solve's buffers do).  If capture is
-    // not possible on this stream the batches are launched directly.
-    struct GraphGuard {
-        cudaGraphExec_t g = nullptr;
-        ~GraphGuard() {
-            if (g) cudaGraphExecDestroy(g);
+    // host's cost of launching it.  A full batch is therefore one CUDA graph.
+    // The kernels read all vectors and scalars from device memory, so the graph
+    // stays valid while the arguments of the launches are the same: it is kept with
+    // the operator, with those arguments (the operator's own buffers, tables
+    // and coefficients) as its key, and captured from a solve's second batch on
+    // where they differ.  Capturing and instantiating 16 iterations is 0.5 to
+    // 1 ms; a projection step solves three times with the same launches (K = 32768,
+    // N = 2, two steps: 49.4 -> 46.9 ms).  The learned
+    // forms, whose launches carry more than their arguments say, keep theirs for
+    // one solve.  If capture is not possible on this stream the batches are
+    // launched directly.
+    const bool keep = !v.zb || (v.mg && !v.zl);
+    std::vector<unsigned char> key;
+    auto add_key = [&](const auto& a) {
+        const unsigned char* q = reinterpret_cast<const unsigned char*>(&a);
+        key.insert(key.end(), q, q + sizeof(a));
+    };
+    auto drop_graph = [&]() {
+        if (s->cg_graph) cudaGraphExecDestroy(s->cg_graph);
+        s->cg_graph = nullptr;
+        s->cg_key.clear();
+    };
+    struct Scope {
+        decltype(drop_graph)& drop;
+        bool keep;
+        ~Scope() {
+            if (!keep) drop();
         }
-    } graph;
-    int gparity = -1;
+    } scope{drop_graph, keep};
     bool use_graph = true;
     auto launch_batch = [&](int it0, int count) -> cudaError_t {
-        if (use_graph && count == CHECK && checks > 0) {
-            const int par = it0 & 1;
-            if (graph.g && par != gparity) {
-                cudaGraphExecDestroy(graph.g);
-                graph.g = nullptr;
-            }
-            if (!graph.g) {
+        if (use_graph && count == CHECK) {
+            key.clear();
+            add_key(s->args);
+            add_key(v);
+            if (v.mg) add_key(*v.mg);
+            const int what[4] = {fp32, it0 & 1, CHECK, 0};
+            add_key(what);
+            add_key(c->stream);
+            if (s->cg_graph && key != s->cg_key && checks > 0) drop_graph();
+            if (!s->cg_graph && checks > 0) {
                 cudaGraph_t g = nullptr;
                 cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed);
                 if (e == cudaSuccess) {
@@ -267,17 +290,17 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
                     const cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
                     if (e == cudaSuccess) e = e2;
                 }
-                if (e == cudaSuccess) e = cudaGraphInstantiate(&graph.g, g, 0);
+                if (e == cudaSuccess) e = cudaGraphInstantiate(&s->cg_graph, g, 0);
                 if (g) cudaGraphDestroy(g);
                 if (e != cudaSuccess) {
                     (void)cudaGetLastError();
-                    graph.g = nullptr;
+                    s->cg_graph = nullptr;
                     use_graph = false;
                 } else {
-                    gparity = par;
+                    s->cg_key = key;
                 }
             }
-            if (graph.g) return cudaGraphLaunch(graph.g, c->stream);
+            if (s->cg_graph && key == s->cg_key) return cudaGraphLaunch(s->cg_graph, c->stream);
         }
         for (int j = 0; j < count; j++) {
             const cudaError_t e = launch_pcg_iteration(s->args, v, fp32, (it0 + j) & 1, pnet, pfa, c->stream);
@@ -397,6 +420,7 @@ void ipdg_teardown(dg_ctx* c) {
     if (!c->ipdg) return;
     for (void* p : c->ipdg->allocs) cudaFree(p);
     if (c->ipdg->d_mg) cudaFree(c->ipdg->d_mg);
+    if (c->ipdg->cg_graph) cudaGraphExecDestroy(c->ipdg->cg_graph);
     delete c->ipdg;
     c->ipdg = nullptr;
 }

@@ -129,3 +129,24 @@ def test_every_order_matches_block_jacobi(gpu_lib, N):
     for precision in (L.DG_PREC_FP64, L.DG_PREC_SPLIT):
         x, st = ps.solve(b, rtol=1e-10, pc=L.DG_PC_MULTILEVEL, precision=precision)
         assert st["rel_residual"] <= 1e-10 and rel_l2(x, x_bj) < 1e-8
+
+
+@pytest.mark.parametrize("N,n_interior", [(2, 3000), (4, 12000)])
+def test_repeated_solves_follow_the_operator(gpu_lib, N, n_interior):
+    """Solves that alternate arithmetic, preconditioner and Helmholtz coefficient on one solver, the batches of
+    iterations kept between them, against one solver per solve: the same launches in the same order, so the same bits."""
+    from hopefoam_gb300 import _lib as L
+
+    ps, b = _solver(n_interior, N, 1.0)
+    ml, bj = L.DG_PC_MULTILEVEL, L.DG_PC_BLOCK_JACOBI
+    seq = [(0.0, ml, 1), (0.0, ml, 1), (0.0, ml, 0), (50.0, ml, 1), (50.0, bj, 1), (50.0, ml, 1), (0.0, ml, 1), (50.0, ml, 0)]
+    fresh = {}
+    for mass, pc, precision in seq:
+        assert ps.ctx.lib.dg_ipdg_set_mass(ps.ctx.h, mass) == L.DG_OK
+        x, _ = ps.solve(b, rtol=1e-10, pc=pc, precision=precision)
+        if (mass, pc, precision) not in fresh:
+            p2, _ = _solver(n_interior, N, 1.0)
+            assert p2.ctx.lib.dg_ipdg_set_mass(p2.ctx.h, mass) == L.DG_OK
+            fresh[mass, pc, precision] = p2.solve(b, rtol=1e-10, pc=pc, precision=precision)[0]
+            p2.ctx.close()
+        assert np.array_equal(x, fresh[mass, pc, precision])
