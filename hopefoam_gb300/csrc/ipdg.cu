@@ -40,6 +40,7 @@
 #include "lpc.hpp"
 #include "mg.hpp"
 #include "pcg_reduce.cuh"
+#include "pdl.cuh"
 
 namespace dgk {
 
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(256, 4) ipdg_apply_kernel(IpdgArgs a, const do
     __shared__ T c1[E][NF];
     __shared__ T c2r[E][NF];
     __shared__ T c2s[E][NF];
+    dependency_wait();
     double beta = 0.0;
     if (pc.S) {
         if (pc.S->done) return;
@@ -305,6 +307,7 @@ __global__ void __launch_bounds__(256) ipdg_lane_trace_kernel(IpdgArgs a, const 
     using FR = LaneFaceRec<N>;
     constexpr int Np = L::Np, Nfp = L::Nfp, Nfq = L::Nfq, NB = 3 * N, R = FR::R, ER = FR::ER, SR = FR::SR,
                   GH = FR::GH;
+    dependency_wait();
     if (pc.S->done) return;
     const double beta = pc.S->beta;
     const bool has_beta = beta != 0.0;
@@ -420,6 +423,7 @@ __global__ void __launch_bounds__(256, N <= 4 ? 3 : 2) ipdg_lane_face_apply_kern
     using L = IpLaneTab<N>;
     using FR = LaneFaceRec<N>;
     constexpr int Np = L::Np, Nfq = L::Nfq, NB = 3 * N, R = FR::R, ER = FR::ER, SR = FR::SR, NH = FR::NH;
+    dependency_wait();
     if (pc.S->done) return;
     const bool mass = a.mass_coef != 0.0;
     const double* __restrict__ p_new = pc.p_new;
@@ -835,6 +839,7 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) bj_kernel(const float* _
 template <int NP>
 __global__ void __launch_bounds__(RowDims<NP>::THREADS) pcg_update_kernel(PcgVecs v, int K, int parity) {
     constexpr int EB = RowDims<NP>::EB;
+    dependency_wait();
     if (v.S->done) return;
     const double alpha = v.S->alpha;
     const double* __restrict__ p = v.p[parity ^ 1];
@@ -1013,18 +1018,14 @@ static cudaError_t apply_n(const IpdgArgs& a, bool fp32, const double* u, double
         if (fp32 && pc.dz && pc.S && pc.p_new && a.lane_tab && a.lane_ftr && a.lane_p0) {
             const int grid = std::max(1, std::min((a.K + 127) / 128, pcg_max_grid(a.K, N, a.sms)));
             const IpLaneTab<N>& tab = *static_cast<const IpLaneTab<N>*>(a.lane_tab);
-            ipdg_lane_trace_kernel<N><<<grid, 256, 0, s>>>(a, tab, u, pc);
-            const cudaError_t e = cudaGetLastError();
+            const cudaError_t e = launch_dependent(ipdg_lane_trace_kernel<N>, grid, 256, s, a, tab, u, pc);
             if (e != cudaSuccess) return e;
-            ipdg_lane_face_apply_kernel<N><<<grid, 256, 0, s>>>(a, tab, y, pc);
-            return cudaGetLastError();
+            return launch_dependent(ipdg_lane_face_apply_kernel<N>, grid, 256, s, a, tab, y, pc);
         }
     }
     if (!fp32 && a.sblocks) return launch_block_apply(a, u, y, pc, s);
     const int grid = apply_grid<N>(a);
-    if (fp32) ipdg_apply_kernel<N, float><<<grid, D::THREADS, 0, s>>>(a, u, y, pc);
-    else ipdg_apply_kernel<N, double><<<grid, D::THREADS, 0, s>>>(a, u, y, pc);
-    return cudaGetLastError();
+    return launch_dependent(fp32 ? ipdg_apply_kernel<N, float> : ipdg_apply_kernel<N, double>, grid, D::THREADS, s, a, u, y, pc);
 }
 
 static cudaError_t apply_dispatch(const IpdgArgs& a, bool fp32, const double* u, double* y, const ApplyPcg& pc,
@@ -1139,9 +1140,8 @@ cudaError_t launch_pcg_iteration(const IpdgArgs& a, const PcgVecs& v, bool fp32,
     ApplyPcg pc{v.p[parity], v.p[parity ^ 1], v.S, v.part, v.dz, v.dp[parity], v.dp[parity ^ 1]};
     cudaError_t e = apply_dispatch(a, fp32, v.z, v.Ap, pc, s);
     if (e != cudaSuccess) return e;
-    ROWS_DISPATCH(a.Np,
-                  (pcg_update_kernel<NP><<<rows_grid<NP>(a), RowDims<NP>::THREADS, 0, s>>>(v, a.K, parity)));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    ROWS_DISPATCH(a.Np, e = launch_dependent(pcg_update_kernel<NP>, rows_grid<NP>(a), RowDims<NP>::THREADS, s, v, a.K, parity));
+    if (e != cudaSuccess) return e;
     if (v.zb && v.mg && v.zl && lpc && lpc->sw) {
         e = launch_schwarz_local(*lpc->sw, v.r, v.r32, lpc->U, &v.S->done, s);
         if (e == cudaSuccess)

@@ -31,6 +31,7 @@
 #include "ipdg.hpp"
 #include "ipdg_rows.cuh"
 #include "pcg_reduce.cuh"
+#include "pdl.cuh"
 
 namespace dgk {
 
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS, 3) block_apply_kernel(Ip
                                                                              double* __restrict__ y, ApplyPcg pc) {
     using R = RowDims<NP>;
     constexpr int EB = R::EB, CS = EB * NP;
+    dependency_wait();
     double beta = 0.0;
     if (pc.S) {
         if (pc.S->done) return;
@@ -271,8 +273,7 @@ size_t block_rows_size(int K, int Np) {
 template <int NP>
 static cudaError_t block_apply_n(const IpdgArgs& a, const double* u, double* y, const ApplyPcg& pc, cudaStream_t s) {
     const int grid = std::max(1, std::min(row_groups<NP>(a.K), 3 * a.sms));
-    block_apply_kernel<NP><<<grid, RowDims<NP>::THREADS, 0, s>>>(a, u, y, pc);
-    return cudaGetLastError();
+    return launch_dependent(block_apply_kernel<NP>, grid, RowDims<NP>::THREADS, s, a, u, y, pc);
 }
 
 cudaError_t launch_block_apply(const IpdgArgs& a, const double* u, double* y, const ApplyPcg& pc, cudaStream_t s) {

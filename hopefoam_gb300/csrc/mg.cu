@@ -12,6 +12,7 @@
 #include "ipdg_rows.cuh"
 #include "mg.hpp"
 #include "pcg_reduce.cuh"
+#include "pdl.cuh"
 
 namespace dgk {
 
@@ -406,6 +407,7 @@ cudaError_t launch_mg_dense(const MgDenseLevel* lv, int count, double* work, int
 // summed in a fixed order
 __global__ void __launch_bounds__(256) mg_restrict_dg_kernel(MgLevels m, const double* __restrict__ r,
                                                              double* __restrict__ r1, const int* __restrict__ done) {
+    dependency_wait();
     if (done && *done) return;
     __shared__ double lam[36 * 3];
     for (int i = threadIdx.x; i < 3 * m.Np; i += blockDim.x) lam[i] = m.lam[i];
@@ -447,6 +449,7 @@ constexpr int kDownLanes = 16, kMLanes = 4, kUpLanes = 4;  // lanes per row: abo
 // r_c = B r (blocks [0, bblocks)) and w = M r (the others)
 __global__ void __launch_bounds__(256) mg_down_kernel(MgLevel a, int nc, int bblocks, const double* __restrict__ r,
                                                       double* __restrict__ rc, const int* __restrict__ done) {
+    dependency_wait();
     if (done && *done) return;
     if ((int)blockIdx.x < bblocks) {
         const int t = blockIdx.x * blockDim.x + threadIdx.x, row = t / kDownLanes, l = t % kDownLanes;
@@ -476,6 +479,7 @@ __device__ __forceinline__ void finish_rz(double dot, int mode, PcgScalars* S, d
 template <bool DOT>
 __global__ void __launch_bounds__(256) mg_up_kernel(MgLevel a, const double* __restrict__ xc, const int* __restrict__ done,
                                                     int mode, PcgScalars* S, double* part) {
+    dependency_wait();
     if (done && *done) return;
     double dot = 0;
     for (int row0 = blockIdx.x * (256 / kUpLanes); row0 < a.n; row0 += gridDim.x * (256 / kUpLanes)) {
@@ -496,6 +500,7 @@ __global__ void __launch_bounds__(256) mg_dense_kernel(int n, const double* __re
                                                        double* __restrict__ x, const int* __restrict__ done, int mode,
                                                        PcgScalars* S, double* part) {
     __shared__ double rs[kDense];
+    dependency_wait();
     if (done && *done) return;
     for (int j = threadIdx.x; j < n; j += blockDim.x) rs[j] = r[j];
     __syncthreads();
@@ -535,6 +540,7 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) mg_collect_kernel(MgLeve
                                                                           float* __restrict__ dz, int mode, PcgScalars* S,
                                                                           double* part) {
     using R = RowDims<NP>;
+    dependency_wait();
     if (mode == 3 && S->done) return;
     int e, i;
     row_of<NP>(e, i);
@@ -584,11 +590,10 @@ static cudaError_t launch_collect(const MgLevels& m, const double* zb, const dou
                                   bool zb_summed, PcgScalars* S, double* part, int grid, cudaStream_t s) {
     const int groups = row_groups<NP>(m.K);
     if (zb_summed)
-        mg_collect_kernel<NP, false><<<groups, RowDims<NP>::THREADS, 0, s>>>(m, zb, m.lv[0].x, r, z, dz, mode, S, part);
-    else
-        mg_collect_kernel<NP, true><<<std::min(groups, grid), RowDims<NP>::THREADS, 0, s>>>(m, zb, m.lv[0].x, r, z, dz, mode,
-                                                                                           S, part);
-    return cudaGetLastError();
+        return launch_dependent(mg_collect_kernel<NP, false>, groups, RowDims<NP>::THREADS, s, m, zb, m.lv[0].x, r, z, dz, mode,
+                                S, part);
+    return launch_dependent(mg_collect_kernel<NP, true>, std::min(groups, grid), RowDims<NP>::THREADS, s, m, zb, m.lv[0].x, r,
+                            z, dz, mode, S, part);
 }
 
 static unsigned nb256(int n) { return (unsigned)((n + 255) / 256); }
@@ -597,24 +602,23 @@ cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const doubl
                                  bool zb_summed, PcgScalars* S, double* part, int grid, cudaStream_t s) {
     const int L = m.nl;
     const int* done = mode == 3 ? &S->done : nullptr;  // a stopped iteration leaves every vector as it is
-    mg_restrict_dg_kernel<<<nb256(8 * m.lv[0].n), 256, 0, s>>>(m, r, m.lv[0].r, done);
-    for (int l = 0; l + 1 < L; l++) {
+    cudaError_t e = launch_dependent(mg_restrict_dg_kernel, nb256(8 * m.lv[0].n), 256, s, m, r, m.lv[0].r, done);
+    for (int l = 0; l + 1 < L && e == cudaSuccess; l++) {
         const int nc = m.lv[l + 1].n, bblocks = (int)nb256(kDownLanes * nc);
-        mg_down_kernel<<<bblocks + nb256(kMLanes * m.lv[l].n), 256, 0, s>>>(m.lv[l], nc, bblocks, m.lv[l].r, m.lv[l + 1].r,
-                                                                            done);
+        e = launch_dependent(mg_down_kernel, bblocks + nb256(kMLanes * m.lv[l].n), 256, s, m.lv[l], nc, bblocks, m.lv[l].r,
+                             m.lv[l + 1].r, done);
     }
     const MgLevel& c = m.lv[L - 1];
-    if (L == 1 && zb_summed)
-        mg_dense_kernel<true><<<(c.n + 7) / 8, 256, 0, s>>>(c.n, m.V, c.r, c.x, done, mode, S, part);
-    else
-        mg_dense_kernel<false><<<(c.n + 7) / 8, 256, 0, s>>>(c.n, m.V, c.r, c.x, done, mode, S, part);
-    for (int l = L - 2; l >= 0; l--) {
+    if (e == cudaSuccess)
+        e = launch_dependent(L == 1 && zb_summed ? mg_dense_kernel<true> : mg_dense_kernel<false>, (c.n + 7) / 8, 256, s, c.n,
+                             m.V, c.r, c.x, done, mode, S, part);
+    for (int l = L - 2; l >= 0 && e == cudaSuccess; l--) {
         const int blocks = (int)nb256(kUpLanes * m.lv[l].n);
-        if (l == 0 && zb_summed)
-            mg_up_kernel<true><<<std::min(blocks, grid / 2), 256, 0, s>>>(m.lv[l], m.lv[l + 1].x, done, mode, S, part);
-        else
-            mg_up_kernel<false><<<blocks, 256, 0, s>>>(m.lv[l], m.lv[l + 1].x, done, mode, S, part);
+        const bool dot = l == 0 && zb_summed;
+        e = launch_dependent(dot ? mg_up_kernel<true> : mg_up_kernel<false>, dot ? std::min(blocks, grid / 2) : blocks, 256, s,
+                             m.lv[l], m.lv[l + 1].x, done, mode, S, part);
     }
+    if (e != cudaSuccess) return e;
     switch (m.Np) {
         case 3: return launch_collect<3>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
         case 6: return launch_collect<6>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
