@@ -66,7 +66,8 @@ struct OzArgs {
     const unsigned char* image;
     const int* eb;
     int* status;
-    unsigned char* flags;  // [tiles][4] elements per group left to plain FP64
+    unsigned char* flags;  // per group of 8 elements, those left to plain FP64
+    int groups;            // groups of 8 elements per tile, 1 .. 4
 };
 
 __device__ __forceinline__ uint32_t idesc_f16(int n) {
@@ -360,13 +361,13 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        umma::mbar_init(bOwn, 16);
+        umma::mbar_init(bOwn, 4 * oa.groups);
         umma::mbar_init(bTrFull, 1);
-        umma::mbar_init(bTrRead, 16);
+        umma::mbar_init(bTrRead, 4 * oa.groups);
         umma::mbar_init(bD1full, 1);
-        umma::mbar_init(bD1read, 16);
+        umma::mbar_init(bD1read, 4 * oa.groups);
         umma::mbar_init(bFin, 1);
-        umma::mbar_init(bA2w, 16);
+        umma::mbar_init(bA2w, 4 * oa.groups);
         umma::mbar_init(bA2free, 1);
         for (int i = 0; i < D::NSLOT; i++) {
             umma::mbar_init(bFull + i, 1);
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = *tmemS;
-    const int ntiles = (a.K + 31) / 32;
+    const int tile_elems = 8 * oa.groups, ntiles = (a.K + tile_elems - 1) / tile_elems;
 
     auto wait = [&](uint64_t* bar, uint32_t phase) {
         if (*dead) return;
@@ -466,7 +467,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
             }
         }
         __syncwarp();
-    } else {
+    } else if ((warp & 3) < oa.groups) {
         // -------------------------------------------------------------- compute warps
         const int sub = warp & 3, cg = warp >> 2, t = cg * 32 + lane;  // t: thread within the element group
         const int el = lane & 7, jv = lane >> 3;                       // element of the group; variable, then point
@@ -498,7 +499,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
         };
 #pragma unroll 1
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            const int gk0 = tile * 32 + 8 * sub;  // the group's elements
+            const int gk0 = tile * tile_elems + 8 * sub;  // the group's elements
             const int nval = max(0, min(8, a.K - gk0)) * 4 * Np;
             const size_t g0 = (size_t)gk0 * 4 * Np;
             double q0[IT], o0[IT];
@@ -614,7 +615,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 flux_written();
             }
             // a bound on the volume flux rows of element e from its nodal extremes (FP32)
-            const bool live = tile * 32 + e < a.K;
+            const bool live = gk0 + el < a.K;
             const double rx = geoS[e * 4], sx = geoS[e * 4 + 1], ry = geoS[e * 4 + 2], sy = geoS[e * 4 + 3];
             float est[4];
             {
@@ -827,7 +828,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
             umma::fence_before_sync();
             group_sync(sub);
             const uint32_t fl = flagS[sub];
-            if (t == 0) oa.flags[4 * tile + sub] = (unsigned char)fl;
+            if (t == 0) oa.flags[gk0 >> 3] = (unsigned char)fl;
             // stage update, coalesced
 #pragma unroll
             for (int it = 0; it < IT; it++) {
@@ -842,8 +843,8 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
         // the elements left to plain FP64 (none, as a rule), after the tiles so that
         // the call costs the loop above no registers
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-            for (uint32_t fl = oa.flags[4 * tile + sub]; fl; fl &= fl - 1) {
-                const int k = tile * 32 + 8 * sub + __ffs((int)fl) - 1;
+            for (uint32_t fl = oa.flags[oa.groups * tile + sub]; fl; fl &= fl - 1) {
+                const int k = tile * tile_elems + 8 * sub + __ffs((int)fl) - 1;
                 if (k < a.K)
                     plain_element<N>(a, k, t, sub, [&](int j) { return striped(A1, sub, j, D::A1S, 32 * K1 * 2); });
             }
@@ -871,7 +872,7 @@ static cudaError_t setup_tc(const dgb::RefOps& ops, int K, OzPlan& plan) {
         *plan.h_status = 0;
         e = cudaHostGetDevicePointer((void**)&plan.status, plan.h_status, 0);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&plan.d_image, im.bytes.size() + im.eb.size() * sizeof(int) + (size_t)(K + 31) / 32 * 4);
+    if (e == cudaSuccess) e = cudaMalloc(&plan.d_image, im.bytes.size() + im.eb.size() * sizeof(int) + (size_t)K / 8 + 4);
     if (e != cudaSuccess) return e;
     plan.d_eb = reinterpret_cast<int*>((unsigned char*)plan.d_image + im.bytes.size());
     plan.d_flags = reinterpret_cast<unsigned char*>(plan.d_eb + im.eb.size());
@@ -900,15 +901,29 @@ void teardown_euler_fp64_tc(OzPlan& plan) {
     plan = OzPlan();
 }
 
+// Groups of 8 elements per tile.  A tile of fewer groups is quicker, but not in
+// proportion, since the chain of products and barriers stays: with 1, 2, 3 groups
+// a tile takes 0.67, 0.76, 0.87 of the time of one with 4, within 0.07 at
+// N = 1 .. 7 with either flux (N = 5, Lax-Friedrichs: 39, 43, 49, 55 us).  A small
+// problem is that chain and nothing else, so its tiles are as small as half of
+// the SMs allow (K = 512, N = 2, Roe: 39 -> 26 us).  Beyond that the SM time counts, for the
+// stages of other contexts run beside this one: at K = 3200, N = 3, tiles of 3
+// groups on 134 SMs are quicker alone (41 -> 37 us) and slower with others (28 -> 29).
+static int tile_groups(int K, int sms) {
+    for (int g = 1; g < 4; g++)
+        if ((K + 8 * g - 1) / (8 * g) <= sms / 2) return g;
+    return 4;
+}
+
 template <int N>
 static cudaError_t launch_tc(const OzArgs& oa, const OzPlan& plan, cudaStream_t s) {
-    const int ntiles = (oa.e.K + 31) / 32;
+    const int ntiles = (oa.e.K + 8 * oa.groups - 1) / (8 * oa.groups);
     euler_stage_fp64_tc_kernel<N><<<std::min(ntiles, plan.sms), kOzThreads, OzDims<N>::SMEM, s>>>(oa);
     return cudaGetLastError();
 }
 
 cudaError_t launch_euler_fp64_tc(int N, const EulerArgs& a, const OzPlan& plan, cudaStream_t s) {
-    const OzArgs oa{a, (const unsigned char*)plan.d_image, plan.d_eb, plan.status, plan.d_flags};
+    const OzArgs oa{a, (const unsigned char*)plan.d_image, plan.d_eb, plan.status, plan.d_flags, tile_groups(a.K, plan.sms)};
     switch (N) {
         case 1: return launch_tc<1>(oa, plan, s);
         case 2: return launch_tc<2>(oa, plan, s);

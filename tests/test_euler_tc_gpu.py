@@ -90,3 +90,25 @@ def test_plain_route(gpu_lib, N, flux):
         rest = np.setdiff1d(np.arange(m.K), touched(20))
         assert np.array_equal(g[:, rest], base[:, rest])
     ctx.close()
+
+
+@pytest.mark.parametrize("N,nx,ny", [(2, 19, 16), (4, 61, 5), (1, 33, 18), (3, 37, 22), (5, 46, 20)])
+def test_tiles_of_fewer_groups(gpu_lib, N, nx, ny):
+    """K = 608, 610, 1188, 1628, 1840: on 152 SMs tiles of 1, 2, 2, 3 and 4 groups of 8 elements, with whole and
+    ragged last tiles.  The last element once more with values that leave it and its neighbours to the plain route."""
+    from hopefoam_gb300.mesh import periodic_square
+
+    m = periodic_square(nx, ny, 10.0, 10.0, perturb=0.1, seed=N)
+    ctx, orc, x, y = _setup(m, N)
+    q = _state(x, y, 10.0)
+    base = _against_oracle(ctx, orc, m, N, q, N % 2)
+    big = q.copy()
+    big[:, -1] *= 2.0 ** 150
+    near = np.unique(np.r_[m.K - 1, m.EToE[-1]])
+    ctx.upload(big)
+    g = ctx.rhs(flux=N % 2)
+    r = orc.euler_rhs(big.reshape(-1), flux=N % 2).reshape(g.shape)
+    assert rel_l2(g[:, near], r[:, near]) < 1e-10
+    rest = np.setdiff1d(np.arange(m.K), near)
+    assert np.array_equal(g[:, rest], base[:, rest])
+    ctx.close()
