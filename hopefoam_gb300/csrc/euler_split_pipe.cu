@@ -7,27 +7,45 @@
 // between two CTA barriers, so the FP64-pipe work of staging (one FP64
 // subtraction and conversion per staged value; GB300 retires two FP64
 // operations per clock per SM) and the memory latency of the epilogue leave
-// the other pipes idle.  Here tile t+1's phases are interleaved with tile t's:
+// the other pipes idle.  Here tile t+1's phases are interleaved with tile t's,
+// and no phase ends in a CTA barrier: sixteen compute warps hand over through
+// mbarriers, each waiting only for what it is about to read or overwrite, and
+// one thread of a warp of its own issues every MMA and bulk copy.
 //
-//   prologue:  stage(t0), GEMM1(t0), faces(t0)
+//   compute warps, prologue:  stage(t0); faces(t0)
 //   per tile t (t+1 = the CTA's next tile):
-//     wait GEMM1(t); request t+1's neighbour traces (cp.async)
-//     volume passes of t (TMEM -> FP32 flux -> chunk operand -> GEMM2 MMAs),
-//       with stage(t+1) in slices between them: pass 0 forms t+1's
+//     wait GEMM1(t)
+//     volume passes of t (TMEM -> FP32 flux -> chunk operand), with stage(t+1)
+//       in slices between them: pass 0 waits for every warp to be through the
+//       end of tile t-1, requests t+1's neighbour traces (cp.async) and forms t+1's
 //       reference state and metrics (after its FP64 tile copy has landed),
 //       the later passes its FP32 deltas and TF32 operand
-//     issue the bulk copy of t+2's FP64 tile and GEMM1(t+1)
-//     wait GEMM2(t); R(t) TMEM -> shared
-//     epilogue(t) (LSERK update, global stores) and faces(t+1) with no
-//       barrier between them
+//     faces(t+1) up to the fluxes, wait GEMM2(t), the fluxes into the lift operand
+//     R(t) TMEM -> shared, epilogue(t) (LSERK update, global stores), within the
+//       four warps of 8 elements
+//   issuer:  per volume pass of t its GEMM2 MMAs, the lift's with the last; once
+//     t+1 is staged GEMM1(t+1) and the bulk copy of t+2's FP64 tile
 //
 // The reference state, its FP64 copy and the metrics are double-buffered by
 // tile parity; the FP64 tile buffer, the FP32 deltas, the GEMM1 operand and
 // the neighbour traces are single-buffered because their readers (faces and
 // GEMM1 of t) have finished before stage(t+1) writes them.  The stage input
-// is re-read from L2 in the epilogue.  Every mbarrier wait is bounded; a
-// timeout sets the status word, and the CTA waits for its copies and MMAs in
-// flight before it frees tensor memory and returns.
+// is re-read from L2 in the epilogue.
+//
+// What bounds it: latency at 16 warps per SM.  With every computation, load and
+// store taken out and only the hand-overs left, the stage with CTA barriers and an
+// issuing thread among the compute warps took 214 of its 358 us (N = 5, K =
+// 131,072, Lax-Friedrichs).  Per stage, K = 131,072, N = 1 .. 6, Lax-Friedrichs:
+// 119, 156, 209, 277, 358, 451 us so; with an issuing warp and mbarriers 116, 144,
+// 202, 277, 330, 410; with the wait for the other warps' face phase moved behind
+// the first fluxes 111, 136, 199, 257, 307, 407; with the face fluxes in the
+// wait for GEMM2 107, 130, 184, 236, 309, 392.  Measured and left out: face fluxes
+// in three warps of their own beside the issuer (359 us at N = 5, 320 at N = 4:
+// a face is a long chain, and three warps do not keep up).
+//
+// Every mbarrier wait is bounded; after a timeout nobody waits any more, the
+// status word is set, and the CTA lets its copies and MMAs in flight end before
+// it frees tensor memory and returns.
 #include <algorithm>
 #include <cstdio>
 
@@ -38,6 +56,11 @@
 #include "umma.cuh"
 
 namespace dgk {
+
+// Sixteen compute warps and a warpgroup whose first warp issues.  A launch gives
+// every warp 96 registers; the compute warps take 104, which the second
+// warpgroup leaves them: 16 * 104 + 4 * 64 = 20 * 96.
+constexpr int kPipeThreads = 640, kComputeRegs = 104, kIssuerRegs = 64;
 
 template <int N>
 struct PipeDims {
@@ -57,10 +80,10 @@ struct PipeDims {
     static constexpr int QB_STRIDE = (SZ_QB + 127) / 128 * 128;
     static constexpr int OFF_QB = OFF_Q64 + a128(S::SZ_Q64);
     static constexpr int OFF_NB = OFF_QB + 2 * QB_STRIDE;
-    static constexpr bool GATHER = OFF_NB + a128(S::SZ_NB_FULL) + 64 <= 232448;
+    static constexpr bool GATHER = OFF_NB + a128(S::SZ_NB_FULL) + 128 <= 232448;
     static constexpr int SZ_NB = GATHER ? S::SZ_NB_FULL : 0;
     static constexpr int OFF_BAR = OFF_NB + a128(SZ_NB);
-    static constexpr int SMEM = OFF_BAR + 64;
+    static constexpr int SMEM = OFF_BAR + 128;
     static_assert(SMEM <= 232448, "shared memory budget");
     // volume passes (two chunks per pass where there are two chunk buffers)
     static constexpr int NPASS = S::PAIR ? (S::NCH + 1) / 2 : S::NCH;
@@ -73,8 +96,8 @@ struct PipeDims {
     static constexpr int DQ_PER = (NDQ + DQ_SLICES - 1) / DQ_SLICES;
 };
 
-// The stage for the tiles bid, bid + nblk, ... of one context (a CTA of 512
-// threads); the single-context kernel runs it with its own block index and
+// The stage for the tiles bid, bid + nblk, ... of one context (a CTA of
+// kPipeThreads threads); the single-context kernel runs it with its own block index and
 // grid size, the mixed-order batch kernel with its share of the grid.
 template <int N>
 __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, const int nblk) {
@@ -92,21 +115,15 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     double* sQ64 = reinterpret_cast<double*>(smem + D::OFF_Q64);
     double* sNB = reinterpret_cast<double*>(smem + D::OFF_NB);
     float* sRS = reinterpret_cast<float*>(smem + D::OFF_AC);  // after GEMM2 completed
-    uint64_t* bar1 = reinterpret_cast<uint64_t*>(smem + D::OFF_BAR);
-    uint64_t* bar2 = bar1 + 1;  // [NBUF]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar1 + 3);
-    uint64_t* bq = bar1 + 4;  // the FP64 tile copy has landed
-    // N = 3 (kArrive): every thread's operand writes of a volume pass after the
-    // first, or of the next tile's staging, are done -- every thread arrives,
-    // only the MMA-issuing thread waits, the other warps go on into the next
-    // pass (measured: N = 3 1.14 -> 1.05 ms per step; no change at N = 2;
-    // slower at N = 4, 5, where the warps that run ahead delay the issuing one)
-    // (each part alone at N = 4, 5 measured slower too: passes 1.39 -> 1.43 and
-    // 1.79 -> 1.85 ms per step, end of staging 1.39 -> 1.40 and 1.79 -> 1.80)
-    constexpr bool kArrive = N == 3;      // the later volume passes
-    constexpr bool kArrivePost = N == 3;  // the end of the next tile's staging
-    uint64_t* bready = bar1 + 5;
-    volatile int* sfail = reinterpret_cast<volatile int*>(bar1 + 6);  // a wait of that path timed out
+    uint64_t* bar1 = reinterpret_cast<uint64_t*>(smem + D::OFF_BAR);  // GEMM1 done
+    uint64_t* bar2 = bar1 + 1;     // [NBUF] the chunk's MMAs done
+    uint64_t* bq = bar1 + 3;       // the FP64 tile copy has landed
+    uint64_t* bready = bar1 + 4;   // a volume pass is in the chunk buffers
+    uint64_t* bstaged = bar1 + 5;  // the next tile is staged; its predecessor's D1 and the tile copy are read
+    uint64_t* bfaces = bar1 + 6;   // the tile's face fluxes are in place; traces, deltas and staged results are read
+    uint64_t* bfin = bar1 + 7;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar1 + 8);
+    volatile int* dead = reinterpret_cast<volatile int*>(bar1 + 9);  // a wait timed out: nobody waits any more
     // reference state / metrics of tile parity b
     auto qbf = [&](int b) { return reinterpret_cast<float*>(smem + D::OFF_QB + b * D::QB_STRIDE); };
     auto qbd = [&](int b) {
@@ -122,15 +139,13 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     const float gamma = (float)a.gamma;
     const int G = nblk;
 
-    uint32_t pq = 0;       // bq phase parity
-    bool qpend = false;    // a tile copy in flight (thread 0)
-    bool g1pend = false;   // a GEMM1 in flight whose completion nobody waited for (thread 0)
-    auto issue_q = [&](int t) {
-        const int k0t = t * E;
-        const uint32_t bytes = (uint32_t)min(E, a.K - k0t) * 4u * (uint32_t)Np * 8u;
-        umma::mbar_arrive_expect_tx(bq, bytes);
-        umma::bulk_g2s(sQ64, a.qin + (size_t)k0t * 4 * Np, bytes, bq);
-        qpend = true;
+    auto wait = [&](uint64_t* bar, uint32_t phase) {
+        if (*dead) return;
+        if (!umma::mbar_wait(bar, phase, kWaitLimit)) *dead = 1;
+    };
+    auto arrive = [&](uint64_t* bar) {
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(bar);
     };
 
     // neighbour traces of a tile's faces into sNB by 8-byte asynchronous copies
@@ -173,23 +188,24 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     };
 
     // stage, part 1: the reference state (mean of the three vertex values,
-    // FP32 and its FP64 copy) and FP32 metrics of tile t into parity b; the
-    // tile's FP64 copy must have landed
+    // FP32 and its FP64 copy) and FP32 metrics of the warp's two elements of tile t
+    // into parity b; the tile's FP64 copy must have landed
     auto stage_ref = [&](int t, int b) {
         const int k0t = t * E, net = min(E, a.K - k0t);
-        if (tid < S::ROWS) {
-            const int e = tid >> 2, v = tid & 3;
+        if (lane < 8) {
+            const int r = 8 * warp + lane, e = r >> 2;
             float qb = 1.f;
             if (e < net) {
-                const double* row = sQ64 + e * 4 * Np + v * Np;  // ring order: vertices at 0, N, 2N
+                const double* row = sQ64 + r * Np;  // ring order: vertices at 0, N, 2N
                 qb = (float)((row[0] + row[N] + row[2 * N]) * (1.0 / 3.0));
             }
-            qbf(b)[tid] = qb;
-            qbd(b)[tid] = (double)qb;
-        } else if (tid < S::ROWS + 4 * E) {
-            const int e = (tid - S::ROWS) >> 2, c = (tid - S::ROWS) & 3;
-            geo(b)[tid - S::ROWS] = e < net ? (float)a.geo[(size_t)(k0t + e) * 4 + c] : 0.f;
+            qbf(b)[r] = qb;
+            qbd(b)[r] = (double)qb;
+        } else if (lane < 16) {
+            const int i = 8 * warp + lane - 8, e = i >> 2;
+            geo(b)[i] = e < net ? (float)a.geo[(size_t)(k0t + e) * 4 + (i & 3)] : 0.f;
         }
+        __syncwarp();
     };
     // stage, part 2: FP32 deltas (this thread's items j0 <= j < j1) into sQF and
     // their TF32 hi / lo into the GEMM1 operand
@@ -232,12 +248,14 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
         umma::mbar_init(bar1, 1);
         for (int b = 0; b < S::NBUF; b++) umma::mbar_init(bar2 + b, 1);
         umma::mbar_init(bq, 1);
-        umma::mbar_init(bready, S::THREADS);
-        *sfail = 0;
+        umma::mbar_init(bready, 16);
+        umma::mbar_init(bstaged, 16);
+        umma::mbar_init(bfaces, 16);
+        umma::mbar_init(bfin, 1);
+        *dead = 0;
         umma::fence_mbar_init();
-        if (t0 < ntiles) issue_q(t0);
     }
-    if (warp == 0) {
+    if (warp == 16) {
         umma::tmem_alloc(tmem_slot, S::TMEM_COLS);
         umma::tmem_relinquish();
     }
@@ -254,33 +272,13 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     const uint32_t aAC = umma::smem_u32(smem + D::OFF_AC);
     constexpr uint32_t LO_B1 = NG * KP1 * 4, LO_B2 = S::SZ_B2 / 2, LO_AC = 128 * KC * 4, LO_AF = 128 * NF * 4,
                        STRIDE_AC = S::AL_AC;
-    uint32_t ph1 = 0;
-    uint32_t ph2 = 0;  // bit b: phase parity of chunk buffer b's MMA barrier
-    uint32_t phr = 0;  // phase parity of bready
-    bool failed = false;
     const int qd = warp & 3, sub = warp >> 2;
     const int my_e = 8 * qd + (lane >> 2), my_v = lane & 3;
 
-    // thread 0: GEMM1 of the tile staged in sA1, completion on bar1
-    auto issue_gemm1 = [&]() {
-#pragma unroll
-        for (int s = 0; s < KP1 / 8; s++) {
-            const uint64_t ah = umma::smem_desc(aA1 + s * 256, 128, (KP1 / 4) * 128);
-            const uint64_t al = umma::smem_desc(aA1 + LO_A1 + s * 256, 128, (KP1 / 4) * 128);
-            const uint64_t bh = umma::smem_desc(aB1 + s * 256, 128, (KP1 / 4) * 128);
-            const uint64_t bl = umma::smem_desc(aB1 + LO_B1 + s * 256, 128, (KP1 / 4) * 128);
-            umma::mma_tf32(tD1, ah, bh, idesc1, s > 0);
-            umma::mma_tf32(tD1, al, bh, idesc1, 1);
-            umma::mma_tf32(tD1, ah, bl, idesc1, 1);
-        }
-        umma::commit(bar1);
-        g1pend = true;
-    };
-
     // face fluxes of tile t (reference state / metrics of parity b) into the
     // lift operand sAF; the neighbour traces are in sNB (GATHER) or are loaded
-    // here
-    auto faces = [&](int t, int b) {
+    // here; operand_free() before the first store
+    auto faces = [&](int t, int b, auto operand_free) {
         const int k0 = t * E, ne = min(E, a.K - k0);
         const float* sQB = qbf(b);
         const double* sQBd = qbd(b);
@@ -293,7 +291,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             const int sbase = (seg < FPW ? seg : 0) * FW;
             const int Gf = warp * FPW + seg;
             const bool gok = seg < FPW && Gf < 3 * E;
-            const int Gc = gok ? Gf : warp * FPW;
+            const int Gc = gok ? Gf : min(warp * FPW, 3 * E - 1);
             const int e = Gc / 3, f = Gc - 3 * e;
             const bool valid = gok && e < ne;
             const int k = k0 + (valid ? e : 0);
@@ -386,6 +384,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
 #pragma unroll
                 for (int sl = 0; sl < 2; sl++) lf_flux_delta(nx, ny, m, rb, dm[sl], pm[sl], dp[sl], pp[sl], F[sl]);
             }
+            operand_free();
 #pragma unroll
             for (int sl = 0; sl < 2; sl++) {
                 const int g = li + sl * FW;
@@ -406,10 +405,11 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             constexpr int SW = S::SW, SPW = S::SPW;
             const int seg = lane / SW, i = lane - seg * SW;  // lanes with seg >= SPW idle
             const int sbase = (seg < SPW ? seg : 0) * SW;
-#pragma unroll 1
-            for (int gbase = warp * SPW; gbase < 3 * E; gbase += (S::THREADS / 32) * SPW) {
+            static_assert(S::THREADS / 32 * SPW >= 3 * E, "one pass over the faces");
+            {
+                const int gbase = warp * SPW < 3 * E ? warp * SPW : 3 * E - 1;
                 const int Gf = gbase + seg;
-                const bool gok = seg < SPW && Gf < 3 * E;
+                const bool gok = seg < SPW && Gf < 3 * E && warp * SPW < 3 * E;
                 const int Gc = gok ? Gf : gbase;
                 const int e = Gc / 3, f = Gc - 3 * e;
                 const bool valid = gok && e < ne;
@@ -484,6 +484,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                     }
                     lf_flux_delta(nx, ny, lam, rb, dm, pm, dp, pp, F);
                 }
+                operand_free();
                 if (valid && i < Nfq) {
 #pragma unroll
                     for (int v = 0; v < 4; v++) {
@@ -498,54 +499,146 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
         }
     };
 
-    // ---- prologue: stage, GEMM1 and face fluxes of the first tile
+    if (warp >= 16) {
+        // ------------------------------------------------------------ tensor-core issuer
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssuerRegs));
+        if (warp == 16 && lane == 0) {
+            auto issue_gemm1 = [&]() {
+#pragma unroll
+                for (int s = 0; s < KP1 / 8; s++) {
+                    const uint64_t ah = umma::smem_desc(aA1 + s * 256, 128, (KP1 / 4) * 128);
+                    const uint64_t al = umma::smem_desc(aA1 + LO_A1 + s * 256, 128, (KP1 / 4) * 128);
+                    const uint64_t bh = umma::smem_desc(aB1 + s * 256, 128, (KP1 / 4) * 128);
+                    const uint64_t bl = umma::smem_desc(aB1 + LO_B1 + s * 256, 128, (KP1 / 4) * 128);
+                    umma::mma_tf32(tD1, ah, bh, idesc1, s > 0);
+                    umma::mma_tf32(tD1, al, bh, idesc1, 1);
+                    umma::mma_tf32(tD1, ah, bl, idesc1, 1);
+                }
+                umma::commit(bar1);
+            };
+            auto issue_mma = [&](int ch, int buf) {
+                constexpr uint32_t sboA = (KC / 4) * 128, sboB = (KP2 / 4) * 128;
+                const uint32_t aC = aAC + buf * STRIDE_AC;
+#pragma unroll
+                for (int s = 0; s < KC / 8; s++) {
+                    const uint64_t ah = umma::smem_desc(aC + s * 256, 128, sboA);
+                    const uint64_t al = umma::smem_desc(aC + LO_AC + s * 256, 128, sboA);
+                    const int kb = (s < CH / 8) ? (ch * CH + 8 * s) : (NG + ch * CH + 8 * (s - CH / 8));
+                    const uint64_t bh = umma::smem_desc(aB2 + kb * 32, 128, sboB);
+                    const uint64_t bl = umma::smem_desc(aB2 + LO_B2 + kb * 32, 128, sboB);
+                    const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
+                    umma::mma_tf32(tD2, ah, bh, idesc2, acc);
+                    umma::mma_tf32(tD2, al, bh, idesc2, 1);
+                    umma::mma_tf32(tD2, ah, bl, idesc2, 1);
+                }
+                if (ch == S::NCH - 1) {
+                    constexpr uint32_t sboF = (NF / 4) * 128;
+#pragma unroll
+                    for (int s = 0; s < NF / 8; s++) {
+                        const int kb = 2 * NG + 8 * s;
+                        const uint64_t ah = umma::smem_desc(aAF + s * 256, 128, sboF);
+                        const uint64_t al = umma::smem_desc(aAF + LO_AF + s * 256, 128, sboF);
+                        const uint64_t bh = umma::smem_desc(aB2 + kb * 32, 128, sboB);
+                        const uint64_t bl = umma::smem_desc(aB2 + LO_B2 + kb * 32, 128, sboB);
+                        umma::mma_tf32(tD2, ah, bh, idesc2, 1);
+                        umma::mma_tf32(tD2, al, bh, idesc2, 1);
+                        umma::mma_tf32(tD2, ah, bl, idesc2, 1);
+                    }
+                }
+                umma::commit(bar2 + buf);
+            };
+            int nq = 0;  // tile copies issued
+            auto issue_q = [&](int t) {
+                if (t >= ntiles || *dead) return;
+                const int k0t = t * E;
+                const uint32_t bytes = (uint32_t)min(E, a.K - k0t) * 4u * (uint32_t)Np * 8u;
+                umma::mbar_arrive_expect_tx(bq, bytes);
+                umma::bulk_g2s(sQ64, a.qin + (size_t)k0t * 4 * Np, bytes, bq);
+                nq++;
+            };
+            uint32_t phr = 0, phs = 0;
+            // the staged tile's GEMM1; the tile after it into the FP64 buffer
+            auto next = [&](int t) {
+                wait(bstaged, phs);
+                phs ^= 1;
+                if (*dead) return;
+                umma::fence_after_sync();
+                issue_gemm1();
+                issue_q(t + G);
+            };
+            issue_q(t0);
+            if (t0 < ntiles) next(t0);
+#pragma unroll 1
+            for (int tile = t0; tile < ntiles && !*dead; tile += G) {
+#pragma unroll 1
+                for (int p = 0; p < D::NPASS; p++) {
+                    wait(bready, phr);
+                    phr ^= 1;
+                    if (*dead) break;
+                    umma::fence_after_sync();
+                    if constexpr (S::PAIR) {
+                        issue_mma(2 * p, 0);
+                        if (2 * p + 1 < S::NCH) issue_mma(2 * p + 1, 1);
+                    } else {
+                        issue_mma(p, 0);
+                    }
+                }
+                if (tile + G < ntiles) next(tile + G);
+            }
+            // everything issued ends before the CTA does
+            umma::commit(bfin);
+            umma::mbar_wait(bfin, 0, kWaitLimit);
+            if (*dead) {
+                if (nq) umma::mbar_wait(bq, (uint32_t)(nq - 1) & 1u, kWaitLimit);
+                atomicExch(sa.status, 1);
+            }
+        }
+        __syncwarp();
+    } else {
+    // ---------------------------------------------------------------- compute warps
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kComputeRegs));
+    uint32_t pq = 0, ph1 = 0, phs = 0, phf = 0;
+    uint32_t ph2 = 0;  // bit b: phase parity of chunk buffer b's MMA barrier
+    // tile t is staged: its operand, deltas and traces
+    auto staged = [&]() {
+        if constexpr (D::GATHER) umma::cp_async_wait_all();  // this thread's copies of the traces
+        umma::fence_async_smem();
+        umma::fence_before_sync();
+        arrive(bstaged);
+    };
+    auto face_phase = [&](int t, int b, auto operand_free) {
+        wait(bstaged, phs);
+        phs ^= 1;
+        faces(t, b, operand_free);
+        umma::fence_async_smem();
+    };
+    // ---- prologue: stage and face fluxes of the first tile
     if (t0 < ntiles) {
         if constexpr (D::GATHER) {
             load_links(t0);
             gather(t0);
             load_links(t0 + G);
         }
-        const bool okq = umma::mbar_wait(bq, pq, kWaitLimit);
+        wait(bq, pq);
         pq ^= 1;
-        if (tid == 0 && okq) qpend = false;
-        if (__syncthreads_or(!okq)) failed = true;
-        if (!failed) {
-            stage_ref(t0, 0);
-            __syncthreads();
-            stage_dq(t0, 0, 0, D::NDQ);
-            if constexpr (D::GATHER) umma::cp_async_wait_all();
-            umma::fence_async_smem();
-            umma::fence_before_sync();
-            __syncthreads();
-            umma::fence_after_sync();
-            if (tid == 0) {
-                if (t0 + G < ntiles) issue_q(t0 + G);
-                issue_gemm1();
-            }
-            faces(t0, 0);
-        }
+        stage_ref(t0, 0);
+        stage_dq(t0, 0, 0, D::NDQ);
+        staged();
+        face_phase(t0, 0, []() {});
+        arrive(bfaces);
     }
 
     int par = 0;  // parity of the current tile's reference-state buffer
-    for (int tile = t0; tile < ntiles && !failed; tile += G, par ^= 1) {
+#pragma unroll 1
+    for (int tile = t0; tile < ntiles; tile += G, par ^= 1) {
         const int k0 = tile * E;
         const int ne = min(E, a.K - k0);
         const int tn = tile + G;  // this CTA's next tile
         const bool has_next = tn < ntiles;
-        // ---- wait for GEMM1(t); the face phase of t is complete after this barrier
-        const bool ok1 = umma::mbar_wait(bar1, ph1, kWaitLimit);
+        // ---- GEMM1(t)
+        wait(bar1, ph1);
         ph1 ^= 1;
-        if (tid == 0 && ok1) g1pend = false;
-        if (__syncthreads_or(!ok1)) { failed = true; break; }
         umma::fence_after_sync();
-        if constexpr (D::GATHER) {
-            // every warp has read sNB: request the next tile's traces (they land
-            // during the volume phase), then the links of the tile after it
-            if (has_next) {
-                gather(tn);
-                load_links(tn + G);
-            }
-        }
         // per-thread element data for the volume flux
         float qbe[4];
 #pragma unroll
@@ -610,45 +703,14 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 b[v * VSTR + FSO + LO] = lo;
             }
         };
-        auto issue_mma = [&](int ch, int buf) {
-            constexpr uint32_t sboA = (KC / 4) * 128, sboB = (KP2 / 4) * 128;
-            const uint32_t aC = aAC + buf * STRIDE_AC;
-#pragma unroll
-            for (int s = 0; s < KC / 8; s++) {
-                const uint64_t ah = umma::smem_desc(aC + s * 256, 128, sboA);
-                const uint64_t al = umma::smem_desc(aC + LO_AC + s * 256, 128, sboA);
-                const int kb = (s < CH / 8) ? (ch * CH + 8 * s) : (NG + ch * CH + 8 * (s - CH / 8));
-                const uint64_t bh = umma::smem_desc(aB2 + kb * 32, 128, sboB);
-                const uint64_t bl = umma::smem_desc(aB2 + LO_B2 + kb * 32, 128, sboB);
-                const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
-                umma::mma_tf32(tD2, ah, bh, idesc2, acc);
-                umma::mma_tf32(tD2, al, bh, idesc2, 1);
-                umma::mma_tf32(tD2, ah, bl, idesc2, 1);
-            }
-            if (ch == S::NCH - 1) {
-                constexpr uint32_t sboF = (NF / 4) * 128;
-#pragma unroll
-                for (int s = 0; s < NF / 8; s++) {
-                    const int kb = 2 * NG + 8 * s;
-                    const uint64_t ah = umma::smem_desc(aAF + s * 256, 128, sboF);
-                    const uint64_t al = umma::smem_desc(aAF + LO_AF + s * 256, 128, sboF);
-                    const uint64_t bh = umma::smem_desc(aB2 + kb * 32, 128, sboB);
-                    const uint64_t bl = umma::smem_desc(aB2 + LO_B2 + kb * 32, 128, sboB);
-                    umma::mma_tf32(tD2, ah, bh, idesc2, 1);
-                    umma::mma_tf32(tD2, al, bh, idesc2, 1);
-                    umma::mma_tf32(tD2, ah, bl, idesc2, 1);
-                }
-            }
-            umma::commit(bar2 + buf);
-        };
         // the slice of stage(tn) that goes with volume pass p
         const int pn = par ^ 1;
         auto stage_slice = [&](int p) {
             if (!has_next) return;
             if (p == 0) {
                 // tn's FP64 tile (issued after stage(t)) has landed by now
-                const bool okq = umma::mbar_wait(bq, pq, kWaitLimit);
-                if (!okq) failed = true;
+                wait(bq, pq);
+                pq ^= 1;
                 stage_ref(tn, pn);
             } else if (D::NPASS > 1) {
                 const int j0 = (p - 1) * D::DQ_PER;
@@ -658,160 +720,78 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
         };
 
         // ---- (C) volume phase of t, stage(tn) in slices
-        if constexpr (S::PAIR) {
-            int prev_n = 0;
+        auto chunk_free = [&](int b) {
+            wait(bar2 + b, (ph2 >> b) & 1u);
+            ph2 ^= 1u << b;
+        };
+        constexpr int CPP = S::PAIR ? 2 : 1;  // chunks per pass
+        int prev_n = 0;
 #pragma unroll 1
-            for (int p = 0; p < D::NPASS; p++) {
-                const int ch0 = 2 * p;
-                const int n = (S::NCH - ch0 >= 2) ? 2 : 1;
-                float x0[4], x1[4];
-                umma::tmem_ld4(tD1 + ((uint32_t)(32 * qd) << 16) + ch0 * CH + sub * 4, x0);
-                if (n == 2) umma::tmem_ld4(tD1 + ((uint32_t)(32 * qd) << 16) + (ch0 + 1) * CH + sub * 4, x1);
-                umma::tmem_ld_wait();
-                float fr0[4], fs0[4], fr1[4], fs1[4];
-                vol_flux(x0, ch0, fr0, fs0);
-                if (n == 2) vol_flux(x1, ch0 + 1, fr1, fs1);
-                stage_slice(p);
-                bool okw = !failed;
-                for (int b = 0; b < prev_n; b++) {
-                    okw = umma::mbar_wait(bar2 + b, (ph2 >> b) & 1u, kWaitLimit) && okw;
-                    ph2 ^= 1u << b;
-                }
-                store_chunk(0, fr0, fs0);
-                if (n == 2) store_chunk(1, fr1, fs1);
-                umma::fence_async_smem();
-                umma::fence_before_sync();
-                if (!kArrive || p == 0) {
-                    // (pass 0 staged tn's reference state, which every thread's later
-                    // slices read: always a CTA barrier)
-                    if (__syncthreads_or(!okw)) { failed = true; break; }
-                    umma::fence_after_sync();
-                    if (tid == 0) {
-                        issue_mma(ch0, 0);
-                        if (n == 2) issue_mma(ch0 + 1, 1);
-                    }
-                } else {
-                    if (!okw) *sfail = 1;
-                    umma::mbar_arrive(bready);
-                    if (tid == 0) {
-                        const bool okr = umma::mbar_wait(bready, phr, kWaitLimit);
-                        if (okr && !*sfail) {
-                            umma::fence_after_sync();
-                            issue_mma(ch0, 0);
-                            if (n == 2) issue_mma(ch0 + 1, 1);
-                        } else {
-                            *sfail = 1;
-                        }
-                    }
-                    phr ^= 1u;
-                    __syncwarp();
-                }
-                prev_n = n;
-            }
-        } else {
-            // one chunk buffer: each pass waits for the previous pass's MMAs
-#pragma unroll 1
-            for (int ch = 0; ch < S::NCH; ch++) {
-                float x[4];
-                umma::tmem_ld4(tD1 + ((uint32_t)(32 * qd) << 16) + ch * CH + sub * 4, x);
-                umma::tmem_ld_wait();
-                float fr[4], fs[4];
-                vol_flux(x, ch, fr, fs);
-                stage_slice(ch);
-                bool okw = !failed;
-                if (ch >= 1) {
-                    okw = umma::mbar_wait(bar2, ph2 & 1u, kWaitLimit) && okw;
-                    ph2 ^= 1u;
-                }
-                if (__syncthreads_or(!okw)) { failed = true; break; }
-                store_chunk(0, fr, fs);
-                umma::fence_async_smem();
-                umma::fence_before_sync();
-                __syncthreads();
-                umma::fence_after_sync();
-                if (tid == 0) issue_mma(ch, 0);
-            }
-        }
-        if (failed) break;
-        // the rest of stage(tn): with one volume pass the deltas follow here
-        if (has_next) {
-            if constexpr (D::NPASS == 1) {
-                __syncthreads();  // tn's reference state
-                stage_dq(tn, pn, 0, D::NDQ);
-            }
-        }
-        if constexpr (D::GATHER) umma::cp_async_wait_all();  // tn's neighbour traces (this thread's copies)
-        umma::fence_async_smem();
-        umma::fence_before_sync();
-        if constexpr (kArrivePost && S::PAIR && D::NPASS > 1) {
-            // the issuing thread waits until every thread's staging of tn is written
-            // and its reads of D1 are done (sQ64 was read in pass 0, before its barrier)
-            umma::mbar_arrive(bready);
-            if (has_next) pq ^= 1;  // every thread waited for tn's tile copy in pass 0
-            if (tid == 0) {
-                const bool okr = umma::mbar_wait(bready, phr, kWaitLimit);
-                if (okr && !*sfail) {
-                    umma::fence_after_sync();
+        for (int p = 0; p < D::NPASS; p++) {
+            const int ch0 = CPP * p;
+            const int n = (S::NCH - ch0 >= CPP) ? CPP : 1;
+            float x0[4], x1[4];
+            umma::tmem_ld4(tD1 + ((uint32_t)(32 * qd) << 16) + ch0 * CH + sub * 4, x0);
+            if (n == 2) umma::tmem_ld4(tD1 + ((uint32_t)(32 * qd) << 16) + (ch0 + 1) * CH + sub * 4, x1);
+            umma::tmem_ld_wait();
+            float fr0[4], fs0[4], fr1[4], fs1[4];
+            vol_flux(x0, ch0, fr0, fs0);
+            if (n == 2) vol_flux(x1, ch0 + 1, fr1, fs1);
+            if (p == 0) {
+                // every warp is through its face phase of t: the traces, the deltas and the
+                // staged results in chunk buffer 0 are read
+                wait(bfaces, phf);
+                phf ^= 1;
+                if constexpr (D::GATHER) {
+                    // the next tile's traces land during the volume phase; then the
+                    // links of the tile after it
                     if (has_next) {
-                        qpend = false;
-                        if (tn + G < ntiles) issue_q(tn + G);
-                        issue_gemm1();
+                        gather(tn);
+                        load_links(tn + G);
                     }
-                } else {
-                    *sfail = 1;
                 }
             }
-            phr ^= 1u;
-            __syncwarp();
-        } else {
-            __syncthreads();
-            umma::fence_after_sync();
-            if (has_next) {
-                pq ^= 1;  // every thread waited for tn's tile copy in pass 0
-                if (tid == 0) {
-                    qpend = false;
-                    if (tn + G < ntiles) issue_q(tn + G);  // sQ64 has been read by stage(tn)
-                    issue_gemm1();                         // D1 has been read by the volume phase of t
-                }
-            }
+            stage_slice(p);
+            for (int b = 0; b < prev_n; b++) chunk_free(b);
+            store_chunk(0, fr0, fs0);
+            if (n == 2) store_chunk(1, fr1, fs1);
+            umma::fence_async_smem();
+            umma::fence_before_sync();
+            arrive(bready);
+            prev_n = n;
         }
-        // the epilogue's RK register values and stage input (L2), loaded while the last MMAs run
-        constexpr int EPI = S::EPI;
+        if (has_next) {
+            if constexpr (D::NPASS == 1) stage_dq(tn, pn, 0, D::NDQ);
+            staged();
+        }
+        // the group's 8 elements (the four warps of one tensor-memory quarter): RK
+        // register values and stage input (L2), loaded while the last MMAs run
+        constexpr int EPI = (8 * 4 * Np + 127) / 128;
         const bool first = sa.first != 0;
-        const double* qtile = a.qin + (size_t)k0 * 4 * Np;
+        const int gt = sub * 32 + lane, nv = max(0, min(8, ne - 8 * qd)) * 4 * Np;
+        const size_t base = (size_t)(k0 + 8 * qd) * 4 * Np;
+        float* const sR = sRS + qd * 8 * 4 * Np;
         float resp[EPI];
         double q0v[EPI];
-        {
-            const size_t base = (size_t)k0 * 4 * Np;
+        auto gemm2_done = [&]() {
             const bool need = a.mode == MODE_LSERK && !first;
             const bool needq = a.mode != MODE_RHS;
 #pragma unroll
             for (int j = 0; j < EPI; j++) {
-                const int i = tid + j * S::THREADS;
-                resp[j] = (need && i < ne * 4 * Np) ? __ldg(sa.res32 + base + i) : 0.f;
-                q0v[j] = (needq && i < ne * 4 * Np) ? __ldg(qtile + i) : 0.0;
+                const int i = gt + j * 128;
+                resp[j] = (need && i < nv) ? __ldg(sa.res32 + base + i) : 0.f;
+                q0v[j] = (needq && i < nv) ? __ldg(a.qin + base + i) : 0.0;
             }
-        }
-        // outstanding GEMM2 commits
-        {
-            bool okw = true;
-            if constexpr (S::PAIR) {
-                constexpr int last_n = (S::NCH % 2 == 0) ? 2 : 1;
-#pragma unroll
-                for (int b = 0; b < last_n; b++) {
-                    okw = umma::mbar_wait(bar2 + b, (ph2 >> b) & 1u, kWaitLimit) && okw;
-                    ph2 ^= 1u << b;
-                }
-            } else {
-                okw = umma::mbar_wait(bar2, ph2 & 1u, kWaitLimit);
-                ph2 ^= 1u;
-            }
-            if (__syncthreads_or(!okw || *sfail)) { failed = true; break; }
-        }
+            for (int b = 0; b < prev_n; b++) chunk_free(b);
+        };
+        // ---- face fluxes of tn while the last MMAs of t run; those read the operand
+        // that the fluxes go to
+        if (has_next) face_phase(tn, pn, gemm2_done);
+        else gemm2_done();
         umma::fence_after_sync();
-        // ---- (D) R (tensor memory) -> staging
+        // ---- (D) R (tensor memory) -> staging, in chunk buffer 0
         {
-            const int e2 = 8 * qd + (lane & 7), v2 = lane >> 3;  // this lane's GEMM2 row (g2row)
+            const int e8 = lane & 7, v2 = lane >> 3;  // this lane's GEMM2 row (g2row)
 #pragma unroll
             for (int col = sub * 8; col < NP2; col += 32) {
                 float val[8];
@@ -820,23 +800,21 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
                     const int p = col + j;
-                    if (p < Np && e2 < ne) sRS[(4 * e2 + v2) * Np + p] = val[j];
+                    if (p < Np) sR[(4 * e8 + v2) * Np + p] = val[j];
                 }
             }
         }
         umma::fence_before_sync();
-        __syncthreads();
+        asm volatile("bar.sync %0, 128;" ::"r"(qd + 1) : "memory");
         // ---- epilogue of t
         {
-            const size_t base = (size_t)k0 * 4 * Np;
             const float rka = sa.rkaf, dtf0 = sa.dtf, rkb = sa.rkbf;
-            const int nv = ne * 4 * Np;
             if (a.mode == MODE_LSERK && !sa.dtk32) {
 #pragma unroll
                 for (int j = 0; j < EPI; j++) {
-                    const int i = tid + j * S::THREADS;
+                    const int i = gt + j * 128;
                     if (i < nv) {
-                        const float R = sRS[i];
+                        const float R = sR[i];
                         const float r = first ? dtf0 * R : fmaf(rka, resp[j], dtf0 * R);
                         sa.res32_out[base + i] = r;
                         a.qout[base + i] = q0v[j] + (double)(rkb * r);
@@ -845,12 +823,12 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             } else {
 #pragma unroll
                 for (int j = 0; j < EPI; j++) {
-                    const int i = tid + j * S::THREADS;
+                    const int i = gt + j * 128;
                     if (i >= nv) break;
-                    const float R = sRS[i];
+                    const float R = sR[i];
                     const double q0 = q0v[j];
                     const size_t idx = base + i;
-                    const float dtf = sa.dtk32 ? dtf0 * sa.dtk32[k0 + i / (4 * Np)] : dtf0;
+                    const float dtf = sa.dtk32 ? dtf0 * sa.dtk32[k0 + 8 * qd + i / (4 * Np)] : dtf0;
                     switch (a.mode) {
                         case MODE_RHS: a.rhs[idx] = (double)R; break;
                         case MODE_LSERK: {
@@ -864,29 +842,23 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 }
             }
         }
-        // ---- face fluxes of tn (no barrier: warps move on as their stores issue)
-        if (has_next) faces(tn, pn);
-    }
-    if (failed && tid == 0) atomicExch(sa.status, 1);
-    // let this CTA's asynchronous work in flight complete before it exits
-    if (tid == 0) {
-        if (qpend) umma::mbar_wait(bq, pq, kWaitLimit);
-        if (g1pend) umma::mbar_wait(bar1, ph1, kWaitLimit);
+        arrive(bfaces);
     }
     if constexpr (D::GATHER) umma::cp_async_wait_all();
+    }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == 0) umma::tmem_dealloc(tmem, S::TMEM_COLS);
+    if (warp == 16) umma::tmem_dealloc(tmem, S::TMEM_COLS);
 }
 
 template <int N>
-__global__ void __launch_bounds__(512, 1) euler_stage_split_pipe_kernel(SplitArgs sa) {
+__global__ void __launch_bounds__(kPipeThreads, 1) euler_stage_split_pipe_kernel(SplitArgs sa) {
     pipe_body<N>(sa, blockIdx.x, gridDim.x);
 }
 
 // One stage of several contexts of orders 1..6 in one launch: blocks
 // [cta_end[g-1], cta_end[g]) run group g's tiles with its order's body.
-__global__ void __launch_bounds__(512, 1) euler_stage_split_batch_kernel(const __grid_constant__ SplitBatchArgs P) {
+__global__ void __launch_bounds__(kPipeThreads, 1) euler_stage_split_batch_kernel(const __grid_constant__ SplitBatchArgs P) {
     int g = 0;
     while (g + 1 < P.ngroups && (int)blockIdx.x >= P.cta_end[g]) g++;
     const int begin = g ? P.cta_end[g - 1] : 0;
@@ -900,6 +872,15 @@ __global__ void __launch_bounds__(512, 1) euler_stage_split_batch_kernel(const _
         case 6: pipe_body<6>(P.sa[g], bid, nblk); break;
         default: break;
     }
+}
+
+// the register split (kComputeRegs, kIssuerRegs) draws on what a block is launched
+// with; a build that launches with less must not run
+static cudaError_t check_registers(const void* kernel) {
+    cudaFuncAttributes at;
+    const cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+    if (e != cudaSuccess) return e;
+    return (at.numRegs + 7) / 8 * 8 * (kPipeThreads / 32) >= 16 * kComputeRegs + 4 * kIssuerRegs ? cudaSuccess : cudaErrorInvalidConfiguration;
 }
 
 static int batch_smem(int N) {
@@ -917,6 +898,8 @@ static int batch_smem(int N) {
 cudaError_t setup_split_batch() {
     int smax = 0;
     for (int n = 1; n <= 6; n++) smax = std::max(smax, batch_smem(n));
+    const cudaError_t e = check_registers((const void*)euler_stage_split_batch_kernel);
+    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(euler_stage_split_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
 }
 
@@ -928,19 +911,21 @@ cudaError_t launch_split_batch(const SplitBatchArgs& P, cudaStream_t s) {
         if (sm == 0) return cudaErrorInvalidValue;
         smax = std::max(smax, sm);
     }
-    euler_stage_split_batch_kernel<<<P.cta_end[P.ngroups - 1], 512, smax, s>>>(P);
+    euler_stage_split_batch_kernel<<<P.cta_end[P.ngroups - 1], kPipeThreads, smax, s>>>(P);
     return cudaGetLastError();
 }
 
 template <int N>
 cudaError_t setup_split_pipe() {
+    const cudaError_t e = check_registers((const void*)euler_stage_split_pipe_kernel<N>);
+    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(euler_stage_split_pipe_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 PipeDims<N>::SMEM);
 }
 
 template <int N>
 cudaError_t launch_split_pipe(const SplitArgs& sa, int grid, cudaStream_t s) {
-    euler_stage_split_pipe_kernel<N><<<grid, SplitDims<N>::THREADS, PipeDims<N>::SMEM, s>>>(sa);
+    euler_stage_split_pipe_kernel<N><<<grid, kPipeThreads, PipeDims<N>::SMEM, s>>>(sa);
     return cudaGetLastError();
 }
 
