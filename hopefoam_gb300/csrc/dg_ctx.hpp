@@ -25,7 +25,7 @@ struct SplitPlan {
     int ctas_per_sm = 1;      // launch shape (persistent grid = SMs used x CTAs per SM)
     int sm_budget = 0;        // SMs the grid is sized for (0: all)
     // kernel variant: tile-serial (every order) or software-pipelined across
-    // tiles (N <= 6, euler_split_pipe.cu)
+    // tiles (euler_split_pipe.cu; the default)
     enum { CLASSIC = 0, PIPE = 1 };
     int variant = CLASSIC;
 };

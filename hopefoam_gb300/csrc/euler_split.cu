@@ -977,16 +977,12 @@ static int setup_n(dg_ctx* c) {
     if (cudaFuncSetAttribute(euler_stage_split_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, D::SMEM) !=
         cudaSuccess)
         return DG_ERR_CUDA;
-    if constexpr (!D::STREAM) {
-        if (setup_split_pipe<N>() != cudaSuccess) return DG_ERR_CUDA;
-        if (setup_split_batch() != cudaSuccess) return DG_ERR_CUDA;
-        c->split.variant = SplitPlan::PIPE;
-        // DGCU_SPLIT_VARIANT=classic selects the tile-serial kernel (A/B measurements)
-        const char* v = getenv("DGCU_SPLIT_VARIANT");
-        if (v && strcmp(v, "classic") == 0) c->split.variant = SplitPlan::CLASSIC;
-    } else {
-        c->split.variant = SplitPlan::CLASSIC;
-    }
+    if (setup_split_pipe<N>() != cudaSuccess) return DG_ERR_CUDA;
+    if (!D::STREAM && setup_split_batch() != cudaSuccess) return DG_ERR_CUDA;
+    c->split.variant = SplitPlan::PIPE;
+    // DGCU_SPLIT_VARIANT=classic selects the tile-serial kernel (A/B measurements)
+    const char* v = getenv("DGCU_SPLIT_VARIANT");
+    if (v && strcmp(v, "classic") == 0) c->split.variant = SplitPlan::CLASSIC;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1022,9 +1018,8 @@ static cudaError_t launch_split_n(const EulerArgs& a, const SplitPlan& plan, cud
     const int sms = (plan.sm_budget > 0 && plan.sm_budget < plan.sms) ? plan.sm_budget : plan.sms;
     const int want = sms * (plan.ctas_per_sm > 0 ? plan.ctas_per_sm : 1);
     const int grid = ntiles < want ? ntiles : want;
-    if constexpr (!D::STREAM) {
-        if (plan.variant == SplitPlan::PIPE && sa.qbulk) return launch_split_pipe<N>(sa, grid, s);
-    }
+    // (the tile copies of N <= 6 want a state aligned to 16 bytes)
+    if (plan.variant == SplitPlan::PIPE && (D::STREAM || sa.qbulk)) return launch_split_pipe<N>(sa, grid, s);
     euler_stage_split_kernel<N><<<grid, D::THREADS, D::SMEM, s>>>(sa);
     return cudaGetLastError();
 }

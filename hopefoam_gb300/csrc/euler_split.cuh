@@ -131,7 +131,7 @@ cudaError_t launch_split_batch(const SplitBatchArgs& P, cudaStream_t s);
 // the stage's kernel arguments from the context-level ones (FP32 scalars, tables)
 int split_fill_args(const EulerArgs& a, const SplitPlan& plan, SplitArgs* sa);
 
-// the pipelined variant of the stage (euler_split_pipe.cu) for N <= 6: the
+// the pipelined variant of the stage (euler_split_pipe.cu): the
 // next tile's staging runs under this tile's volume phase and its face phase
 // under this tile's epilogue
 template <int N>

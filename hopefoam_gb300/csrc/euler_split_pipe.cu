@@ -1,5 +1,5 @@
-// euler_split_pipe.cu -- the split-precision fused DG Euler stage for orders
-// N <= 6, software-pipelined across tiles (sm_103a).
+// euler_split_pipe.cu -- the split-precision fused DG Euler stage,
+// software-pipelined across tiles (sm_103a).
 //
 // Same arithmetic, operands, tensor-memory layout and results as
 // euler_stage_split_kernel (euler_split.cu, which documents them); only the
@@ -30,7 +30,10 @@
 // tile parity; the FP64 tile buffer, the FP32 deltas, the GEMM1 operand and
 // the neighbour traces are single-buffered because their readers (faces and
 // GEMM1 of t) have finished before stage(t+1) writes them.  The stage input
-// is re-read from L2 in the epilogue.
+// is re-read from L2 in the epilogue.  At N = 7 there is no FP64 tile buffer
+// and no buffer of deltas (SplitDims): a volume pass reads what it stages from
+// memory ahead of its fluxes, the face phase takes the deltas from the GEMM1
+// operand, and the issuer streams the volume operator's slices.
 //
 // What bounds it: latency at 16 warps per SM.  With every computation, load and
 // store taken out and only the hand-overs left, the stage with CTA barriers and an
@@ -39,7 +42,8 @@
 // 119, 156, 209, 277, 358, 451 us so; with an issuing warp and mbarriers 116, 144,
 // 202, 277, 330, 410; with the wait for the other warps' face phase moved behind
 // the first fluxes 111, 136, 199, 257, 307, 407; with the face fluxes in the
-// wait for GEMM2 107, 130, 184, 236, 309, 392.  Measured and left out: face fluxes
+// wait for GEMM2 107, 130, 184, 236, 309, 395; N = 7, K = 320,000, against the
+// tile-serial kernel: Roe 1609 -> 1430, Lax-Friedrichs 1523 -> 1346.  Measured and left out: face fluxes
 // in three warps of their own beside the issuer (359 us at N = 5, 320 at N = 4:
 // a face is a long chain, and three warps do not keep up).
 //
@@ -65,12 +69,12 @@ constexpr int kPipeThreads = 640, kComputeRegs = 104, kIssuerRegs = 64;
 template <int N>
 struct PipeDims {
     using S = SplitDims<N>;
-    static_assert(!S::STREAM, "the pipelined stage covers N <= 6");
     static constexpr int al(int x) { return (x + 1023) / 1024 * 1024; }  // tensor-core operands
     static constexpr int a128(int x) { return (x + 127) / 128 * 128; }    // everything else
     static constexpr int OFF_B1 = 0;
     static constexpr int OFF_B2 = OFF_B1 + al(S::SZ_B1);
-    static constexpr int OFF_A1 = OFF_B2 + al(S::SZ_B2);
+    static constexpr int OFF_BC = OFF_B2 + al(S::SZ_B2);  // N = 7: streamed [Sr | Ss] slices
+    static constexpr int OFF_A1 = OFF_BC + (S::STREAM ? S::NBUF * S::AL_BC : 0);
     static constexpr int OFF_AC = OFF_A1 + al(S::SZ_A1);
     static constexpr int OFF_AF = OFF_AC + S::NBUF * S::AL_AC;
     static constexpr int OFF_QF = OFF_AF + al(S::SZ_AF);
@@ -92,6 +96,7 @@ struct PipeDims {
     // rows 8w .. 8w + 7, lane = 4 (row % 8) + (k % 4), KP1 / 4 steps along K
     static constexpr int NDQ = S::KP1 / 4;
     static_assert(S::THREADS == 512 && S::ROWS == 128, "16 warps x 8 rows");
+    static_assert(!S::STREAM || (S::NBUF == 2 && S::NCH % 2 == 0), "slices alternate like the chunk buffers");
     static constexpr int DQ_SLICES = NPASS > 1 ? NPASS - 1 : 1;
     static constexpr int DQ_PER = (NDQ + DQ_SLICES - 1) / DQ_SLICES;
 };
@@ -118,12 +123,13 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     uint64_t* bar1 = reinterpret_cast<uint64_t*>(smem + D::OFF_BAR);  // GEMM1 done
     uint64_t* bar2 = bar1 + 1;     // [NBUF] the chunk's MMAs done
     uint64_t* bq = bar1 + 3;       // the FP64 tile copy has landed
-    uint64_t* bready = bar1 + 4;   // a volume pass is in the chunk buffers
-    uint64_t* bstaged = bar1 + 5;  // the next tile is staged; its predecessor's D1 and the tile copy are read
-    uint64_t* bfaces = bar1 + 6;   // the tile's face fluxes are in place; traces, deltas and staged results are read
-    uint64_t* bfin = bar1 + 7;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar1 + 8);
-    volatile int* dead = reinterpret_cast<volatile int*>(bar1 + 9);  // a wait timed out: nobody waits any more
+    uint64_t* bready = bar1 + 4;   // [2] a volume pass is in the chunk buffers (N = 7: in chunk buffer b)
+    uint64_t* bstaged = bar1 + 6;  // the next tile is staged; its predecessor's D1 and the tile copy are read
+    uint64_t* bfaces = bar1 + 7;   // the tile's face fluxes are in place; traces, deltas and staged results are read
+    uint64_t* bfin = bar1 + 8;
+    uint64_t* bfull = bar1 + 9;    // [2] N = 7: the operator slice has landed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar1 + 11);
+    volatile int* dead = reinterpret_cast<volatile int*>(bar1 + 12);  // a wait timed out: nobody waits any more
     // reference state / metrics of tile parity b
     auto qbf = [&](int b) { return reinterpret_cast<float*>(smem + D::OFF_QB + b * D::QB_STRIDE); };
     auto qbd = [&](int b) {
@@ -187,6 +193,33 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
         }
     };
 
+    // N = 7: no FP64 tile copy; what a volume pass stages is read from memory ahead
+    // of its fluxes
+    double pre[S::STREAM ? (D::DQ_PER > 3 ? D::DQ_PER : 3) : 1];
+    float pgeo = 0.f;
+    // the rows and K offsets of this thread in the core-matrix mapping
+    const int cm_r = 8 * warp + (lane >> 2), cm_k = lane & 3;
+    auto fetch_ref = [&](int t) {
+        if constexpr (S::STREAM) {
+            const int k0t = t * E, net = min(E, a.K - k0t), r = 8 * warp + (lane & 7);
+            if (lane < 8 && (r >> 2) < net) {
+                const double* row = a.qin + (size_t)k0t * 4 * Np + (size_t)r * Np;
+#pragma unroll
+                for (int j = 0; j < 3; j++) pre[j] = __ldg(row + j * N);
+            } else if (lane >= 8 && lane < 16 && (r >> 2) < net) {
+                pgeo = (float)a.geo[(size_t)(k0t + (r >> 2)) * 4 + (r & 3)];
+            }
+        }
+    };
+    auto fetch_dq = [&](int t, int j0, int j1) {
+        if constexpr (S::STREAM) {
+            const int net = min(E, a.K - t * E);
+            const double* src = a.qin + (size_t)t * E * 4 * Np + (size_t)cm_r * Np + cm_k;
+#pragma unroll
+            for (int j = 0; j < D::DQ_PER; j++)
+                if (j0 + j < j1 && cm_r < 4 * net && 4 * (j0 + j) + cm_k < Np) pre[j] = __ldg(src + 4 * (j0 + j));
+        }
+    };
     // stage, part 1: the reference state (mean of the three vertex values,
     // FP32 and its FP64 copy) and FP32 metrics of the warp's two elements of tile t
     // into parity b; the tile's FP64 copy must have landed
@@ -196,38 +229,54 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             const int r = 8 * warp + lane, e = r >> 2;
             float qb = 1.f;
             if (e < net) {
-                const double* row = sQ64 + r * Np;  // ring order: vertices at 0, N, 2N
-                qb = (float)((row[0] + row[N] + row[2 * N]) * (1.0 / 3.0));
+                if constexpr (S::STREAM) {
+                    qb = (f64s::trunc_f32(pre[0]) + f64s::trunc_f32(pre[1]) + f64s::trunc_f32(pre[2])) * (1.f / 3.f);
+                } else {
+                    const double* row = sQ64 + r * Np;  // ring order: vertices at 0, N, 2N
+                    qb = (float)((row[0] + row[N] + row[2 * N]) * (1.0 / 3.0));
+                }
             }
             qbf(b)[r] = qb;
-            qbd(b)[r] = (double)qb;
+            if constexpr (!S::STREAM) qbd(b)[r] = (double)qb;
         } else if (lane < 16) {
             const int i = 8 * warp + lane - 8, e = i >> 2;
-            geo(b)[i] = e < net ? (float)a.geo[(size_t)(k0t + e) * 4 + (i & 3)] : 0.f;
+            if constexpr (S::STREAM) geo(b)[i] = e < net ? pgeo : 0.f;
+            else geo(b)[i] = e < net ? (float)a.geo[(size_t)(k0t + e) * 4 + (i & 3)] : 0.f;
         }
         __syncwarp();
     };
     // stage, part 2: FP32 deltas (this thread's items j0 <= j < j1) into sQF and
-    // their TF32 hi / lo into the GEMM1 operand
+    // their TF32 hi / lo into the GEMM1 operand (N = 7: only there, hi + lo is exact;
+    // by integer and FP32 operations, f64split.cuh)
     constexpr uint32_t LO_A1 = 128 * KP1 * 4;
-    // the rows and K offsets of this thread in the core-matrix mapping
-    const int cm_r = 8 * warp + (lane >> 2), cm_k = lane & 3;
     auto stage_dq = [&](int t, int b, int j0, int j1) {
         const int net = min(E, a.K - t * E);
         if (cm_r >= 4 * net) return;  // rows of a missing element (tail tile)
-        const double qr = qbd(b)[cm_r];
-        const double* src = sQ64 + cm_r * Np + cm_k;
-        float* qf = sQF + cm_r * Np + cm_k;
         float* dst = sA1 + (warp * (KP1 / 4)) * 32 + lane;
+        if constexpr (S::STREAM) {
+            const float qr = qbf(b)[cm_r];
 #pragma unroll
-        for (int j = j0; j < j1; j++) {
-            if (j < D::NDQ && 4 * j + cm_k < Np) {
-                const float d = (float)(src[4 * j] - qr);
-                qf[4 * j] = d;
-                float hi, lo;
-                umma::split_tf32(d, hi, lo);
-                dst[32 * j] = hi;
-                dst[32 * j + LO_A1 / 4] = lo;
+            for (int j = 0; j < D::DQ_PER; j++)
+                if (j0 + j < j1 && 4 * (j0 + j) + cm_k < Np) {
+                    float hi, lo;
+                    umma::split_tf32(f64s::minus_f32(pre[j], qr), hi, lo);
+                    dst[32 * (j0 + j)] = hi;
+                    dst[32 * (j0 + j) + LO_A1 / 4] = lo;
+                }
+        } else {
+            const double qr = qbd(b)[cm_r];
+            const double* src = sQ64 + cm_r * Np + cm_k;
+            float* qf = sQF + cm_r * Np + cm_k;
+#pragma unroll
+            for (int j = j0; j < j1; j++) {
+                if (j < D::NDQ && 4 * j + cm_k < Np) {
+                    const float d = (float)(src[4 * j] - qr);
+                    qf[4 * j] = d;
+                    float hi, lo;
+                    umma::split_tf32(d, hi, lo);
+                    dst[32 * j] = hi;
+                    dst[32 * j + LO_A1 / 4] = lo;
+                }
             }
         }
     };
@@ -248,7 +297,10 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
         umma::mbar_init(bar1, 1);
         for (int b = 0; b < S::NBUF; b++) umma::mbar_init(bar2 + b, 1);
         umma::mbar_init(bq, 1);
-        umma::mbar_init(bready, 16);
+        for (int b = 0; b < 2; b++) {
+            umma::mbar_init(bready + b, 16);
+            umma::mbar_init(bfull + b, 1);
+        }
         umma::mbar_init(bstaged, 16);
         umma::mbar_init(bfaces, 16);
         umma::mbar_init(bfin, 1);
@@ -270,6 +322,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     const uint32_t aB1 = umma::smem_u32(sB1), aB2 = umma::smem_u32(sB2);
     const uint32_t aA1 = umma::smem_u32(sA1), aAF = umma::smem_u32(sAF);
     const uint32_t aAC = umma::smem_u32(smem + D::OFF_AC);
+    const uint32_t aBC = umma::smem_u32(smem + D::OFF_BC);
     constexpr uint32_t LO_B1 = NG * KP1 * 4, LO_B2 = S::SZ_B2 / 2, LO_AC = 128 * KC * 4, LO_AF = 128 * NF * 4,
                        STRIDE_AC = S::AL_AC;
     const int qd = warp & 3, sub = warp >> 2;
@@ -300,7 +353,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
 #pragma unroll
             for (int v = 0; v < 4; v++) {
                 qbv[v] = sQB[4 * (valid ? e : 0) + v];
-                qbdv[v] = sQBd[4 * (valid ? e : 0) + v];
+                qbdv[v] = S::STREAM ? 0.0 : sQBd[4 * (valid ? e : 0) + v];
             }
             float own[2][4], nbr[2][4];
 #pragma unroll
@@ -311,7 +364,14 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 if (valid && i < Nfp) {
                     const int pos = (f * N + i) % NB;
 #pragma unroll
-                    for (int v = 0; v < 4; v++) own[sl][v] = sQF[e * 4 * Np + v * Np + pos];
+                    for (int v = 0; v < 4; v++) {
+                        if constexpr (S::STREAM) {
+                            const uint32_t off = umma::kmajor_offset(4 * e + v, pos, KP1) >> 2;
+                            own[sl][v] = sA1[off] + sA1[off + LO_A1 / 4];
+                        } else {
+                            own[sl][v] = sQF[e * 4 * Np + v * Np + pos];
+                        }
+                    }
                     if constexpr (D::GATHER) {
                         const double* nv = sNB + (size_t)((3 * e + f) * Nfp + i) * 4;
 #pragma unroll
@@ -330,7 +390,9 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                             vs = Nfp;
                         }
 #pragma unroll
-                        for (int v = 0; v < 4; v++) nbr[sl][v] = (float)(__ldg(src + v * vs) - qbdv[v]);
+                        for (int v = 0; v < 4; v++)
+                            nbr[sl][v] = S::STREAM ? f64s::minus_f32(__ldg(src + v * vs), qbv[v])
+                                                   : (float)(__ldg(src + v * vs) - qbdv[v]);
                     }
                 }
             }
@@ -516,16 +578,24 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 }
                 umma::commit(bar1);
             };
-            auto issue_mma = [&](int ch, int buf) {
+            auto issue_mma = [&](int ch, int buf, int slice) {
                 constexpr uint32_t sboA = (KC / 4) * 128, sboB = (KP2 / 4) * 128;
                 const uint32_t aC = aAC + buf * STRIDE_AC;
 #pragma unroll
                 for (int s = 0; s < KC / 8; s++) {
                     const uint64_t ah = umma::smem_desc(aC + s * 256, 128, sboA);
                     const uint64_t al = umma::smem_desc(aC + LO_AC + s * 256, 128, sboA);
-                    const int kb = (s < CH / 8) ? (ch * CH + 8 * s) : (NG + ch * CH + 8 * (s - CH / 8));
-                    const uint64_t bh = umma::smem_desc(aB2 + kb * 32, 128, sboB);
-                    const uint64_t bl = umma::smem_desc(aB2 + LO_B2 + kb * 32, 128, sboB);
+                    uint64_t bh, bl;
+                    if constexpr (S::STREAM) {
+                        // the streamed slice has the chunk's own K layout [Sr 16 | Ss 16]
+                        const uint32_t bC = aBC + slice * S::AL_BC;
+                        bh = umma::smem_desc(bC + s * 256, 128, sboA);
+                        bl = umma::smem_desc(bC + S::SZ_BC / 2 + s * 256, 128, sboA);
+                    } else {
+                        const int kb = (s < CH / 8) ? (ch * CH + 8 * s) : (NG + ch * CH + 8 * (s - CH / 8));
+                        bh = umma::smem_desc(aB2 + kb * 32, 128, sboB);
+                        bl = umma::smem_desc(aB2 + LO_B2 + kb * 32, 128, sboB);
+                    }
                     const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
                     umma::mma_tf32(tD2, ah, bh, idesc2, acc);
                     umma::mma_tf32(tD2, al, bh, idesc2, 1);
@@ -535,11 +605,13 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                     constexpr uint32_t sboF = (NF / 4) * 128;
 #pragma unroll
                     for (int s = 0; s < NF / 8; s++) {
-                        const int kb = 2 * NG + 8 * s;
+                        // lift part: k = 2 NG + 8 s of the resident image, or k = 8 s of the lift's own
+                        const int kb = S::STREAM ? 8 * s : 2 * NG + 8 * s;
+                        constexpr uint32_t sbo = S::STREAM ? sboF : sboB;
                         const uint64_t ah = umma::smem_desc(aAF + s * 256, 128, sboF);
                         const uint64_t al = umma::smem_desc(aAF + LO_AF + s * 256, 128, sboF);
-                        const uint64_t bh = umma::smem_desc(aB2 + kb * 32, 128, sboB);
-                        const uint64_t bl = umma::smem_desc(aB2 + LO_B2 + kb * 32, 128, sboB);
+                        const uint64_t bh = umma::smem_desc(aB2 + kb * 32, 128, sbo);
+                        const uint64_t bl = umma::smem_desc(aB2 + LO_B2 + kb * 32, 128, sbo);
                         umma::mma_tf32(tD2, ah, bh, idesc2, 1);
                         umma::mma_tf32(tD2, al, bh, idesc2, 1);
                         umma::mma_tf32(tD2, ah, bl, idesc2, 1);
@@ -549,7 +621,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             };
             int nq = 0;  // tile copies issued
             auto issue_q = [&](int t) {
-                if (t >= ntiles || *dead) return;
+                if (S::STREAM || t >= ntiles || *dead) return;
                 const int k0t = t * E;
                 const uint32_t bytes = (uint32_t)min(E, a.K - k0t) * 4u * (uint32_t)Np * 8u;
                 umma::mbar_arrive_expect_tx(bq, bytes);
@@ -566,21 +638,51 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 issue_gemm1();
                 issue_q(t + G);
             };
+            // N = 7: slices of the operator, one per chunk and again for every tile, in two
+            // buffers; g counts them
+            const int mine = t0 < ntiles ? (ntiles - t0 + G - 1) / G * S::NCH : 0;
+            int nsl = 0;
+            uint32_t ph2i = 0;
+            auto issue_slice = [&]() {
+                if (nsl >= mine || *dead) return;
+                const int b = nsl & 1;
+                umma::mbar_arrive_expect_tx(bfull + b, S::SZ_BC);
+                umma::bulk_g2s(smem + D::OFF_BC + b * S::AL_BC, sa.b2 + S::SZ_B2 / 4 + (size_t)(nsl % S::NCH) * (S::SZ_BC / 4),
+                               S::SZ_BC, bfull + b);
+                nsl++;
+            };
             issue_q(t0);
+            if constexpr (S::STREAM) {
+                issue_slice();
+                issue_slice();
+            }
             if (t0 < ntiles) next(t0);
+            int g = 0;
 #pragma unroll 1
             for (int tile = t0; tile < ntiles && !*dead; tile += G) {
 #pragma unroll 1
                 for (int p = 0; p < D::NPASS; p++) {
-                    wait(bready, phr);
-                    phr ^= 1;
+                    const int buf = S::STREAM ? p & 1 : 0;
+                    wait(bready + buf, (phr >> buf) & 1u);
+                    phr ^= 1u << buf;
+                    if constexpr (S::STREAM) wait(bfull + (g & 1), (uint32_t)(g >> 1) & 1u);
                     if (*dead) break;
                     umma::fence_after_sync();
                     if constexpr (S::PAIR) {
-                        issue_mma(2 * p, 0);
-                        if (2 * p + 1 < S::NCH) issue_mma(2 * p + 1, 1);
+                        issue_mma(2 * p, 0, 0);
+                        if (2 * p + 1 < S::NCH) issue_mma(2 * p + 1, 1, 0);
                     } else {
-                        issue_mma(p, 0);
+                        issue_mma(p, buf, S::STREAM ? g & 1 : 0);
+                    }
+                    if constexpr (S::STREAM) {
+                        // the MMAs before these are through with their slice: the next one into its place
+                        if (g > 0) {
+                            const int o = buf ^ 1;
+                            wait(bar2 + o, (ph2i >> o) & 1u);
+                            ph2i ^= 1u << o;
+                            issue_slice();
+                        }
+                        g++;
                     }
                 }
                 if (tile + G < ntiles) next(tile + G);
@@ -590,6 +692,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             umma::mbar_wait(bfin, 0, kWaitLimit);
             if (*dead) {
                 if (nq) umma::mbar_wait(bq, (uint32_t)(nq - 1) & 1u, kWaitLimit);
+                for (int q = max(0, nsl - 2); q < nsl; q++) umma::mbar_wait(bfull + (q & 1), (uint32_t)(q >> 1) & 1u, kWaitLimit);
                 atomicExch(sa.status, 1);
             }
         }
@@ -619,10 +722,20 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             gather(t0);
             load_links(t0 + G);
         }
-        wait(bq, pq);
-        pq ^= 1;
-        stage_ref(t0, 0);
-        stage_dq(t0, 0, 0, D::NDQ);
+        if constexpr (S::STREAM) {
+            fetch_ref(t0);
+            stage_ref(t0, 0);
+#pragma unroll 1
+            for (int j = 0; j < D::NDQ; j += D::DQ_PER) {
+                fetch_dq(t0, j, min(D::NDQ, j + D::DQ_PER));
+                stage_dq(t0, 0, j, min(D::NDQ, j + D::DQ_PER));
+            }
+        } else {
+            wait(bq, pq);
+            pq ^= 1;
+            stage_ref(t0, 0);
+            stage_dq(t0, 0, 0, D::NDQ);
+        }
         staged();
         face_phase(t0, 0, []() {});
         arrive(bfaces);
@@ -709,8 +822,10 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             if (!has_next) return;
             if (p == 0) {
                 // tn's FP64 tile (issued after stage(t)) has landed by now
-                wait(bq, pq);
-                pq ^= 1;
+                if constexpr (!S::STREAM) {
+                    wait(bq, pq);
+                    pq ^= 1;
+                }
                 stage_ref(tn, pn);
             } else if (D::NPASS > 1) {
                 const int j0 = (p - 1) * D::DQ_PER;
@@ -725,7 +840,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             ph2 ^= 1u << b;
         };
         constexpr int CPP = S::PAIR ? 2 : 1;  // chunks per pass
-        int prev_n = 0;
+        [[maybe_unused]] int prev_n = 0;
 #pragma unroll 1
         for (int p = 0; p < D::NPASS; p++) {
             const int ch0 = CPP * p;
@@ -733,6 +848,10 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             float x0[4], x1[4];
             umma::tmem_ld4(tD1 + ((uint32_t)(32 * qd) << 16) + ch0 * CH + sub * 4, x0);
             if (n == 2) umma::tmem_ld4(tD1 + ((uint32_t)(32 * qd) << 16) + (ch0 + 1) * CH + sub * 4, x1);
+            if (has_next) {
+                if (p == 0) fetch_ref(tn);
+                else fetch_dq(tn, (p - 1) * D::DQ_PER, min(D::NDQ, p * D::DQ_PER));
+            }
             umma::tmem_ld_wait();
             float fr0[4], fs0[4], fr1[4], fs1[4];
             vol_flux(x0, ch0, fr0, fs0);
@@ -752,13 +871,21 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 }
             }
             stage_slice(p);
-            for (int b = 0; b < prev_n; b++) chunk_free(b);
-            store_chunk(0, fr0, fs0);
-            if (n == 2) store_chunk(1, fr1, fs1);
-            umma::fence_async_smem();
-            umma::fence_before_sync();
-            arrive(bready);
-            prev_n = n;
+            if constexpr (S::STREAM) {
+                if (p >= 2) chunk_free(p & 1);
+                store_chunk(p & 1, fr0, fs0);
+                umma::fence_async_smem();
+                umma::fence_before_sync();
+                arrive(bready + (p & 1));
+            } else {
+                for (int b = 0; b < prev_n; b++) chunk_free(b);
+                store_chunk(0, fr0, fs0);
+                if (n == 2) store_chunk(1, fr1, fs1);
+                umma::fence_async_smem();
+                umma::fence_before_sync();
+                arrive(bready);
+                prev_n = n;
+            }
         }
         if (has_next) {
             if constexpr (D::NPASS == 1) stage_dq(tn, pn, 0, D::NDQ);
@@ -782,7 +909,12 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 resp[j] = (need && i < nv) ? __ldg(sa.res32 + base + i) : 0.f;
                 q0v[j] = (needq && i < nv) ? __ldg(a.qin + base + i) : 0.0;
             }
-            for (int b = 0; b < prev_n; b++) chunk_free(b);
+            if constexpr (S::STREAM) {
+                chunk_free(0);
+                chunk_free(1);
+            } else {
+                for (int b = 0; b < prev_n; b++) chunk_free(b);
+            }
         };
         // ---- face fluxes of tn while the last MMAs of t run; those read the operand
         // that the fluxes go to
@@ -935,11 +1067,13 @@ template cudaError_t setup_split_pipe<3>();
 template cudaError_t setup_split_pipe<4>();
 template cudaError_t setup_split_pipe<5>();
 template cudaError_t setup_split_pipe<6>();
+template cudaError_t setup_split_pipe<7>();
 template cudaError_t launch_split_pipe<1>(const SplitArgs&, int, cudaStream_t);
 template cudaError_t launch_split_pipe<2>(const SplitArgs&, int, cudaStream_t);
 template cudaError_t launch_split_pipe<3>(const SplitArgs&, int, cudaStream_t);
 template cudaError_t launch_split_pipe<4>(const SplitArgs&, int, cudaStream_t);
 template cudaError_t launch_split_pipe<5>(const SplitArgs&, int, cudaStream_t);
 template cudaError_t launch_split_pipe<6>(const SplitArgs&, int, cudaStream_t);
+template cudaError_t launch_split_pipe<7>(const SplitArgs&, int, cudaStream_t);
 
 }  // namespace dgk

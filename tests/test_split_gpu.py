@@ -249,10 +249,11 @@ def test_conservation_at_full_size(gpu_lib, case):
     ctx.close()
 
 
-@pytest.mark.parametrize("N,nx,ny", [(1, 71, 70), (2, 64, 38), (3, 71, 70), (4, 49, 50), (5, 71, 70), (6, 77, 32)])
+@pytest.mark.parametrize("N,nx,ny", [(1, 71, 70), (2, 64, 38), (3, 71, 70), (4, 49, 50), (5, 71, 70), (6, 77, 32),
+                                     (7, 71, 70), (7, 49, 50), (7, 3, 5)])
 def test_split_tiles_per_block(gpu_lib, N, nx, ny):
-    """One, two and three tiles of 32 elements per block of the pipelined stage (K = 4864 = 152 tiles, 4900, 4928,
-    9940; whole and ragged last tiles), both fluxes: the right-hand side against the FP64 path within the tolerance of
+    """Less than a tile, one, two and three tiles of 32 elements per block of the pipelined stage (K = 30, 4864 = 152
+    tiles, 4900, 4928, 9940; whole and ragged last tiles), both fluxes: the right-hand side against the FP64 path within the tolerance of
     the parity meshes (the error falls with h), and two steps that repeat to the bit."""
     from hopefoam_gb300 import _lib as L
     from hopefoam_gb300 import euler
