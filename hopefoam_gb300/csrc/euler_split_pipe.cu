@@ -17,14 +17,16 @@
 //     wait GEMM1(t)
 //     volume passes of t (TMEM -> FP32 flux -> chunk operand), with stage(t+1)
 //       in slices between them: pass 0 waits for every warp to be through the
-//       end of tile t-1, requests t+1's neighbour traces (cp.async) and forms t+1's
-//       reference state and metrics (after its FP64 tile copy has landed),
-//       the later passes its FP32 deltas and TF32 operand
+//       end of tile t-1 and forms t+1's reference state and metrics (after its
+//       FP64 tile copy has landed), the later passes its FP32 deltas and TF32
+//       operand
 //     faces(t+1) up to the fluxes, wait GEMM2(t), the fluxes into the lift operand
 //     R(t) TMEM -> shared, epilogue(t) (LSERK update, global stores), within the
 //       four warps of 8 elements
 //   issuer:  per volume pass of t its GEMM2 MMAs, the lift's with the last; once
 //     t+1 is staged GEMM1(t+1) and the bulk copy of t+2's FP64 tile
+//   the three warps beside the issuer:  t+1's neighbour traces (cp.async) when
+//     the face phase of t has read its own
 //
 // The reference state, its FP64 copy and the metrics are double-buffered by
 // tile parity; the FP64 tile buffer, the FP32 deltas, the GEMM1 operand and
@@ -42,7 +44,8 @@
 // 119, 156, 209, 277, 358, 451 us so; with an issuing warp and mbarriers 116, 144,
 // 202, 277, 330, 410; with the wait for the other warps' face phase moved behind
 // the first fluxes 111, 136, 199, 257, 307, 407; with the face fluxes in the
-// wait for GEMM2 107, 130, 184, 236, 309, 395; N = 7, K = 320,000, against the
+// wait for GEMM2 107, 130, 184, 236, 309, 395; with the traces requested by other
+// warps (N <= 5) 105, 131, 181, 234, 296.  N = 7, K = 320,000, against the
 // tile-serial kernel: Roe 1609 -> 1430, Lax-Friedrichs 1523 -> 1346.  Measured and left out: face fluxes
 // in three warps of their own beside the issuer (359 us at N = 5, 320 at N = 4:
 // a face is a long chain, and three warps do not keep up).
@@ -61,10 +64,11 @@
 
 namespace dgk {
 
-// Sixteen compute warps and a warpgroup whose first warp issues.  A launch gives
+// Sixteen compute warps and a warpgroup whose first warp issues and whose others
+// request the neighbour traces.  A launch gives
 // every warp 96 registers; the compute warps take 104, which the second
 // warpgroup leaves them: 16 * 104 + 4 * 64 = 20 * 96.
-constexpr int kPipeThreads = 640, kComputeRegs = 104, kIssuerRegs = 64;
+constexpr int kPipeThreads = 640, kComputeRegs = 104, kIssuerRegs = 64, kTraceWarps = 3;
 
 template <int N>
 struct PipeDims {
@@ -158,12 +162,13 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     // (the neighbour element's node in its own face order with the rotation
     // applied, or the boundary slot's trace); cn[j]: the face link of this
     // thread's task j, loaded ahead
-    constexpr int GT = (3 * E * Nfp + S::THREADS - 1) / S::THREADS;
+    constexpr int FT = 32 * kTraceWarps, GT = (3 * E * Nfp + FT - 1) / FT;
+    const int ft = tid - 17 * 32;
     int cn[GT];
     auto load_links = [&](int t) {
 #pragma unroll
         for (int j = 0; j < GT; j++) {
-            const int i = tid + j * S::THREADS;
+            const int i = ft + j * FT;
             cn[j] = (t < ntiles && i < 3 * min(E, a.K - t * E) * Nfp) ? __ldg(a.conn + (size_t)t * E * 3 + i / Nfp) : 0;
         }
     };
@@ -172,7 +177,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
         const int nt = 3 * min(E, a.K - kt) * Nfp;
 #pragma unroll
         for (int j = 0; j < GT; j++) {
-            const int i = tid + j * S::THREADS;
+            const int i = ft + j * FT;
             if (i >= nt) break;
             const int ef = i / Nfp, ii = i - ef * Nfp;
             const int c = cn[j];
@@ -301,7 +306,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             umma::mbar_init(bready + b, 16);
             umma::mbar_init(bfull + b, 1);
         }
-        umma::mbar_init(bstaged, 16);
+        umma::mbar_init(bstaged, 16 + (D::GATHER ? kTraceWarps : 0));
         umma::mbar_init(bfaces, 16);
         umma::mbar_init(bfin, 1);
         *dead = 0;
@@ -564,7 +569,30 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     if (warp >= 16) {
         // ------------------------------------------------------------ tensor-core issuer
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssuerRegs));
-        if (warp == 16 && lane == 0) {
+        if (warp > 16) {
+            // ---------------------------------------------------- neighbour traces
+            if constexpr (D::GATHER) {
+                uint32_t phf = 0;
+                if (t0 < ntiles) {
+                    load_links(t0);
+                    gather(t0);
+                    load_links(t0 + G);
+                    umma::cp_async_wait_all();
+                    arrive(bstaged);
+                }
+#pragma unroll 1
+                for (int tn = t0 + G; tn < ntiles; tn += G) {
+                    // every warp has read the traces of the tile before; these land during
+                    // its volume phase
+                    wait(bfaces, phf);
+                    phf ^= 1;
+                    gather(tn);
+                    load_links(tn + G);
+                    umma::cp_async_wait_all();
+                    arrive(bstaged);
+                }
+            }
+        } else if (lane == 0) {
             auto issue_gemm1 = [&]() {
 #pragma unroll
                 for (int s = 0; s < KP1 / 8; s++) {
@@ -704,7 +732,6 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     uint32_t ph2 = 0;  // bit b: phase parity of chunk buffer b's MMA barrier
     // tile t is staged: its operand, deltas and traces
     auto staged = [&]() {
-        if constexpr (D::GATHER) umma::cp_async_wait_all();  // this thread's copies of the traces
         umma::fence_async_smem();
         umma::fence_before_sync();
         arrive(bstaged);
@@ -717,11 +744,6 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     };
     // ---- prologue: stage and face fluxes of the first tile
     if (t0 < ntiles) {
-        if constexpr (D::GATHER) {
-            load_links(t0);
-            gather(t0);
-            load_links(t0 + G);
-        }
         if constexpr (S::STREAM) {
             fetch_ref(t0);
             stage_ref(t0, 0);
@@ -861,14 +883,6 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 // staged results in chunk buffer 0 are read
                 wait(bfaces, phf);
                 phf ^= 1;
-                if constexpr (D::GATHER) {
-                    // the next tile's traces land during the volume phase; then the
-                    // links of the tile after it
-                    if (has_next) {
-                        gather(tn);
-                        load_links(tn + G);
-                    }
-                }
             }
             stage_slice(p);
             if constexpr (S::STREAM) {
