@@ -462,77 +462,51 @@ __global__ void __launch_bounds__(256) mg_down_kernel(MgLevel a, int nc, int bbl
     }
 }
 
-// Where the level on the vertices comes out of the cycle, r1.x1 with r1 = P^T r
-// and x1 its result is what the correction adds to r.z: the sum over vertices
-// replaces one over all rows, which would read r again.  Finishes the iteration
-// or leaves rz, from S->rzb = r.zb.
-__device__ __forceinline__ void finish_rz(double dot, int mode, PcgScalars* S, double* part) {
-    double val[1] = {dot}, tot[1];
-    if (grid_sum<1>(val, part, gridDim.x, &S->counter, tot) && threadIdx.x == 0) {
-        const double rz = S->rzb + tot[0];
-        if (mode == 3) pcg_finish(S, rz, 0.0, S->rr);
-        else S->rz = rz;
-    }
-}
-
-// x = w + B^T x_c; DOT: and x.r
-template <bool DOT>
-__global__ void __launch_bounds__(256) mg_up_kernel(MgLevel a, const double* __restrict__ xc, const int* __restrict__ done,
-                                                    int mode, PcgScalars* S, double* part) {
+// x = w + B^T x_c
+__global__ void __launch_bounds__(256) mg_up_kernel(MgLevel a, const double* __restrict__ xc, const int* __restrict__ done) {
     dependency_wait();
     if (done && *done) return;
-    double dot = 0;
-    for (int row0 = blockIdx.x * (256 / kUpLanes); row0 < a.n; row0 += gridDim.x * (256 / kUpLanes)) {
-        const int row = row0 + threadIdx.x / kUpLanes, l = threadIdx.x % kUpLanes;
-        const double s = row_dot<kUpLanes>(a.tptr, a.tcol, a.tval, xc, row, row < a.n, l);
-        if (row < a.n && l == 0) {
-            const double x = a.w[row] + s;
-            a.x[row] = x;
-            if (DOT) dot += x * a.r[row];
-        }
-    }
-    if (DOT) finish_rz(dot, mode, S, part);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, row = t / kUpLanes, l = t % kUpLanes;
+    const double s = row_dot<kUpLanes>(a.tptr, a.tcol, a.tval, xc, row, row < a.n, l);
+    if (row < a.n && l == 0) a.x[row] = a.w[row] + s;
 }
 
-// x = V r, one warp per row, r staged in shared memory; DOT: and x.r
-template <bool DOT>
+// x = V r, one warp per row, r staged in shared memory
 __global__ void __launch_bounds__(256) mg_dense_kernel(int n, const double* __restrict__ V, const double* __restrict__ r,
-                                                       double* __restrict__ x, const int* __restrict__ done, int mode,
-                                                       PcgScalars* S, double* part) {
+                                                       double* __restrict__ x, const int* __restrict__ done) {
     __shared__ double rs[kDense];
     dependency_wait();
     if (done && *done) return;
     for (int j = threadIdx.x; j < n; j += blockDim.x) rs[j] = r[j];
     __syncthreads();
     const int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
-    double dot = 0;
-    if (row < n) {
-        const double* v = V + (size_t)row * n;
-        double s0 = 0, s1 = 0;
-        int j = lane;
+    if (row >= n) return;
+    const double* v = V + (size_t)row * n;
+    double s0 = 0, s1 = 0;
+    int j = lane;
 #pragma unroll 4
-        for (; j + 32 < n; j += 64) {
-            s0 += v[j] * rs[j];
-            s1 += v[j + 32] * rs[j + 32];
-        }
-        if (j < n) s0 += v[j] * rs[j];
-        s0 += s1;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        if (lane == 0) {
-            x[row] = s0;
-            dot = s0 * rs[row];
-        }
+    for (; j + 32 < n; j += 64) {
+        s0 += v[j] * rs[j];
+        s1 += v[j + 32] * rs[j + 32];
     }
-    if (DOT) finish_rz(dot, mode, S, part);
+    if (j < n) s0 += v[j] * rs[j];
+    s0 += s1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    if (lane == 0) x[row] = s0;
 }
 
 // z = zb + P x1, and dz from the mirror of zb to that of z: z - z0 = (zb - zb0) +
 // (c - c0).  Bound by the FP64 pipe: three operations for c, one each for z and
-// c - c0, which is rounded to FP32 by integer operations.  DOT (the learned
-// forms, whose r.zb nobody has summed): r.z as well, finishing like the learned
-// preconditioner's collect.  K = 101,246, N = 4: 34 us with the sum over
-// all rows here, 22 us without (and 8 us more in the kernel that sums the vertices).
+// c - c0, which is rounded to FP32 by integer operations.  What the correction adds
+// to r.z is r1.x1 with r1 = P^T r and x1 the cycle's result: the first kDotBlocks
+// blocks sum it over the vertices beside the others and finish the iteration, or
+// leave rz, from S->rzb = r.zb.  DOT (the learned forms, whose r.zb nobody has
+// summed): r.z over all rows instead, finishing like the learned preconditioner's
+// collect.  K = 101,246, N = 4: 34 us with the sum over all rows, 22 us with
+// the vertices' sum in the kernel before (and 8 us there), 22 us with it here.
+constexpr int kDotBlocks = 64;
+
 template <int NP, bool DOT>
 __global__ void __launch_bounds__(RowDims<NP>::THREADS) mg_collect_kernel(MgLevels m, const double* __restrict__ zb,
                                                                           const double* __restrict__ x1,
@@ -545,10 +519,23 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) mg_collect_kernel(MgLeve
     int e, i;
     row_of<NP>(e, i);
     const bool lane_ok = e < R::EB;
+    if (!DOT && blockIdx.x < kDotBlocks) {
+        const MgLevel& a = m.lv[0];
+        double dot = 0;
+        for (int v = blockIdx.x * R::THREADS + threadIdx.x; v < a.n; v += kDotBlocks * R::THREADS) dot += a.x[v] * a.r[v];
+        double val[1] = {dot}, tot[1];
+        if (grid_sum<1>(val, part, kDotBlocks, &S->counter, tot) && threadIdx.x == 0) {
+            const double rz = S->rzb + tot[0];
+            if (mode == 3) pcg_finish(S, rz, 0.0, S->rr);
+            else S->rz = rz;
+        }
+        return;
+    }
+    const int blk = blockIdx.x - (DOT ? 0 : kDotBlocks), nblk = gridDim.x - (DOT ? 0 : kDotBlocks);
     const double l0 = m.lam[3 * i], l1 = m.lam[3 * i + 1], l2 = m.lam[3 * i + 2];
     __shared__ double c0s[R::WA ? 1 : R::EB];
     double rz = 0;
-    for (int grp = blockIdx.x; grp < row_groups<NP>(m.K); grp += gridDim.x) {
+    for (int grp = blk; grp < row_groups<NP>(m.K); grp += nblk) {
         const int k = grp * R::EB + e;
         const bool act = lane_ok && k < m.K;
         const size_t t = (size_t)k * NP + i;
@@ -590,7 +577,7 @@ static cudaError_t launch_collect(const MgLevels& m, const double* zb, const dou
                                   bool zb_summed, PcgScalars* S, double* part, int grid, cudaStream_t s) {
     const int groups = row_groups<NP>(m.K);
     if (zb_summed)
-        return launch_dependent(mg_collect_kernel<NP, false>, groups, RowDims<NP>::THREADS, s, m, zb, m.lv[0].x, r, z, dz, mode,
+        return launch_dependent(mg_collect_kernel<NP, false>, groups + kDotBlocks, RowDims<NP>::THREADS, s, m, zb, m.lv[0].x, r, z, dz, mode,
                                 S, part);
     return launch_dependent(mg_collect_kernel<NP, true>, std::min(groups, grid), RowDims<NP>::THREADS, s, m, zb, m.lv[0].x, r,
                             z, dz, mode, S, part);
@@ -609,15 +596,9 @@ cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const doubl
                              m.lv[l + 1].r, done);
     }
     const MgLevel& c = m.lv[L - 1];
-    if (e == cudaSuccess)
-        e = launch_dependent(L == 1 && zb_summed ? mg_dense_kernel<true> : mg_dense_kernel<false>, (c.n + 7) / 8, 256, s, c.n,
-                             m.V, c.r, c.x, done, mode, S, part);
-    for (int l = L - 2; l >= 0 && e == cudaSuccess; l--) {
-        const int blocks = (int)nb256(kUpLanes * m.lv[l].n);
-        const bool dot = l == 0 && zb_summed;
-        e = launch_dependent(dot ? mg_up_kernel<true> : mg_up_kernel<false>, dot ? std::min(blocks, grid / 2) : blocks, 256, s,
-                             m.lv[l], m.lv[l + 1].x, done, mode, S, part);
-    }
+    if (e == cudaSuccess) e = launch_dependent(mg_dense_kernel, (c.n + 7) / 8, 256, s, c.n, m.V, c.r, c.x, done);
+    for (int l = L - 2; l >= 0 && e == cudaSuccess; l--)
+        e = launch_dependent(mg_up_kernel, nb256(kUpLanes * m.lv[l].n), 256, s, m.lv[l], m.lv[l + 1].x, done);
     if (e != cudaSuccess) return e;
     switch (m.Np) {
         case 3: return launch_collect<3>(m, zb, r, z, dz, mode, zb_summed, S, part, grid, s);
