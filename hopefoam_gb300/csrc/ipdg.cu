@@ -1074,7 +1074,10 @@ cudaError_t launch_invert_blocks(double* blocks, float* blocks32, int K, int Np,
 template <int NP>
 static int rows_grid(const IpdgArgs& a) {
     const int ngroups = (a.K + RowDims<NP>::EB - 1) / RowDims<NP>::EB;
-    return std::max(1, std::min(ngroups, 8 * a.sms));  // 256 threads x 32 registers: 8 CTAs per SM
+    // as many as are resident: from Np = 15 on the block row takes the update to 64
+    // registers, 4 CTAs per SM, and a second wave of CTAs costs more than longer loops
+    // (K = 101,246, N = 4, multilevel solve 27.5 ms with 8, 27.0 with 4); below, up to 8
+    return std::max(1, std::min(ngroups, (NP >= 15 ? 4 : 8) * a.sms));
 }
 
 template <int NP>
