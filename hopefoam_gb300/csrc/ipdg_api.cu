@@ -226,7 +226,7 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
         const int rcp = persist_rows(c, v, fp32, &prows);
         if (rcp) return rcp;
     }
-    const bool persist = prows != nullptr;
+    bool persist = prows != nullptr;
     const int CHECK = persist ? (refresh > 0 ? 16 * refresh : 256) : 16;
     if (persist && refresh > 0) refresh = 1;
     int checks = 0;
@@ -310,11 +310,17 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
     };
     while (h.it < limit) {
         const int batch = std::min(CHECK, limit - h.it);
-        if (persist)
-            IP_CUDA(c, launch_pcg_persistent(s->args, v, fp32, prows, s->d_corner, s->d_slots, &s->exchanges, h.it & 1,
-                                             batch, c->stream));
-        else
-            IP_CUDA(c, launch_batch(h.it, batch));
+        if (persist) {
+            const cudaError_t e = launch_pcg_persistent(s->args, v, fp32, prows, s->d_corner, s->d_slots, &s->exchanges,
+                                                        h.it & 1, batch, c->stream);
+            if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has (a partition of it)
+                (void)cudaGetLastError();
+                persist = false;
+            } else {
+                IP_CUDA(c, e);
+            }
+        }
+        if (!persist) IP_CUDA(c, launch_batch(h.it, batch));
         IP_CUDA(c, cudaMemcpyAsync(&h, s->d_S, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
         IP_CUDA(c, cudaStreamSynchronize(c->stream));
         checks++;
