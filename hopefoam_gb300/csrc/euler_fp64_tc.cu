@@ -841,7 +841,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
             }
         }
         // the elements left to plain FP64 (none, as a rule), after the tiles so that
-        // the call costs the loop above no registers
+        // the call costs the loop above no registers.  The group's flags are thread 0's
+        // stores, the last tile's with no barrier behind it yet: every thread must read
+        // the same, since plain_element has the group's barrier inside
+        group_sync(sub);
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
             for (uint32_t fl = oa.flags[oa.groups * tile + sub]; fl; fl &= fl - 1) {
                 const int k = tile * tile_elems + 8 * sub + __ffs((int)fl) - 1;
@@ -878,6 +881,7 @@ static cudaError_t setup_tc(const dgb::RefOps& ops, int K, OzPlan& plan) {
     plan.d_flags = reinterpret_cast<unsigned char*>(plan.d_eb + im.eb.size());
     e = cudaMemcpy(plan.d_image, im.bytes.data(), im.bytes.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(plan.d_eb, im.eb.data(), im.eb.size() * sizeof(int), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemset(plan.d_flags, 0, (size_t)K / 8 + 4);
     if (e == cudaSuccess) plan.ready = true;
     return e;
 }

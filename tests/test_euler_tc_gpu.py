@@ -112,3 +112,32 @@ def test_tiles_of_fewer_groups(gpu_lib, N, nx, ny):
     rest = np.setdiff1d(np.arange(m.K), near)
     assert np.array_equal(g[:, rest], base[:, rest])
     ctx.close()
+
+
+@pytest.mark.parametrize("N,nx,ny", [(1, 3, 3), (2, 5, 5), (3, 3, 7), (4, 3, 11), (1, 35, 35), (1, 49, 50), (2, 71, 70)])
+@pytest.mark.parametrize("flux", [0, 1])
+def test_route_changes_between_launches(gpu_lib, N, nx, ny, flux):
+    """Elements that take the plain route in one launch and not in the next, on contexts whose flags no launch has written
+    yet and over many launches: one to three tiles per block, last groups of two and four elements (K = 18, 50, 42, 66, 2450,
+    4900, 9940), where three of a group's four warps have little or nothing to update.  Each launch gives the bits that
+    its state has on a context of its own; the scaled state against the oracle as in test_plain_route."""
+    from hopefoam_gb300.mesh import periodic_square
+
+    m = periodic_square(nx, ny, 10.0, 10.0, perturb=0.1, seed=N)
+    ctx, orc, x, y = _setup(m, N)
+    q = _state(x, y, 10.0)
+    big = q.copy()
+    big[:, -1] *= 2.0 ** 150  # the last element: with its neighbours beyond the FP32 exponents
+    every = q * 2.0 ** 150
+    want = []
+    for w in (q, big, every):
+        c, _, _, _ = _setup(m, N)
+        c.upload(w)
+        want.append(c.rhs(flux=flux))
+        c.close()
+    for j in (1, 0, 2, 0, 1, 2, 1) * 4:
+        ctx.upload((q, big, every)[j])
+        assert np.array_equal(ctx.rhs(flux=flux), want[j])
+    r = orc.euler_rhs(every.reshape(-1), flux=flux).reshape(want[2].shape)
+    assert rel_l2(want[2], r) < 1e-10
+    ctx.close()
