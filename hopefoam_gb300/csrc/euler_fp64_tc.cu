@@ -6,8 +6,8 @@
 // cubature and face points, weak derivative, lift) are 18,400.  Here those
 // run as exact integer products on tcgen05 (ozaki.cuh: seven base-256
 // digits per value, FP16 operands, FP32 accumulators that hold exact
-// integers), with an error against 64 bits below the FMA chain's; the FP64
-// pipe keeps the point-wise fluxes (25 operations per cubature point with
+// integers), with an error against extended precision no larger than the FMA
+// chain's (kFluxSlack); the FP64 pipe keeps the point-wise fluxes (25 operations per cubature point with
 // reciprocals from FP32 seeds) and the Runge-Kutta update.
 //
 // One CTA per SM walks tiles of 32 elements (128 operand rows).  Warps
@@ -24,17 +24,17 @@
 //   4. result rows -> FP64, stage update.
 // The metrics carry the element's time step, so the results are dt R.
 // The digits of a row share one exponent.  For the nodal rows it is the row's
-// own; for the flux rows it comes from the face fluxes and from a bound on
-// the volume fluxes formed from the element's nodal extremes.  An element
-// whose fluxes leave that bound, or with values that are not finite or
-// outside the FP32 exponent range, is left to plain FP64 after the tiles, as
-// euler_fp64.cu does it (plain_element).  All of this is per element: results
-// do not depend on an element's place in the mesh.
+// own (for neighbour traces each face's own); for the flux rows it comes from the
+// face fluxes and from the volume fluxes at the nodes, in FP32, doubled.  An element
+// whose fluxes leave that bound or stay too far below it, whose density or
+// energy varies too much (kFluxSlack, kRhoDepth, kEnergyDepth), or with values that
+// are not finite or outside the FP32 exponent range, is left to plain FP64 after the
+// tiles, as euler_fp64.cu does it (plain_element).  All of this is per element:
+// results do not depend on an element's place in the mesh.
 //
-// Measured, LSERK4 stage, against the kernel of euler_fp64.cu: K = 32768,
-// N = 5, LF 2.66 ms -> 396 us; K = 9800, N = 7, Roe 2.62 ms -> 281 us;
-// K = 3200, N = 3, LF 78 -> 41 us; so it is taken at every order and size.
-// Right-hand sides against 80-bit arithmetic: 2.7e-13 relative at N = 5, both.
+// Measured, LSERK4 stage in a queue of steps, against the kernel of euler_fp64.cu: K = 32768,
+// N = 5, LF 2.66 ms -> 399 us; K = 9794, N = 7, Roe 2.62 ms -> 197 us;
+// K = 3200, N = 3, LF 78 -> 26 us; so it is taken at every order and size.
 // What bounds it now: the FP64 pipe is busy half of the time (58,000 of
 // 117,000 cycles per tile at N = 5: 25,000 in the face fluxes, 30,000 in the
 // volume fluxes); the four warps of a scheduler run their integer phases
@@ -60,6 +60,20 @@ namespace dgk {
 namespace {
 
 constexpr int kOzThreads = 544;
+
+// What an element may lose to the common exponents of its rows, in bits; beyond, it
+// is left to plain FP64.  A value is cut at 2^-56 of its row's bound, FP64 arithmetic rounds
+// at 2^-53 of the value.  kFluxSlack: how far the bound of a flux row may lie above
+// the largest flux that it held.  kRhoDepth, kEnergyDepth: how far a density or an
+// energy at a point may lie below the row's largest nodal value.  With these, the
+// error of the right-hand side against extended precision has, over random elements of
+// one kind, a median of 0.5 to 1.1 of the plain kernel's (N = 1 .. 7, both fluxes, density,
+// pressure or velocity varying by 1.5, 10, 25, 100 and 900 inside an element, neighbours up
+// to 900 times apart), and single elements no more than twice its.  Densities 25 times
+// below, without that limit: twice the error in an ill-conditioned element at N = 7; 100 times: 1.3 as
+// the median at N = 4.  The exponent from products of nodal extremes in place of nodal fluxes,
+// which this kernel used before: 2.5 at contrast 10, 20 at 100, 200 at 900.
+constexpr int kFluxSlack = 3, kRhoDepth = 4, kEnergyDepth = 9;
 
 struct OzArgs {
     EulerArgs e;
@@ -103,18 +117,19 @@ __device__ __forceinline__ void arrived(float (&d)[R][4]) {
     for (int s = 0; s < R; s++) asm volatile("" : "+f"(d[s][0]), "+f"(d[s][1]), "+f"(d[s][2]), "+f"(d[s][3]));
 }
 
-// four consecutive columns of seven digit groups (stride P) -> FP64 values
-// of the lane's row
-template <int P>
-__device__ __forceinline__ void load7(uint32_t taddr, int ebab, double x[4]) {
-    float d[7][4];
+// four consecutive columns of eight digit groups (stride P) -> FP64 values
+// of the lane's row; ebab(c): the bounds of both rows added
+template <int P, typename E>
+__device__ __forceinline__ void load8(uint32_t taddr, E ebab, double x[4]) {
+    float d[8][4];
 #pragma unroll
-    for (int s = 0; s < 7; s++) umma::tmem_ld4(taddr + s * P, d[s]);
+    for (int s = 0; s < 8; s++) umma::tmem_ld4(taddr + s * P, d[s]);
     arrived(d);
 #pragma unroll
     for (int c = 0; c < 4; c++)
-        x[c] = oz::combine7(oz::acc_int22(d[0][c]), oz::acc_int22(d[1][c]), oz::acc_int22(d[2][c]), oz::acc_int22(d[3][c]),
-                            oz::acc_int22(d[4][c]), oz::acc_int22(d[5][c]), oz::acc_int22(d[6][c]), ebab);
+        x[c] = oz::combine_nodal(oz::acc_int22(d[0][c]), oz::acc_int22(d[1][c]), oz::acc_int22(d[2][c]), oz::acc_int22(d[3][c]),
+                                 oz::acc_int22(d[4][c]), oz::acc_int22(d[5][c]), oz::acc_int22(d[6][c]), oz::acc_int22(d[7][c]),
+                                 ebab(c));
 }
 
 struct FaceSide {
@@ -194,19 +209,16 @@ __device__ __forceinline__ bool bounded_wait(uint64_t* bar, uint32_t phase) {
 __device__ __forceinline__ void group_sync(int sub) { asm volatile("bar.sync %0, 128;" ::"r"(sub + 1) : "memory"); }
 
 // One operator piece: operand slices at `as` (AS bytes apart, reduction KP)
-// times the piece's digit blocks of P rows, digit pairs into columns d + P s.
-// Nodal operands keep the pairs i + j <= 6, flux operands i + j <= 7 (the zero
-// block 7 of their operator starts every group).  Unrolled: one thread issues
-// every MMA, and their rate is the piece's latency.
-template <int AS, int KP, int P, bool FLUX>
+// times the piece's digit blocks of P rows, digit pairs i + j = s <= 7 into columns
+// d + P s (the zero block 7 of the operator starts every group).  Unrolled: one
+// thread issues every MMA, and their rate is the piece's latency.
+template <int AS, int KP, int P>
 __device__ __forceinline__ void digit_product(uint32_t d, uint32_t as, uint32_t bs, bool start) {
     constexpr uint32_t SBO = (uint32_t)(KP / 8) << 7;
     const uint64_t ad = umma::smem_desc(as, 128, SBO), bd = umma::smem_desc(bs, 128, SBO);
 #pragma unroll
     for (int i = 0; i < oz::kSlices; i++) {
-        constexpr int S = oz::kSlices;
-        const int nj = FLUX ? (i == 0 ? S + 1 : S + 1 - i) : S - i;
-        const int n = (nj * P + 15) & ~15;
+        const int n = ((oz::kSlices + 1 - i) * P + 15) & ~15;
 #pragma unroll
         for (int ks = 0; ks < KP / 16; ks++)
 #pragma unroll
@@ -270,48 +282,45 @@ __device__ __noinline__ void plain_element(const EulerArgs& a, int k, int t, int
             *sc((4 + v) * Ng + g) = sx * fx[v] + sy * fy[v];
         }
     }
-    if (t < 3) {
-        const int f = t, c = a.conn[(size_t)k * 3 + f];
-        double nx, ny, fsc, lam = 0;
+    // face fluxes, a thread a point; the wave speeds of a face meet in the scratch
+    const int f = t / Nfq, i = t - f * Nfq;
+    double nx = 0, ny = 0, fsc = 0, qm[4], qp[4];
+    if (t < NF) {
+        const int c = a.conn[(size_t)k * 3 + f];
         face_normal(f, rx, sx, ry, sy, nx, ny, fsc);
-        auto side = [&](int i, double qm[4], double qp[4]) {
 #pragma unroll 1
-            for (int v = 0; v < 4; v++) {
-                double m = 0, p = 0;
+        for (int v = 0; v < 4; v++) {
+            double m = 0, p = 0;
 #pragma unroll 1
-                for (int j = 0; j < Nfp; j++) {
-                    const double w = a.ops.If[i * Nfp + j];
-                    m += w * qe[v * Np + (f * N + j) % NB];
-                    double o;
-                    if (c >= 0) {
-                        const int fn = c & 3, jj = ((c >> 2) & 1) ? (N - j) : j;
-                        o = a.qin[((size_t)(c >> 3) * 4 + v) * Np + (fn * N + jj) % NB];
-                    } else {
-                        o = a.btrace[((size_t)(-1 - c) * 4 + v) * Nfp + j];
-                    }
-                    p += w * o;
+            for (int j = 0; j < Nfp; j++) {
+                const double w = a.ops.If[i * Nfp + j];
+                m += w * qe[v * Np + (f * N + j) % NB];
+                double o;
+                if (c >= 0) {
+                    const int fn = c & 3, jj = ((c >> 2) & 1) ? (N - j) : j;
+                    o = a.qin[((size_t)(c >> 3) * 4 + v) * Np + (fn * N + jj) % NB];
+                } else {
+                    o = a.btrace[((size_t)(-1 - c) * 4 + v) * Nfp + j];
                 }
-                qm[v] = m;
-                qp[v] = p;
+                p += w * o;
             }
-        };
-        if (a.flux != 1)
-#pragma unroll 1
-            for (int i = 0; i < Nfq; i++) {
-                double qm[4], qp[4];
-                side(i, qm, qp);
-                lam = fmax(lam, wave_speed(gamma, nx, ny, qm));
-                lam = fmax(lam, wave_speed(gamma, nx, ny, qp));
-            }
-#pragma unroll 1
-        for (int i = 0; i < Nfq; i++) {
-            double qm[4], qp[4], F[4];
-            side(i, qm, qp);
-            if (a.flux == 1) roe_flux(gamma, nx, ny, qm, qp, F);
-            else lf_flux(gamma, nx, ny, lam, qm, qp, F);
-#pragma unroll 1
-            for (int v = 0; v < 4; v++) *sc(8 * Ng + v * NF + f * Nfq + i) = fsc * F[v];
+            qm[v] = m;
+            qp[v] = p;
         }
+        if (a.flux != 1) *sc(8 * Ng + 4 * NF + t) = fmax(wave_speed(gamma, nx, ny, qm), wave_speed(gamma, nx, ny, qp));
+    }
+    if (a.flux != 1) group_sync(sub);
+    if (t < NF) {
+        double F[4], lam = 0;
+        if (a.flux == 1) {
+            roe_flux(gamma, nx, ny, qm, qp, F);
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < Nfq; j++) lam = fmax(lam, *sc(8 * Ng + 4 * NF + f * Nfq + j));
+            lf_flux(gamma, nx, ny, lam, qm, qp, F);
+        }
+#pragma unroll 1
+        for (int v = 0; v < 4; v++) *sc(8 * Ng + v * NF + t) = fsc * F[v];
     }
     group_sync(sub);
 #pragma unroll 1
@@ -348,10 +357,11 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
     double* nrmS = reinterpret_cast<double*>(smem + D::OFF_NRM);
     int* connS = reinterpret_cast<int*>(smem + D::OFF_CONN);
     uint32_t* maxq = reinterpret_cast<uint32_t*>(smem + D::OFF_MAXQ);
-    int* minr = reinterpret_cast<int*>(smem + D::OFF_MINR);
-    int* e3S = reinterpret_cast<int*>(smem + D::OFF_E3);
+    uint32_t* h3S = reinterpret_cast<uint32_t*>(smem + D::OFF_H3);
+    uint32_t* estS = reinterpret_cast<uint32_t*>(smem + D::OFF_EST);
     uint32_t* maxf = reinterpret_cast<uint32_t*>(smem + D::OFF_MAXF);
     uint32_t* flagS = reinterpret_cast<uint32_t*>(smem + D::OFF_FLAG);
+    uint32_t* reachS = reinterpret_cast<uint32_t*>(smem + D::OFF_REACH);
     int* ebS = reinterpret_cast<int*>(smem + D::OFF_EB);
     volatile int* dead = reinterpret_cast<volatile int*>(smem + D::OFF_DEAD);
     uint32_t* tmemS = reinterpret_cast<uint32_t*>(smem + D::OFF_TMEM);
@@ -447,10 +457,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                     const uint32_t b = take();
                     if (*dead) break;
                     umma::fence_after_sync();
-                    if (flux) digit_product<D::A2S, 32, D::NP2, true>(tmem + D::T_RES, a2, b, p == 3);
-                    else if (p == 0) digit_product<D::A1S, K1, 32, false>(tmem + D::T_OWN, a1, b, true);
-                    else if (p == 1) digit_product<D::A2S, 32, 32, false>(tmem + D::T_NBR, a2, b, true);
-                    else digit_product<D::A1S, K1, 16, false>(tmem + D::T_CUB, a1, b, true);
+                    if (flux) digit_product<D::A2S, 32, D::NP2>(tmem + D::T_RES, a2, b, p == 3);
+                    else if (p == 0) digit_product<D::A1S, K1, 32>(tmem + D::T_OWN, a1, b, true);
+                    else if (p == 1) digit_product<D::A2S, 32, 32>(tmem + D::T_NBR, a2, b, true);
+                    else digit_product<D::A1S, K1, 16>(tmem + D::T_CUB, a1, b, true);
                     if (flux || p == 1) umma::commit(bA2free);
                     if (p == 1) umma::commit(bTrFull);
                     else if (!flux && p > 1) umma::commit(bD1full);
@@ -475,7 +485,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
         const uint32_t tlane = tmem + ((uint32_t)(32 * sub) << 16);
         const int ebV = ebS[D::NP2], ebI = ebS[D::NP2 + 1];
         const double g1 = a.gamma - 1.0;
-        const float g1f = fabsf((float)g1);
+        const float g1f = (float)g1;
         constexpr int IT = (32 * Np + 127) / 128;
         uint32_t phT = 0, phD = 0;
         int use = 0;
@@ -524,6 +534,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 maxf[sub * 32 + t - 64] = 0u;
             } else if (t == 96) {
                 flagS[sub] = 0u;
+                reachS[sub] = 0u;
             }
             constexpr int LPR = D::LPR, RPW = 32 / LPR;  // rows per warp pass
 #pragma unroll 1
@@ -533,27 +544,14 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 const double* src = a.qin + ((size_t)(gk0 + i) * 4 + v) * Np + 8 * kb;
                 double x[8];
                 uint32_t mx = 0;
-                int mn = 0x7FF00000;
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    x[j] = 0.0;
-                    if (in && 8 * kb + j < Np) {
-                        x[j] = src[j];
-                        mn = min(mn, __double2hiint(x[j]));
-                    }
-                }
+                for (int j = 0; j < 8; j++) x[j] = in && 8 * kb + j < Np ? src[j] : 0.0;
 #pragma unroll
                 for (int j = 0; j < 8; j++) mx = max(mx, oz::mag_hi(x[j]));
 #pragma unroll
-                for (int o = 1; o < LPR; o <<= 1) {
-                    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-                    mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-                }
+                for (int o = 1; o < LPR; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
                 const int eb = oz::row_bound(mx);
-                if (kb == 0) {
-                    maxq[(8 * sub + i) * 4 + v] = mx;
-                    if (v == 0) minr[8 * sub + i] = mn;
-                }
+                if (kb == 0) maxq[(8 * sub + i) * 4 + v] = mx;
                 if (kb < D::KB1) {
                     uint64_t y[8];
 #pragma unroll
@@ -592,20 +590,33 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                     x[j] = 0.0;
                     if (src[j]) x[j] = *src[j];
                 }
-                uint32_t mx = 0;
+                uint32_t mx[3] = {0, 0, 0};  // a face point takes its own face's nodes only: a bound per face
                 flux_free();
 #pragma unroll
-                for (int j = 0; j < 8; j++) mx = max(mx, oz::mag_hi(x[j]));
-                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const int eb = oz::row_bound(mx);
+                for (int j = 0; j < 8; j++) {
+                    const int f = (8 * kb + j) / Nfp;
+                    const uint32_t h = oz::mag_hi(x[j]);
+#pragma unroll
+                    for (int g = 0; g < 3; g++) mx[g] = max(mx[g], f == g ? h : 0u);
+                }
+#pragma unroll
+                for (int g = 0; g < 3; g++) {
+                    mx[g] = max(mx[g], __shfl_xor_sync(0xffffffffu, mx[g], 1));
+                    mx[g] = max(mx[g], __shfl_xor_sync(0xffffffffu, mx[g], 2));
+                }
                 if (kb == 0) {
-                    e3S[(8 * sub + i) * 4 + v] = eb;
-                    if (!oz::row_ok(mx) || !oz::row_ok(maxq[(8 * sub + i) * 4 + v])) atomicOr(flagS + sub, 1u << i);
+#pragma unroll
+                    for (int g = 0; g < 3; g++) h3S[((8 * sub + i) * 4 + v) * 3 + g] = mx[g];
+                    if (!oz::row_ok(mx[0]) || !oz::row_ok(mx[1]) || !oz::row_ok(mx[2]) ||
+                        !oz::row_ok(maxq[(8 * sub + i) * 4 + v]))
+                        atomicOr(flagS + sub, 1u << i);
                 }
                 uint64_t y[8];
 #pragma unroll
-                for (int j = 0; j < 8; j++) y[j] = oz::biased(x[j], eb);
+                for (int j = 0; j < 8; j++) {
+                    const int f = (8 * kb + j) / Nfp;
+                    y[j] = oz::biased(x[j], oz::row_bound(f == 0 ? mx[0] : f == 1 ? mx[1] : mx[2]));
+                }
                 unsigned char* dst = A2 + (((4 * sub + v) * 4 + kb) << 7) + (i << 4);
 #pragma unroll
                 for (int s = 0; s < oz::kSlices; s++)
@@ -614,24 +625,38 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                                    oz::digit_pair(y[4], y[5], s), oz::digit_pair(y[6], y[7], s));
                 flux_written();
             }
-            // a bound on the volume flux rows of element e from its nodal extremes (FP32)
+            // the largest volume flux at the nodes (FP32), two elements a warp: what the
+            // exponent of the flux rows comes from
+#pragma unroll 1
+            for (int u = 0; u < 2; u++) {
+                const int i = 2 * cg + u;
+                const double* gk = geoS + (8 * sub + i) * 4;
+                const float rx = oz::trunc32(gk[0]), sx = oz::trunc32(gk[1]), ry = oz::trunc32(gk[2]), sy = oz::trunc32(gk[3]);
+                float mf[4] = {0.f, 0.f, 0.f, 0.f};
+                for (int n = lane; n < Np && gk0 + i < a.K; n += 32) {
+                    float q[4];
+#pragma unroll
+                    for (int v = 0; v < 4; v++) q[v] = oz::trunc32(a.qin[((size_t)(gk0 + i) * 4 + v) * Np + n]);
+                    const float ir = __fdividef(1.f, q[0]), uf = q[1] * ir, vf = q[2] * ir;
+                    const float p = g1f * (q[3] - 0.5f * (q[1] * uf + q[2] * vf)), H = (q[3] + p) * ir;
+                    const float Mr = rx * q[1] + ry * q[2], Ms = sx * q[1] + sy * q[2];
+                    mf[0] = fmaxf(mf[0], fmaxf(fabsf(Mr), fabsf(Ms)));
+                    mf[1] = fmaxf(mf[1], fmaxf(fabsf(Mr * uf + rx * p), fabsf(Ms * uf + sx * p)));
+                    mf[2] = fmaxf(mf[2], fmaxf(fabsf(Mr * vf + ry * p), fabsf(Ms * vf + sy * p)));
+                    mf[3] = fmaxf(mf[3], fmaxf(fabsf(Mr * H), fabsf(Ms * H)));
+                }
+#pragma unroll
+                for (int v = 0; v < 4; v++) {
+                    const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(mf[v]));
+                    if (lane == 0) estS[(8 * sub + i) * 4 + v] = m;
+                }
+            }
             const bool live = gk0 + el < a.K;
             const double rx = geoS[e * 4], sx = geoS[e * 4 + 1], ry = geoS[e * 4 + 2], sy = geoS[e * 4 + 3];
-            float est[4];
-            {
-                auto up = [](uint32_t h) { return oz::trunc32(__hiloint2double((int)h, -1)); };
-                const float rmax = up(maxq[e * 4]), m = up(maxq[e * 4 + 1]), n = up(maxq[e * 4 + 2]),
-                            E = up(maxq[e * 4 + 3]);
-                const float ir = __fdividef(1.f, fmaxf(oz::trunc32(__hiloint2double(minr[e], 0)), 1e-3f * rmax));
-                const float frx = fabsf(oz::trunc32(rx)), fry = fabsf(oz::trunc32(ry)), fsx = fabsf(oz::trunc32(sx)),
-                            fsy = fabsf(oz::trunc32(sy));
-                const float Mr = frx * m + fry * n, Ms = fsx * m + fsy * n, M = fmaxf(Mr, Ms);
-                const float p = g1f * E;
-                est[0] = M;
-                est[1] = M * (m * ir) + fmaxf(frx, fsx) * p;
-                est[2] = M * (n * ir) + fmaxf(fry, fsy) * p;
-                est[3] = M * ((E + p) * ir);
-            }
+            // a density or an energy whose digits lie too far below its row's largest value
+            auto deep = [](double rho, uint32_t rmax, double E, uint32_t emax) {
+                return oz::mag_hi(rho) + ((uint32_t)kRhoDepth << 20) < rmax || oz::mag_hi(E) + ((uint32_t)kEnergyDepth << 20) < emax;
+            };
             // ---- 2. face fluxes
             waitw(bTrFull, phT);
             phT ^= 1;
@@ -654,11 +679,16 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 }
                 if (gi < D::NG4) {
                     double qm[4], qp[4];
-                    load7<32>(tlane + D::T_OWN + 4 * gi, eb1 + ebI, qm);
-                    load7<32>(tlane + D::T_NBR + 4 * gi, e3S[ownrow] + ebI, qp);
+                    load8<32>(tlane + D::T_OWN + 4 * gi, [&](int) { return eb1 + ebI; }, qm);
+                    load8<32>(tlane + D::T_NBR + 4 * gi,
+                              [&](int c) { return oz::row_bound(h3S[ownrow * 3 + min(4 * gi + c, NF - 1) / Nfq]) + ebI; }, qp);
                     transpose4(qm, lane);
                     transpose4(qp, lane);
-                    const double* nr = nrmS + e * 9 + min(pt, NF - 1) / Nfq * 3;
+                    const int f = min(pt, NF - 1) / Nfq;
+                    if (pt < NF && (deep(qm[0], maxq[e * 4], qm[3], maxq[e * 4 + 3]) ||
+                                    deep(qp[0], h3S[e * 12 + f], qp[3], h3S[e * 12 + 9 + f])))
+                        bad = 1u;
+                    const double* nr = nrmS + e * 9 + f * 3;
                     if (a.flux == 1) {
                         roe_flux_fast(g1, nr[0], nr[1], qm, qp, F);
 #pragma unroll
@@ -722,13 +752,16 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
             }
             if (bad) atomicOr(flagS + sub, 1u << el);
             group_sync(sub);
+            uint32_t reach = 0;
 #pragma unroll
             for (int v = 0; v < 4; v++) {
-                // one bit above the estimate for points between the nodes
-                const float b = fminf(2.f * est[v], 1e38f);
+                // one bit above the nodes' largest for points between them
+                const float b = fminf(2.f * __uint_as_float(estS[e * 4 + v]), 1e38f);
                 const int ee = b > 0.f ? (int)(__float_as_uint(b) >> 23) - 127 + 1 + 1022 : 0;
-                eb2[v] = max(oz::row_bound(maxf[e * 4 + v]), ee);
+                const int ef = oz::row_bound(maxf[e * 4 + v]);
+                eb2[v] = max(ef, ee);
                 if (eb2[v] > 1700 || (eb2[v] != 0 && eb2[v] < 300)) bad = 1u;
+                if (ef + kFluxSlack >= eb2[v]) reach |= 1u << v;
             }
             flux_free();
 #pragma unroll 1
@@ -758,7 +791,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 phD ^= 1;
                 umma::fence_after_sync();
                 double q[4];
-                if (p0 < Ng) load7<16>(tlane + D::T_CUB + 4 * cg, eb1 + ebV, q);
+                if (p0 < Ng) load8<16>(tlane + D::T_CUB + 4 * cg, [&](int) { return eb1 + ebV; }, q);
                 umma::fence_before_sync();
                 arrive(bD1read);
                 uint64_t yr[4], ys[4];
@@ -772,11 +805,13 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                     double Fr[4] = {Mr, fma(Mr, u, rx * p), fma(Mr, v, ry * p), Mr * H};
                     double Fs[4] = {Ms, fma(Ms, u, sx * p), fma(Ms, v, sy * p), Ms * H};
                     const bool ok = live && pt < Ng;
+                    if (ok && deep(q[0], maxq[e * 4], q[3], maxq[e * 4 + 3])) bad = 1u;
 #pragma unroll
                     for (int w = 0; w < 4; w++) {
                         if (!ok) Fr[w] = Fs[w] = 0.0;
-                        const uint32_t h = max(oz::mag_hi(Fr[w]), oz::mag_hi(Fs[w]));
-                        if (oz::row_bound(h) > eb2[w]) bad = 1u;
+                        const int b = oz::row_bound(max(oz::mag_hi(Fr[w]), oz::mag_hi(Fs[w])));
+                        if (b > eb2[w]) bad = 1u;
+                        if (b + kFluxSlack >= eb2[w]) reach |= 1u << w;
                         yr[w] = oz::biased(Fr[w], eb2[w]);
                         ys[w] = oz::biased(Fs[w], eb2[w]);
                     }
@@ -794,6 +829,9 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 flux_written();
             }
             if (bad) atomicOr(flagS + sub, 1u << el);
+            reach |= __shfl_xor_sync(0xffffffffu, reach, 8);
+            reach |= __shfl_xor_sync(0xffffffffu, reach, 16);
+            if (jv == 0) atomicOr(reachS + sub, reach << (4 * el));
             // ---- 4. result rows; the update's operands are on their way meanwhile
             const double* other = a.mode == MODE_LSERK ? a.res : a.mode == MODE_SSP2 ? a.qold : nullptr;
 #pragma unroll
@@ -827,7 +865,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
             }
             umma::fence_before_sync();
             group_sync(sub);
-            const uint32_t fl = flagS[sub];
+            uint32_t fl = flagS[sub];
+            const uint32_t far = ~reachS[sub];  // a flux row whose bound its fluxes stayed far below
+#pragma unroll
+            for (int i = 0; i < 8; i++) fl |= ((far >> (4 * i)) & 15u) ? 1u << i : 0u;
             if (t == 0) oa.flags[gk0 >> 3] = (unsigned char)fl;
             // stage update, coalesced
 #pragma unroll

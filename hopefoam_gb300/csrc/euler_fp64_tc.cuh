@@ -29,10 +29,11 @@ struct OzDims {
     static constexpr int NG4 = (NF + 3) / 4;             // groups of 4 face points
     static_assert(NF <= 32 && NT <= 32 && NG4 <= 8, "face operand sizes");
     // operator pieces in the order they are consumed per tile
-    static constexpr int B1F = oz::kSlices * 32 * K1 * 2;   // own nodes -> face points
-    static constexpr int B3 = oz::kSlices * 32 * 32 * 2;    // neighbour face nodes -> face points
-    static constexpr int B1 = oz::kSlices * 16 * K1 * 2;    // own nodes -> one chunk of cubature points
-    static constexpr int B2 = (oz::kSlices + 1) * NP2 * 32 * 2;  // one chunk's fluxes (or the face fluxes) -> nodes
+    // (seven digit blocks and a block of zeros, which starts the eighth accumulator)
+    static constexpr int B1F = (oz::kSlices + 1) * 32 * K1 * 2;   // own nodes -> face points
+    static constexpr int B3 = (oz::kSlices + 1) * 32 * 32 * 2;    // neighbour face nodes -> face points
+    static constexpr int B1 = (oz::kSlices + 1) * 16 * K1 * 2;    // own nodes -> one chunk of cubature points
+    static constexpr int B2 = (oz::kSlices + 1) * NP2 * 32 * 2;   // one chunk's fluxes (or the face fluxes) -> nodes
     // order: own traces, neighbour traces, chunk 0's interpolation, face fluxes,
     // then per chunk c the interpolation of chunk c + 1 and the fluxes of chunk c
     static constexpr int PIECES = 2 * NC + 3;
@@ -50,10 +51,10 @@ struct OzDims {
     static constexpr int cmax(int a, int b) { return a > b ? a : b; }
     static constexpr int SLOT = cmax(cmax(B1F, B3), cmax(B1, B2));
     static constexpr int NSLOT = N == 7 ? 3 : 4;
-    // tensor memory columns: face traces (own, neighbour), then the result
-    // groups over them; the cubature accumulators above
-    static constexpr int T_OWN = 0, T_NBR = 224, T_RES = 0, T_CUB = 384;
-    static_assert(8 * NP2 <= T_CUB, "tensor memory");
+    // tensor memory columns, eight digit groups each: face traces (own, neighbour), then
+    // the result groups and the cubature accumulators over them
+    static constexpr int T_OWN = 0, T_NBR = 256, T_RES = 0, T_CUB = 384;
+    static_assert(8 * NP2 <= T_CUB && T_CUB + 8 * 16 <= 512 && T_NBR + 8 * 32 <= 512, "tensor memory");
     // shared memory
     static constexpr int A1S = 128 * K1 * 2, A2S = 128 * 32 * 2;  // one digit slice of each operand
     static constexpr int OFF_A1 = 0;
@@ -64,17 +65,18 @@ struct OzDims {
     static constexpr int OFF_NRM = OFF_GEO + 32 * 4 * 8;          // [32][3][3] nx, ny, sJ/J
     static constexpr int OFF_CONN = OFF_NRM + 32 * 9 * 8;         // [32][3]
     static constexpr int OFF_MAXQ = OFF_CONN + 32 * 3 * 4;        // [32][4] high word of max |q|
-    static constexpr int OFF_MINR = OFF_MAXQ + 128 * 4;           // [32] high word of min rho
-    static constexpr int OFF_E3 = OFF_MINR + 32 * 4;              // [32][4] bound of the neighbour traces
-    static constexpr int OFF_MAXF = OFF_E3 + 128 * 4;             // [32][4] high word of max |face flux|
+    static constexpr int OFF_H3 = OFF_MAXQ + 128 * 4;             // [32][4][3] the same of a face's neighbour trace
+    static constexpr int OFF_EST = OFF_H3 + 384 * 4;              // [32][4] max |volume flux| at the nodes (FP32)
+    static constexpr int OFF_MAXF = OFF_EST + 128 * 4;            // [32][4] high word of max |face flux|
     static constexpr int OFF_FLAG = OFF_MAXF + 128 * 4;           // [4] elements left to plain FP64
-    static constexpr int OFF_EB = OFF_FLAG + 4 * 4;               // [NP2 + 2] operator bounds
+    static constexpr int OFF_REACH = OFF_FLAG + 4 * 4;            // [4] flux rows that came near their bound, 4 bits an element
+    static constexpr int OFF_EB = OFF_REACH + 4 * 4;              // [NP2 + 2] operator bounds
     static constexpr int OFF_DEAD = OFF_EB + (NP2 + 2) * 4;
     static constexpr int OFF_TMEM = OFF_DEAD + 4;
     static constexpr int OFF_BAR = (OFF_TMEM + 4 + 7) / 8 * 8;    // mbarriers
     static constexpr int SMEM = OFF_BAR + (8 + 2 * NSLOT) * 8;
     static_assert(SMEM <= 232448, "shared memory");
-    static_assert((8 * Ng + 4 * NF) * 8 <= oz::kSlices * 32 * K1 * 2, "scratch of the plain route");
+    static_assert((8 * Ng + 5 * NF) * 8 <= oz::kSlices * 32 * K1 * 2, "scratch of the plain route");
     static_assert(32 * Np * 8 <= oz::kSlices * 2048, "result staging");
 };
 

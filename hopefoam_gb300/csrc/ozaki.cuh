@@ -119,16 +119,22 @@ OZ_HD double from_fixed(int64_t Z, int ex) {
     return m == 0 ? 0.0 : bits_d(q | (s & 0x8000000000000000ull));
 }
 
-// seven accumulators (pairs i + j <= 6), each below 2^22 in magnitude: the
-// base-256 digits of 2^24 hi + lo.  Z = 2^20 hi + lo / 16 is the sum times
-// 2^(58 - EA - EB): it fits 63 bits when sum |b| < 32 2^EB over the row of b.
-OZ_HD double combine7(int d0, int d1, int d2, int d3, int d4, int d5, int d6, int ebab) {
+// Eight accumulators (pairs i + j <= 7) of a nodal product, each below 2^22 in
+// magnitude: the base-256 digits of 2^32 hi + lo.  Z = 2^20 hi + lo / 2^12 is the
+// sum times 2^(58 - EA - EB): it fits 63 bits when sum |b| < 32 2^EB over the row
+// of b.
+OZ_HD double combine_nodal(int d0, int d1, int d2, int d3, int d4, int d5, int d6, int d7, int ebab) {
     const int64_t hi = (int64_t)(d0 * 256 + d1) * 65536 + (d2 * 256 + d3);
-    const int64_t lo = (int64_t)(d4 * 256 + d5) * 256 + d6;
-    return from_fixed((hi << 20) + (lo >> 4), ebab - 2044 - 58);
+    const int64_t lo = (int64_t)(d4 * 256 + d5) * 65536 + (d6 * 256 + d7);
+    return from_fixed((hi << 20) + (lo >> 12), ebab - 2044 - 58);
 }
 
-// eight accumulators (pairs i + j <= 7), each below 2^24; Z is the sum times
+// the same without the last group
+OZ_HD double combine7(int d0, int d1, int d2, int d3, int d4, int d5, int d6, int ebab) {
+    return combine_nodal(d0, d1, d2, d3, d4, d5, d6, 0, ebab);
+}
+
+// eight accumulators of a flux product, each below 2^24; Z is the sum times
 // 2^(56 - EA - EB) and fits when sum |b| < 128 2^EB.  ebab: the biased bounds
 // of both rows added.
 OZ_HD double combine8(const int* d, int ebab) {

@@ -141,3 +141,54 @@ def test_route_changes_between_launches(gpu_lib, N, nx, ny, flux):
     r = orc.euler_rhs(every.reshape(-1), flux=flux).reshape(want[2].shape)
     assert rel_l2(want[2], r) < 1e-10
     ctx.close()
+
+
+@pytest.mark.parametrize("N", range(1, 8))
+@pytest.mark.parametrize("element_dt", [False, True])
+def test_steps_of_plain_route_elements(gpu_lib, N, element_dt):
+    """LSERK4 and SSP-RK2 steps, with one step size and with one per element, where some elements take the plain route
+    (a density 100 times lower at one end) and the others do not: against
+    the same updates written out with the right-hand sides of the library.  Only round-off of the updates differs (ten
+    stages, each a few units in the last place of the state, and of the step folded into the metrics): 1e-14 of the state's norm."""
+    from hopefoam_gb300 import _lib as L
+    from hopefoam_gb300.mesh import periodic_square
+    from oracle.oracle import lserk4_coeffs
+
+    m = periodic_square(5, 7, 10.0, 10.0, perturb=0.1, seed=N)
+    ctx, orc, x, y = _setup(m, N)
+    q = _state(x, y, 10.0)
+    near = np.array([0, 9, 33, 50, 51, 69])
+    rest = np.setdiff1d(np.arange(m.K), near)
+    for k in near:
+        t = (x[k] - x[k].min()) / (x[k].max() - x[k].min())
+        u, v = q[1, k] / q[0, k], q[2, k] / q[0, k]
+        q[0, k] = 1 + 99 * t
+        q[1, k], q[2, k], q[3, k] = q[0, k] * u, q[0, k] * v, 60 + 0.5 * q[0, k] * (u * u + v * v)
+    factor = np.random.default_rng(N).uniform(0.5, 1.5, m.K) if element_dt else np.ones(m.K)
+    assert ctx.lib.dg_set_element_dt(ctx.h, L.dptr(factor) if element_dt else None) == L.DG_OK
+    dt = 1e-4
+    step = dt * factor[None, :, None]
+
+    def rhs(w):
+        ctx.upload(w)
+        return ctx.rhs(flux=N % 2)
+
+    w, res = q.copy(), np.zeros_like(q)
+    a, b = lserk4_coeffs()[:2]
+    for _ in range(2):
+        for ai, bi in zip(a, b):
+            res = ai * res + step * rhs(w)
+            w = w + bi * res
+    ctx.upload(q)
+    ctx.lserk4(dt, 2, flux=N % 2)
+    g = ctx.download()
+    assert rel_l2(g[:, near], w[:, near]) < 1e-14 and rel_l2(g[:, rest], w[:, rest]) < 1e-14
+    w = q.copy()
+    for _ in range(2):
+        w1 = w + step * rhs(w)
+        w = 0.5 * (w + (w1 + step * rhs(w1)))
+    ctx.upload(q)
+    ctx.ssprk2(dt, 2, flux=N % 2)
+    g = ctx.download()
+    assert rel_l2(g[:, near], w[:, near]) < 1e-14 and rel_l2(g[:, rest], w[:, rest]) < 1e-14
+    ctx.close()
