@@ -133,7 +133,7 @@ void restore_streams(dg_batch* b) {
 
 int check_groups(dg_batch* b, int precision) {
     for (size_t g = 0; g < b->groups.size(); g++) {
-        int rc = check_split_status(b->groups[g], precision);
+        int rc = check_stage_status(b->groups[g], precision);
         if (rc) {
             b->err = b->groups[g]->err;
             return rc;

@@ -70,7 +70,17 @@ EulerArgs base_args(dg_ctx* c, int flux) {
     return a;
 }
 
+// The FP64 stage reports bounded-wait timeouts in a mapped host word: what has
+// landed by now (everything, once the stream has been synchronised).
+int fp64_status(dg_ctx* c) {
+    if (!c->oz.h_status || !*(volatile int*)c->oz.h_status) return DG_OK;
+    *(volatile int*)c->oz.h_status = 0;
+    return fail(c, DG_ERR_TIMEOUT, "FP64 stage: tensor-core completion wait timed out");
+}
+
 int run_stage(dg_ctx* c, const EulerArgs& a, int precision) {
+    const int rc = fp64_status(c);  // no step goes on from a stage known to have given up
+    if (rc) return rc;
     cudaError_t e;
     if (precision == DG_PREC_FP64) e = launch_euler_fp64(c->N, a, c->oz, c->stream);
     else if (precision == DG_PREC_SPLIT) e = launch_euler_split(c->N, a, c->split, c->stream);
@@ -79,17 +89,9 @@ int run_stage(dg_ctx* c, const EulerArgs& a, int precision) {
     return DG_OK;
 }
 
-// The FP64 stage reports bounded-wait timeouts in a mapped host word, read
-// once the stream has been synchronised.
-int fp64_status(dg_ctx* c) {
-    if (!c->oz.h_status || !*(volatile int*)c->oz.h_status) return DG_OK;
-    *(volatile int*)c->oz.h_status = 0;
-    return fail(c, DG_ERR_TIMEOUT, "FP64 stage: tensor-core completion wait timed out");
-}
-
 // The split kernel reports bounded-wait timeouts in a device status word.
-int split_status_impl(dg_ctx* c, int precision) {
-    if (precision != DG_PREC_SPLIT) return DG_OK;
+int stage_status_impl(dg_ctx* c, int precision) {
+    if (precision != DG_PREC_SPLIT) return fp64_status(c);
     int st = 0;
     DG_CUDA(c, cudaMemcpyAsync(&st, c->split.d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -111,7 +113,8 @@ int run_args_impl(dg_ctx* c, int flux, int precision) {
 
 }  // namespace
 
-int check_split_status(dg_ctx* c, int precision) { return split_status_impl(c, precision); }
+int check_stage_status(dg_ctx* c, int precision) { return stage_status_impl(c, precision); }
+int check_fp64_status(dg_ctx* c) { return fp64_status(c); }
 int check_run_args(dg_ctx* c, int flux, int precision) { return run_args_impl(c, flux, precision); }
 
 int euler_stage_mode(dg_ctx* c, const double* qin, double* qout, const double* qold, int mode, double dt, int flux,
@@ -340,6 +343,8 @@ int dg_upload_state_device(dg_ctx* c, const double* q_dev) {
 
 int dg_download_state_device(dg_ctx* c, double* q_dev) {
     if (!c || !q_dev) return DG_ERR_ARG;
+    const int rc = fp64_status(c);
+    if (rc) return rc;
     cudaError_t e = launch_to_reference(c->d_q[c->cur], q_dev, c->d_ring, c->K, c->Np, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "to_reference");
     return DG_OK;
@@ -386,7 +391,7 @@ int dg_euler_rhs(dg_ctx* c, int flux, int precision, double* rhs_host) {
     if ((rc = refresh_boundary_traces(c, a.qin))) return rc;
     rc = run_stage(c, a, precision);
     if (rc) return rc;
-    rc = check_split_status(c, precision);
+    rc = check_stage_status(c, precision);
     if (rc) return rc;
     cudaError_t e = launch_to_reference(a.rhs, c->d_stage, c->d_ring, c->K, c->Np, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "to_reference");
@@ -409,7 +414,7 @@ int dg_euler_rhs_device(dg_ctx* c, int flux, int precision, double* rhs_dev) {
     if (rc) return rc;
     cudaError_t e = launch_to_reference(a.rhs, rhs_dev, c->d_ring, c->K, c->Np, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "to_reference");
-    return DG_OK;
+    return fp64_status(c);
 }
 
 int dg_forward_euler_stage(dg_ctx* c, double dt, int flux, int precision) {
@@ -425,13 +430,13 @@ int dg_forward_euler_stage(dg_ctx* c, double dt, int flux, int precision) {
     rc = run_stage(c, a, precision);
     if (rc) return rc;
     c->cur ^= 1;
-    return DG_OK;
+    return fp64_status(c);
 }
 
 int dg_sync(dg_ctx* c) {
     if (!c) return DG_ERR_ARG;
     if (c->split.ready) {
-        const int rc = check_split_status(c, DG_PREC_SPLIT);
+        const int rc = check_stage_status(c, DG_PREC_SPLIT);
         if (rc) return rc;
     }
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -458,7 +463,7 @@ int dg_lserk4_step(dg_ctx* c, double dt, int nsteps, int flux, int precision) {
             if (rc) return rc;
             c->cur ^= 1;
         }
-    return check_split_status(c, precision);
+    return check_stage_status(c, precision);
 }
 
 int dg_ssprk2_step(dg_ctx* c, double dt, int nsteps, int flux, int precision) {
@@ -484,7 +489,7 @@ int dg_ssprk2_step(dg_ctx* c, double dt, int nsteps, int flux, int precision) {
         rc = run_stage(c, a, precision);
         if (rc) return rc;
     }
-    return check_split_status(c, precision);
+    return check_stage_status(c, precision);
 }
 
 int dg_cfl_dt(dg_ctx* c, double cfl, double* dt) {

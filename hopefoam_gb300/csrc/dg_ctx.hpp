@@ -86,8 +86,10 @@ int lserk_stage_args(dg_ctx* c, double dt, int stage, int flux, dgk::EulerArgs* 
 bool has_dynamic_traces(const dg_ctx* c);
 // validates flux / precision / boundary state for stepping
 int check_run_args(dg_ctx* c, int flux, int precision);
-// reads and clears the split kernel's timeout flag (synchronises c->stream)
-int check_split_status(dg_ctx* c, int precision);
+// reads and clears the stage's timeout report: the split kernel's flag
+// (synchronises c->stream), or what has landed of the FP64 kernel's
+int check_stage_status(dg_ctx* c, int precision);
+int check_fp64_status(dg_ctx* c);
 // one Euler stage kernel (mode: StageMode) from qin into qout with the given
 // boundary traces (null: the context's)
 int euler_stage_mode(dg_ctx* c, const double* qin, double* qout, const double* qold, int mode, double dt, int flux,

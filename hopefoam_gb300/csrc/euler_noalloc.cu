@@ -71,6 +71,8 @@ extern "C" int dg_euler_rhs_noalloc(dg_ctx* c, const double* q_dev, double* rhs_
                      "dg_euler_rhs_noalloc: 4*K*Np = " + std::to_string(n) +
                          " exceeds the fixed scratch of 524288 values; use dg_euler_rhs");
     if (c->nb > 0 && !c->btrace_set) return nfail(c, DG_ERR_ARG, "boundary traces not set");
+    const int landed = check_fp64_status(c);
+    if (landed) return landed;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nfail(c, DG_ERR_CUDA, "cudaGetDevice failed");

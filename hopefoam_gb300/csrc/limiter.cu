@@ -693,7 +693,7 @@ int dg_limited_ssprk2_step(dg_ctx* c, double dt, const double* bdata_host, int f
     // the context's traces: the state's boundary field
     if (nb > 0) LIM_CUDA(c, cudaMemcpyAsync(c->d_btrace, s->bq, nbv * sizeof(double), cudaMemcpyDeviceToDevice, st));
     c->btrace_set = true;
-    return check_split_status(c, precision);
+    return check_stage_status(c, precision);
 }
 
 }  // extern "C"

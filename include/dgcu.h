@@ -147,7 +147,8 @@ int dg_euler_rhs_device(dg_ctx* ctx, int flux, int precision, double* rhs_dev);
 int dg_forward_euler_stage(dg_ctx* ctx, double dt, int flux, int precision);
 
 /* Waits for the context's queued work; reports a bounded-wait timeout of a
- * split-precision kernel queued by a stream-ordered call (DG_ERR_TIMEOUT). */
+ * kernel queued by a stream-ordered call (DG_ERR_TIMEOUT).  Calls that do not
+ * wait report one of an FP64 stage that has landed by then, once. */
 int dg_sync(dg_ctx* ctx);
 
 /* nsteps low-storage RK4 steps (5 stages each, coefficients of
