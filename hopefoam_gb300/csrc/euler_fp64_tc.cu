@@ -468,13 +468,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 }
             // everything issued ends before the CTA does
             umma::commit(bFin);
-            umma::mbar_wait(bFin, 0, kWaitLimit);
-            if (*dead) {
+            if (!umma::mbar_wait(bFin, 0, kWaitLimit)) *dead = 1;
+            if (*dead)
                 for (long long n = nuse; n < nload; n++)
                     umma::mbar_wait(bFull + (int)(n % D::NSLOT), (uint32_t)((n / D::NSLOT) & 1), kWaitLimit);
-                *reinterpret_cast<volatile int*>(oa.status) = 1;
-                __threadfence_system();
-            }
         }
         __syncwarp();
     } else if ((warp & 3) < oa.groups) {
@@ -895,6 +892,11 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
     }
     umma::fence_before_sync();
     __syncthreads();
+    // whoever gave up, and whenever
+    if (threadIdx.x == 0 && *dead) {
+        *reinterpret_cast<volatile int*>(oa.status) = 1;
+        __threadfence_system();
+    }
     if (warp == 16) {
         umma::fence_after_sync();
         umma::tmem_relinquish();

@@ -717,11 +717,10 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             }
             // everything issued ends before the CTA does
             umma::commit(bfin);
-            umma::mbar_wait(bfin, 0, kWaitLimit);
+            if (!umma::mbar_wait(bfin, 0, kWaitLimit)) *dead = 1;
             if (*dead) {
                 if (nq) umma::mbar_wait(bq, (uint32_t)(nq - 1) & 1u, kWaitLimit);
                 for (int q = max(0, nsl - 2); q < nsl; q++) umma::mbar_wait(bfull + (q & 1), (uint32_t)(q >> 1) & 1u, kWaitLimit);
-                atomicExch(sa.status, 1);
             }
         }
         __syncwarp();
@@ -994,6 +993,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
     }
     umma::fence_before_sync();
     __syncthreads();
+    if (tid == 0 && *dead) atomicExch(sa.status, 1);  // whoever gave up, and whenever
     if (warp == 16) umma::tmem_dealloc(tmem, S::TMEM_COLS);
 }
 
