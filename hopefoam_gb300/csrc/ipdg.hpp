@@ -82,6 +82,7 @@ struct PcgScalars {
     int it;         // iterations taken
     unsigned int counter;  // arrival counter of the grid-wide sums
     int gaveup;            // a bounded wait of the cooperative iterations gave up (ipdg_persist.cu)
+    int skip;              // multilevel mode: done as this iteration's first kernel of the correction saw it
 };
 
 struct ApplyPcg {

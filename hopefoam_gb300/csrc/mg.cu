@@ -403,12 +403,17 @@ cudaError_t launch_mg_dense(const MgDenseLevel* lv, int count, double* work, int
 // building the levels 95 -> 30 ms there (rows merged in place instead of
 // sorted triplets, a vectorised inverse, one upload).
 
-// r1 = P^T r; eight lanes per vertex, one incident element corner each,
+// r1 = P^T r, and for the collect kernel whether this iteration still runs (S
+// is null outside the iterations); eight lanes per vertex, one incident element corner each,
 // summed in a fixed order
 __global__ void __launch_bounds__(256) mg_restrict_dg_kernel(MgLevels m, const double* __restrict__ r,
-                                                             double* __restrict__ r1, const int* __restrict__ done) {
+                                                             double* __restrict__ r1, PcgScalars* S) {
     dependency_wait();
-    if (done && *done) return;
+    if (S) {
+        const int done = S->done;
+        if (blockIdx.x == 0 && threadIdx.x == 0) S->skip = done;
+        if (done) return;
+    }
     __shared__ double lam[36 * 3];
     for (int i = threadIdx.x; i < 3 * m.Np; i += blockDim.x) lam[i] = m.lam[i];
     __syncthreads();
@@ -515,7 +520,7 @@ __global__ void __launch_bounds__(RowDims<NP>::THREADS) mg_collect_kernel(MgLeve
                                                                           double* part) {
     using R = RowDims<NP>;
     dependency_wait();
-    if (mode == 3 && S->done) return;
+    if (mode == 3 && S->skip) return;  // not S->done: this launch's own blocks may set that while others start
     int e, i;
     row_of<NP>(e, i);
     const bool lane_ok = e < R::EB;
@@ -589,7 +594,7 @@ cudaError_t launch_mg_correction(const MgLevels& m, const double* r, const doubl
                                  bool zb_summed, PcgScalars* S, double* part, int grid, cudaStream_t s) {
     const int L = m.nl;
     const int* done = mode == 3 ? &S->done : nullptr;  // a stopped iteration leaves every vector as it is
-    cudaError_t e = launch_dependent(mg_restrict_dg_kernel, nb256(8 * m.lv[0].n), 256, s, m, r, m.lv[0].r, done);
+    cudaError_t e = launch_dependent(mg_restrict_dg_kernel, nb256(8 * m.lv[0].n), 256, s, m, r, m.lv[0].r, mode == 3 ? S : nullptr);
     for (int l = 0; l + 1 < L && e == cudaSuccess; l++) {
         const int nc = m.lv[l + 1].n, bblocks = (int)nb256(kDownLanes * nc);
         e = launch_dependent(mg_down_kernel, bblocks + nb256(kMLanes * m.lv[l].n), 256, s, m.lv[l], nc, bblocks, m.lv[l].r,
