@@ -39,6 +39,7 @@ struct IpdgState {
     bool sb_ready = false, sb_none = false;  // current; no memory for them
     float* d_sblocks32 = nullptr;  // FP32 rows of the cooperative iterations of small problems
     bool sb32_ready = false;
+    bool coop_none = false;  // the device does not hold the cooperative launch at once
     double* d_corner = nullptr;
     // a batch of PCG iterations as a CUDA graph, and the arguments of its launches (run_cg)
     cudaGraphExec_t cg_graph = nullptr;
@@ -111,6 +112,14 @@ int ialloc(dg_ctx* c, IpdgState* s, T** p, size_t n) {
     }
     s->allocs.push_back((void*)*p);
     return DG_OK;
+}
+
+template <typename T>
+void ifree(IpdgState* s, T** p) {
+    if (!*p) return;
+    s->allocs.erase(std::find(s->allocs.begin(), s->allocs.end(), (void*)*p));
+    cudaFree(*p);
+    *p = nullptr;
 }
 
 template <typename T>
@@ -222,13 +231,16 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
     // small problems: cooperative launches of many iterations (in FP32 arithmetic
     // as many as between two residual replacements)
     const void* prows = nullptr;
-    if (persist_fits(s->args, v, fp32)) {
+    if (!s->coop_none && persist_fits(s->args, v, fp32)) {
         const int rcp = persist_rows(c, v, fp32, &prows);
         if (rcp) return rcp;
     }
     bool persist = prows != nullptr;
-    const int CHECK = persist ? (refresh > 0 ? 16 * refresh : 256) : 16;
-    if (persist && refresh > 0) refresh = 1;
+    int CHECK = 16, every = refresh;  // iterations between two looks at S, and looks between two replacements
+    if (persist) {
+        CHECK = refresh > 0 ? 16 * refresh : 256;
+        every = refresh > 0 ? 1 : 0;
+    }
     int checks = 0;
     *stop = 0;
     *iters = 0;
@@ -309,13 +321,23 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
         return cudaSuccess;
     };
     while (h.it < limit) {
-        const int batch = std::min(CHECK, limit - h.it);
+        int batch = std::min(CHECK, limit - h.it);
         if (persist) {
             const cudaError_t e = launch_pcg_persistent(s->args, v, fp32, prows, s->d_corner, s->d_slots, &s->exchanges,
                                                         h.it & 1, batch, c->stream);
-            if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device has (a partition of it)
+            if (e == cudaErrorCooperativeLaunchTooLarge) {
+                // fewer SMs than the device has (a partition of it): the general iterations, as
+                // if they had been taken from the start, for this operator's solves from now on
                 (void)cudaGetLastError();
                 persist = false;
+                s->coop_none = true;
+                CHECK = 16;
+                every = refresh;
+                batch = std::min(CHECK, limit - h.it);
+                ifree(s, &s->d_sblocks32);
+                ifree(s, &s->d_corner);
+                ifree(s, &s->d_slots);
+                s->sb32_ready = false;
             } else {
                 IP_CUDA(c, e);
             }
@@ -337,7 +359,7 @@ int run_cg(dg_ctx* c, const PcgVecs& v, bool fp32, double tol2, int limit, const
             }
         }
         const bool claim = h.done == 1;
-        const bool periodic = refresh > 0 && checks % refresh == 0;
+        const bool periodic = every > 0 && checks % every == 0;
         if (!b || (!claim && !periodic)) {
             if (claim) break;
             continue;
