@@ -459,7 +459,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
 #pragma unroll
                     for (int v = 0; v < 4; v++) {
                         float hi, lo;
-                        umma::split_tf32(-fsc * F[sl][v], hi, lo);
+                        umma::split_tf32(__fmul_rn(-0.5f * fsc, F[sl][v]), hi, lo);
                         const uint32_t off = umma::kmajor_offset(g2row(e, v), f * Nfq + g, NF) >> 2;
                         sAF[off] = hi;
                         sAF[off + LO_AF / 4] = lo;
@@ -556,7 +556,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
 #pragma unroll
                     for (int v = 0; v < 4; v++) {
                         float hi, lo;
-                        umma::split_tf32(-fsc * F[v], hi, lo);
+                        umma::split_tf32(__fmul_rn(-0.5f * fsc, F[v]), hi, lo);
                         const uint32_t off = umma::kmajor_offset(g2row(e, v), f * Nfq + i, NF) >> 2;
                         sAF[off] = hi;
                         sAF[off + LO_AF / 4] = lo;
@@ -810,8 +810,8 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 flux_delta(bref, dq, d, fx, fy);
 #pragma unroll
                 for (int v = 0; v < 4; v++) {
-                    fr[v] = rx * fx[v] + ry * fy[v];
-                    fs[v] = sx * fx[v] + sy * fy[v];
+                    fr[v] = fmaf(ry, fy[v], __fmul_rn(rx, fx[v]));
+                    fs[v] = fmaf(sy, fy[v], __fmul_rn(sx, fx[v]));
                 }
             } else {
 #pragma unroll

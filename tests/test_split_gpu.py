@@ -275,3 +275,35 @@ def test_split_tiles_per_block(gpu_lib, N, nx, ny):
             s.append(ctx.download())
         assert np.array_equal(s[0], s[1])
     ctx.close()
+
+
+@pytest.mark.parametrize("N", range(1, 8))
+@pytest.mark.parametrize("flux", [0, 1])
+def test_split_results_do_not_depend_on_the_place_of_a_tile(gpu_lib, N, flux):
+    """Five copies of a mesh of 150 tiles in one context, so that a copy's tiles are the first, the second, ... of their
+    blocks: every copy has the bits of the mesh alone, the right-hand side and the state after steps of both schemes."""
+    from hopefoam_gb300 import _lib as L
+    from hopefoam_gb300 import euler
+    from hopefoam_gb300.batch import concat_meshes
+    from hopefoam_gb300.mesh import periodic_square
+
+    m = periodic_square(50, 48, 10.0, 10.0, perturb=0.1, seed=N)
+    ops = euler.reference_operators(N)
+    q = euler.isentropic_vortex(*euler.node_coords(m, ops["r"], ops["s"]), x0=5.0, y0=5.0, uinf=0.7, vinf=0.2)
+
+    def results(mesh, state):
+        ctx = euler.EulerContext(mesh, N)
+        ctx.upload(state)
+        out = [ctx.rhs(flux=flux, precision=L.DG_PREC_SPLIT)]
+        ctx.lserk4(1e-3, 2, flux=flux, precision=L.DG_PREC_SPLIT)
+        out.append(ctx.download())
+        ctx.ssprk2(1e-3, 1, flux=flux, precision=L.DG_PREC_SPLIT)
+        out.append(ctx.download())
+        ctx.close()
+        return out
+
+    alone = results(m, q)
+    copies = results(concat_meshes([m] * 5), np.concatenate([q] * 5, axis=1))
+    for a, c in zip(alone, copies):
+        for j in range(5):
+            assert np.array_equal(c[:, j * m.K:(j + 1) * m.K], a), j
