@@ -131,6 +131,21 @@ void restore_streams(dg_batch* b) {
     for (size_t g = 0; g < b->groups.size(); g++) b->groups[g]->stream = b->saved[g];
 }
 
+// SMs for each group in proportion to its weight, at least one each; their sum
+// is the device's where it has as many as groups
+std::vector<int> sm_shares(int sms, const std::vector<double>& weight) {
+    const int G = (int)weight.size();
+    double tot = 0;
+    for (double w : weight) tot += w;
+    std::vector<int> n(G);
+    int used = 0;
+    for (int g = 0; g < G; g++) used += n[g] = std::max(1, (int)std::floor(sms * weight[g] / tot));
+    for (int g = 0; used < sms; g = (g + 1) % G, used++) n[g]++;
+    // groups raised to one SM: their surplus from the largest
+    for (; used > sms && used > G; used--) --*std::max_element(n.begin(), n.end());
+    return n;
+}
+
 int check_groups(dg_batch* b, int precision) {
     for (size_t g = 0; g < b->groups.size(); g++) {
         int rc = check_stage_status(b->groups[g], precision);
@@ -142,8 +157,22 @@ int check_groups(dg_batch* b, int precision) {
     return DG_OK;
 }
 
-// milliseconds for nsteps (events on the main stream), state advanced
-int time_steps(dg_batch* b, double dt, int nsteps, int flux, int precision, float* ms) {
+// milliseconds for nsteps (events on the main stream), state advanced; side by
+// side also each group's own (group_ms)
+int time_steps(dg_batch* b, double dt, int nsteps, int flux, int precision, float* ms, std::vector<float>* group_ms = nullptr) {
+    const size_t G = group_ms ? b->groups.size() : 0;
+    std::vector<cudaEvent_t> ends;
+    struct Ends {
+        std::vector<cudaEvent_t>& v;
+        ~Ends() {
+            for (cudaEvent_t e : v) cudaEventDestroy(e);
+        }
+    } guard{ends};
+    for (size_t g = 0; g < G; g++) {
+        cudaEvent_t e;
+        B_CUDA(b, cudaEventCreate(&e));
+        ends.push_back(e);
+    }
     cudaEvent_t e0, e1;
     B_CUDA(b, cudaEventCreate(&e0));
     B_CUDA(b, cudaEventCreate(&e1));
@@ -151,9 +180,14 @@ int time_steps(dg_batch* b, double dt, int nsteps, int flux, int precision, floa
     int rc = issue_steps(b, dt, nsteps, flux, precision);
     restore_streams(b);
     if (!rc) {
+        for (size_t g = 0; g < G; g++) B_CUDA(b, cudaEventRecord(ends[g], b->streams[g]));
         B_CUDA(b, cudaEventRecord(e1, b->main));
         B_CUDA(b, cudaEventSynchronize(e1));
         B_CUDA(b, cudaEventElapsedTime(ms, e0, e1));
+        for (size_t g = 0; g < G; g++) {
+            B_CUDA(b, cudaEventSynchronize(ends[g]));
+            B_CUDA(b, cudaEventElapsedTime(&(*group_ms)[g], e0, ends[g]));
+        }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -287,19 +321,24 @@ int dg_batch_tune(dg_batch* b, double dt, int flux, int precision, int steps_per
     }
     std::vector<int> budget(G, b->sms);
     if (!rc && G > 1) {
-        // side by side: SMs split in proportion to each group's time alone
-        double tot = 0;
-        for (float t : t_alone) tot += t;
-        int used = 0;
-        for (int g = 0; g < G; g++) {
-            budget[g] = std::max(1, (int)std::floor(b->sms * t_alone[g] / tot));
-            used += budget[g];
-        }
-        for (int g = 0; used < b->sms; g = (g + 1) % G, used++) budget[g]++;
-        b->sm_budget = budget;
+        // side by side: SMs split in proportion to each group's time alone, then to what each
+        // needed beside the others.  The kernels of several orders slow each other down, the
+        // small orders most (five orders, 512 cases: 37 % at N = 3, 13 % at N = 6), so the first split leaves
+        // SMs idle: 39.5 ms a step, 37.0 after; one launch per stage, on the same shares, 36.6 and 35.1.
+        std::vector<double> weight(t_alone.begin(), t_alone.end());
+        std::vector<float> tg(G, 0.f);
         b->concurrent = 1;
-        apply_shape(b);
-        rc = time_steps(b, dt, steps_per_trial, flux, precision, &t_conc);
+        for (int trial = 0; trial < 3 && !rc; trial++) {
+            b->sm_budget = sm_shares(b->sms, weight);
+            if (trial && b->sm_budget == budget) break;
+            apply_shape(b);
+            float t = 0;
+            rc = time_steps(b, dt, steps_per_trial, flux, precision, &t, &tg);
+            if (rc || t >= t_conc) break;
+            t_conc = t;
+            budget = b->sm_budget;
+            for (int g = 0; g < G; g++) weight[g] = (double)tg[g] * budget[g];
+        }
     }
     float t_fused = 1e30f;
     if (!rc && fused_ok(b, precision)) {
@@ -345,18 +384,15 @@ int dg_batch_set_schedule(dg_batch* b, int schedule, int precision) {
         return bfail(b, DG_ERR_UNSUPPORTED, "one launch per stage needs split precision, orders <= 6, <= 8 groups");
     const int G = (int)b->groups.size();
     if (schedule != 0 && b->sm_budget.size() == (size_t)G) {
-        // SM shares in proportion to the groups' element-node counts unless tuned before
+        // SM shares in proportion to the groups' work unless tuned before.  Beside others
+        // an element costs about (Np + 12) of one unit (7.2, 9.9, 11.6, 14.2, 17 ns a step on one of 152 SMs'
+        // share at N = 2 .. 6); by element-node counts the small orders came out last
         int sum = 0;
         for (int v : b->sm_budget) sum += v;
         if (sum != b->sms) {
-            double tot = 0;
-            for (const dg_ctx* c : b->groups) tot += (double)c->K * c->Np;
-            int used = 0;
-            for (int g = 0; g < G; g++) {
-                b->sm_budget[g] = std::max(1, (int)std::floor(b->sms * (double)b->groups[g]->K * b->groups[g]->Np / tot));
-                used += b->sm_budget[g];
-            }
-            for (int g = 0; used < b->sms; g = (g + 1) % G, used++) b->sm_budget[g]++;
+            std::vector<double> weight;
+            for (const dg_ctx* c : b->groups) weight.push_back((double)c->K * (c->Np + 12));
+            b->sm_budget = sm_shares(b->sms, weight);
         }
     }
     drop_graph(b);

@@ -145,3 +145,39 @@ def test_batch_conservation_full_size(gpu_lib):
         worst = max(worst, float(np.max(np.abs(t1 - t0)) / np.max(np.abs(t0))))
     print("512 cases, 10 split steps: worst relative drift of a case's totals %.2e" % worst)
     assert worst < 5e-10
+
+
+@pytest.mark.parametrize("kmax,n", [(300, 7), (6000, 12)])
+def test_sm_shares(gpu_lib, kmax, n):
+    """The SM shares of the groups, untuned and tuned: at least one each and the device's SMs in all, and no effect on
+    the states."""
+    import ctypes
+
+    import torch
+
+    from hopefoam_gb300 import _lib as L
+    from hopefoam_gb300.batch import EulerBatch, batch_cases
+
+    def share(b, g):
+        v = [ctypes.c_int32() for _ in range(3)]
+        assert b.lib.dg_batch_get_shape(b.h, g, *[ctypes.byref(x) for x in v]) == L.DG_OK
+        return v[1].value
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    cases = batch_cases(n=n, seed=1, orders=(2, 3, 5, 6), kmin=60, kmax=kmax)
+    want = None
+    for tuned in (False, True):
+        for schedule in (0, 1, 2):
+            b = EulerBatch(cases)
+            if tuned:
+                b.tune(precision=L.DG_PREC_SPLIT, steps_per_trial=1)
+            b.set_schedule(schedule, precision=L.DG_PREC_SPLIT)
+            if schedule:
+                shares = [share(b, g) for g in range(len(b.groups))]
+                assert min(shares) >= 1 and sum(shares) == sms
+            b.run(2, precision=L.DG_PREC_SPLIT)
+            got = b.states()
+            b.close()
+            if want is None:
+                want = got
+            assert all(np.array_equal(x, y) for x, y in zip(got, want))
