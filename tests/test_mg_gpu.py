@@ -150,3 +150,30 @@ def test_repeated_solves_follow_the_operator(gpu_lib, N, n_interior):
             fresh[mass, pc, precision] = p2.solve(b, rtol=1e-10, pc=pc, precision=precision)[0]
             p2.ctx.close()
         assert np.array_equal(x, fresh[mass, pc, precision])
+
+
+@pytest.mark.parametrize("N,n_interior,precision", [(3, 300, 0), (3, 300, 1), (2, 3000, 0), (4, 6000, 1)])
+def test_boundary_types_change_between_solves(gpu_lib, N, n_interior, precision):
+    """Boundary types and the Helmholtz coefficient changed after solves, when the assembled rows, the levels and a batch of
+    iterations are kept already (small problems in one launch, larger ones in batches): the bits of a fresh solver."""
+    from hopefoam_gb300 import _lib as L
+
+    ps, b = _solver(n_interior, N, 1.0)
+    nb = ps.ctx.n_bfaces
+    types = [np.zeros(nb, np.int32), (np.arange(nb) % 3 == 0).astype(np.int32), np.where(np.arange(nb) % 2, 2, 0).astype(np.int32)]
+
+    def prepare(p, t, mass):
+        assert p.ctx.lib.dg_ipdg_set_boundary_types(p.ctx.h, L.iptr(types[t])) == L.DG_OK
+        assert p.ctx.lib.dg_ipdg_set_mass(p.ctx.h, mass) == L.DG_OK
+
+    for t, mass, pc in ((0, 0.0, "MULTILEVEL"), (1, 0.0, "MULTILEVEL"), (1, 20.0, "BLOCK_JACOBI"), (2, 20.0, "MULTILEVEL"),
+                        (0, 0.0, "BLOCK_JACOBI"), (0, 0.0, "MULTILEVEL")):
+        prepare(ps, t, mass)
+        kw = dict(rtol=1e-8, maxit=20000, pc=getattr(L, "DG_PC_" + pc), precision=precision)
+        x, st = ps.solve(b, **kw)
+        fresh, _ = _solver(n_interior, N, 1.0)
+        prepare(fresh, t, mass)
+        y, st2 = fresh.solve(b, **kw)
+        fresh.ctx.close()
+        assert st["iterations"] == st2["iterations"] and np.array_equal(x, y), (t, mass, pc)
+    ps.ctx.close()
