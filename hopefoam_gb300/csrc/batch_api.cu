@@ -26,7 +26,6 @@ struct dg_batch {
     // streams; 2: every stage of every group in one launch (the mixed-order
     // kernel, each group on its share of the SMs)
     int concurrent = 0;
-    std::vector<int> ctas_per_sm;    // per group
     std::vector<int> sm_budget;      // per group (concurrent schedule)
     // captured graph
     cudaGraphExec_t exec = nullptr;
@@ -51,10 +50,7 @@ int bfail(dg_batch* b, int code, const std::string& m) {
     } while (0)
 
 void apply_shape(dg_batch* b) {
-    for (size_t g = 0; g < b->groups.size(); g++) {
-        b->groups[g]->split.ctas_per_sm = b->ctas_per_sm[g];
-        b->groups[g]->split.sm_budget = b->concurrent == 1 ? b->sm_budget[g] : 0;
-    }
+    for (size_t g = 0; g < b->groups.size(); g++) b->groups[g]->split.sm_budget = b->concurrent == 1 ? b->sm_budget[g] : 0;
 }
 
 void drop_graph(dg_batch* b) {
@@ -64,12 +60,12 @@ void drop_graph(dg_batch* b) {
 }
 
 // the mixed-order single launch per stage needs split precision, orders
-// 1..6 on the pipelined body, 16-byte aligned states and no per-stage
+// 1..6, 16-byte aligned states and no per-stage
 // boundary-trace refresh
 bool fused_ok(const dg_batch* b, int precision) {
     if (precision != DG_PREC_SPLIT || b->groups.size() > (size_t)dgk::SplitBatchArgs::MAXG) return false;
     for (const dg_ctx* c : b->groups) {
-        if (c->N > 6 || !c->split.ready || c->split.variant == dgk::SplitPlan::CLASSIC) return false;
+        if (c->N > 6 || !c->split.ready) return false;
         if (has_dynamic_traces(c)) return false;
         if ((reinterpret_cast<uintptr_t>(c->d_q[0]) & 15u) || (reinterpret_cast<uintptr_t>(c->d_q[1]) & 15u))
             return false;
@@ -229,7 +225,6 @@ int dg_batch_create(dg_ctx* const* groups, int n_groups, dg_batch** out) {
             b->joins.push_back(e);
         }
     }
-    b->ctas_per_sm.assign(n_groups, 1);
     b->sm_budget.assign(n_groups, b->sms);
     if (!ok) {
         dg_batch_destroy(b);
@@ -244,10 +239,7 @@ int dg_batch_destroy(dg_batch* b) {
     if (b->main) cudaStreamSynchronize(b->main);
     drop_graph(b);
     restore_streams(b);
-    for (dg_ctx* c : b->groups) {
-        c->split.ctas_per_sm = 1;
-        c->split.sm_budget = 0;
-    }
+    for (dg_ctx* c : b->groups) c->split.sm_budget = 0;
     for (cudaStream_t s : b->streams) cudaStreamDestroy(s);
     for (cudaEvent_t e : b->joins) cudaEventDestroy(e);
     if (b->fork) cudaEventDestroy(b->fork);
@@ -277,44 +269,30 @@ int dg_batch_tune(dg_batch* b, double dt, int flux, int precision, int steps_per
     }
     // work weights: one stage of each group alone on the whole GPU
     b->concurrent = 0;
-    std::vector<int> cps_best(G, 1);
     std::vector<float> t_alone(G, 0.f);
     int rc = DG_OK;
     for (int g = 0; g < G && !rc; g++) {
         dg_ctx* c = b->groups[g];
-        // CTAs per SM: 1, and 2 where two CTAs fit (split kernel, small orders)
-        const int max_cps = (precision == DG_PREC_SPLIT && c->N <= 2) ? 2 : 1;
-        float best = 1e30f;
-        for (int cps = 1; cps <= max_cps && !rc; cps++) {
-            std::vector<dg_ctx*> only{c};
-            dg_batch one;  // a one-group view sharing the streams
-            one.groups = only;
-            one.saved = {c->stream};
-            one.main = b->main;
-            one.fork = b->fork;
-            one.joins = {b->joins[g]};
-            one.streams = {b->streams[g]};
-            one.concurrent = 0;
-            one.ctas_per_sm = {cps};
-            one.sm_budget = {b->sms};
-            apply_shape(&one);
-            float ms = 0;
-            rc = time_steps(&one, dt, 1, flux, precision, &ms);  // warm
-            if (!rc) rc = time_steps(&one, dt, steps_per_trial, flux, precision, &ms);
-            one.main = nullptr;  // not owned
-            one.fork = nullptr;
-            one.joins.clear();
-            one.streams.clear();
-            if (!rc && ms < best) {
-                best = ms;
-                cps_best[g] = cps;
-            }
-        }
-        t_alone[g] = best;
+        std::vector<dg_ctx*> only{c};
+        dg_batch one;  // a one-group view sharing the streams
+        one.groups = only;
+        one.saved = {c->stream};
+        one.main = b->main;
+        one.fork = b->fork;
+        one.joins = {b->joins[g]};
+        one.streams = {b->streams[g]};
+        one.concurrent = 0;
+        one.sm_budget = {b->sms};
+        apply_shape(&one);
+        rc = time_steps(&one, dt, 1, flux, precision, &t_alone[g]);  // warm
+        if (!rc) rc = time_steps(&one, dt, steps_per_trial, flux, precision, &t_alone[g]);
+        one.main = nullptr;  // not owned
+        one.fork = nullptr;
+        one.joins.clear();
+        one.streams.clear();
     }
     float t_seq = 0, t_conc = 1e30f;
     if (!rc) {
-        b->ctas_per_sm = cps_best;
         b->concurrent = 0;
         apply_shape(b);
         rc = time_steps(b, dt, steps_per_trial, flux, precision, &t_seq);
@@ -403,7 +381,7 @@ int dg_batch_set_schedule(dg_batch* b, int schedule, int precision) {
 
 int dg_batch_get_shape(const dg_batch* b, int group, int* ctas_per_sm, int* sm_budget, int* concurrent) {
     if (!b || group < 0 || group >= (int)b->groups.size()) return DG_ERR_ARG;
-    if (ctas_per_sm) *ctas_per_sm = b->ctas_per_sm[group];
+    if (ctas_per_sm) *ctas_per_sm = 1;  // a CTA takes an SM's registers
     if (sm_budget) *sm_budget = b->concurrent ? b->sm_budget[group] : b->sms;  // schedules 1 and 2: its share
     if (concurrent) *concurrent = b->concurrent;
     return DG_OK;

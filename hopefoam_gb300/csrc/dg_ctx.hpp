@@ -22,12 +22,7 @@ struct SplitPlan {
     size_t if32_offset = 0;   // FP32 face interpolation table, in floats
     int* d_status = nullptr;  // bounded-wait timeout flag
     float* d_res32 = nullptr; // FP32 low-storage RK register
-    int ctas_per_sm = 1;      // launch shape (persistent grid = SMs used x CTAs per SM)
-    int sm_budget = 0;        // SMs the grid is sized for (0: all)
-    // kernel variant: tile-serial (every order) or software-pipelined across
-    // tiles (euler_split_pipe.cu; the default)
-    enum { CLASSIC = 0, PIPE = 1 };
-    int variant = CLASSIC;
+    int sm_budget = 0;        // SMs the persistent grid is sized for, one CTA each (0: all)
 };
 
 cudaError_t launch_euler_split(int N, const EulerArgs& a, const SplitPlan& plan, cudaStream_t s);

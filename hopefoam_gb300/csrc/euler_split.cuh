@@ -1,6 +1,6 @@
 // euler_split.cuh -- shared definitions of the split-precision Euler stage
-// kernels (euler_split.cu, euler_split_pipe.cu): tile sizes and the
-// shared-memory layout per order, the kernel arguments, the GEMM2 row order.
+// (euler_split.cu, euler_split_pipe.cu): tile and operand sizes per order,
+// the kernel arguments, the GEMM2 row order.
 #pragma once
 
 #include <cstdint>
@@ -45,7 +45,7 @@ struct SplitDims {
     static constexpr int FW = (Nfq + 1) / 2;
     static constexpr int FPW = 32 / FW;
     static_assert(FP == 1 || (16 * FPW >= 3 * E && 2 * FW >= Nfp), "one-pass face groups");
-    // shared-memory layout (bytes, operand buffers 1024-aligned)
+    // operand sizes (bytes; their places: PipeDims in euler_split_pipe.cu)
     static constexpr int SZ_B1 = 2 * NG * KP1 * 4;    // Vg hi/lo
     static constexpr int SZ_BC = 2 * NP2 * KC * 4;    // one streamed [Sr|Ss] chunk hi/lo
     static constexpr int SZ_B2 = STREAM ? 2 * NP2 * NF * 4    // Lift hi/lo
@@ -55,35 +55,14 @@ struct SplitDims {
     static constexpr int SZ_AF = 2 * ROWS * NF * 4;   // face flux hi/lo
     static constexpr int SZ_QF = STREAM ? 0 : E * 4 * Np * 4;   // FP32 deltas of the tile state
     static constexpr int SZ_Q64 = STREAM ? 0 : E * 4 * Np * 8;  // FP64 tile state
-    // reference state FP32 (+ FP64 copy on the resident path), FP32 metrics
-    static constexpr int OFF_GEO_IN_QB = ROWS * 4 + (STREAM ? 0 : ROWS * 8);
-    static constexpr int SZ_QB = OFF_GEO_IN_QB + E * 4 * 4;
     // the neighbour traces of the tile's faces, FP64 [3 E][Nfp][4], gathered
-    // by asynchronous copies while the tile is staged, where shared memory
-    // has room for them (N <= 5); otherwise the face phase loads them itself
+    // by asynchronous copies where shared memory has room for them (N <= 5);
+    // otherwise the face phase loads them itself
     static constexpr int SZ_NB_FULL = 3 * E * Nfp * 4 * 8;
     static constexpr int al(int x) { return (x + 1023) / 1024 * 1024; }
-    static constexpr int OFF_B1 = 0;
-    static constexpr int OFF_B2 = OFF_B1 + al(SZ_B1);
     static constexpr int AL_BC = al(SZ_BC);           // stride between streamed operand buffers
-    static constexpr int OFF_BC = OFF_B2 + al(SZ_B2);
-    static constexpr int OFF_A1 = OFF_BC + (STREAM ? NBUF * AL_BC : 0);
-    static constexpr int OFF_AC = OFF_A1 + al(SZ_A1);
     static constexpr int AL_AC = al(SZ_AC);           // stride between chunk buffers
-    static constexpr int OFF_AF = OFF_AC + NBUF * AL_AC;
-    static constexpr int OFF_QF = OFF_AF + al(SZ_AF);
-    static constexpr int OFF_Q64 = OFF_QF + al(SZ_QF);
-    static constexpr int OFF_QB = OFF_Q64 + al(SZ_Q64);
-    static constexpr int OFF_NB = OFF_QB + al(SZ_QB);
-    static constexpr bool GATHER = !STREAM && OFF_NB + al(SZ_NB_FULL) + 64 <= 232448;
-    static constexpr int SZ_NB = GATHER ? SZ_NB_FULL : 0;
-    static constexpr int OFF_BAR = OFF_NB + al(SZ_NB);
-    static constexpr int SMEM = OFF_BAR + 64;
-    static constexpr int RS_FLOATS = E * 4 * Np;      // epilogue staging (aliases chunk buffer 0)
-    static constexpr int TILE_VALS = E * 4 * Np;
-    static constexpr int EPI = (TILE_VALS + THREADS - 1) / THREADS;  // tile values per thread
-    static_assert(RS_FLOATS * 4 <= SZ_AC, "epilogue staging does not fit");
-    static_assert(SMEM <= 232448, "shared memory budget");
+    static_assert(E * 4 * Np * 4 <= SZ_AC, "epilogue staging (in chunk buffer 0) does not fit");
     static_assert(Nfq <= SW && Nfp <= SW, "face segment width");
     static_assert(!STREAM || NBUF == 2, "streamed operand buffers pair with two chunk buffers");
     static constexpr int TMEM_COLS = 256;
@@ -116,7 +95,7 @@ constexpr uint32_t kWaitLimit = 1u << 22;
 // stores are free of bank conflicts.  GEMM1 keeps r = 4 e + v.
 __device__ __forceinline__ int g2row(int e, int v) { return ((e >> 3) << 5) | (v << 3) | (e & 7); }
 
-// one stage of several contexts (orders 1..6, pipelined body) in one launch:
+// one stage of several contexts (orders 1..6) in one launch:
 // group g runs on blocks [cta_end[g-1], cta_end[g])
 struct SplitBatchArgs {
     static constexpr int MAXG = 8;
@@ -131,9 +110,7 @@ cudaError_t launch_split_batch(const SplitBatchArgs& P, cudaStream_t s);
 // the stage's kernel arguments from the context-level ones (FP32 scalars, tables)
 int split_fill_args(const EulerArgs& a, const SplitPlan& plan, SplitArgs* sa);
 
-// the pipelined variant of the stage (euler_split_pipe.cu): the
-// next tile's staging runs under this tile's volume phase and its face phase
-// under this tile's epilogue
+// the stage's kernel (euler_split_pipe.cu)
 template <int N>
 cudaError_t launch_split_pipe(const SplitArgs& sa, int grid, cudaStream_t s);
 template <int N>

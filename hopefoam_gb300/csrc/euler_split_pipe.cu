@@ -1,14 +1,10 @@
 // euler_split_pipe.cu -- the split-precision fused DG Euler stage,
-// software-pipelined across tiles (sm_103a).
+// software-pipelined across tiles (sm_103a).  Arithmetic and operands: euler_split.cu.
 //
-// Same arithmetic, operands, tensor-memory layout and results as
-// euler_stage_split_kernel (euler_split.cu, which documents them); only the
-// order of the work per CTA differs.  There, every phase of a tile runs
-// between two CTA barriers, so the FP64-pipe work of staging (one FP64
-// subtraction and conversion per staged value; GB300 retires two FP64
-// operations per clock per SM) and the memory latency of the epilogue leave
-// the other pipes idle.  Here tile t+1's phases are interleaved with tile t's,
-// and no phase ends in a CTA barrier: sixteen compute warps hand over through
+// The FP64-pipe work of staging (one FP64 subtraction and conversion per staged value;
+// GB300 retires two FP64 operations per clock per SM) and the memory latency of the
+// epilogue leave the other pipes idle.  So tile t+1's phases are interleaved with tile
+// t's, and no phase ends in a CTA barrier: sixteen compute warps hand over through
 // mbarriers, each waiting only for what it is about to read or overwrite, and
 // one thread of a warp of its own issues every MMA and bulk copy.
 //
@@ -45,8 +41,8 @@
 // 202, 277, 330, 410; with the wait for the other warps' face phase moved behind
 // the first fluxes 111, 136, 199, 257, 307, 407; with the face fluxes in the
 // wait for GEMM2 107, 130, 184, 236, 309, 395; with the traces requested by other
-// warps (N <= 5) 105, 131, 181, 234, 296.  N = 7, K = 320,000, against the
-// tile-serial kernel: Roe 1609 -> 1430, Lax-Friedrichs 1523 -> 1346.  Measured and left out: face fluxes
+// warps (N <= 5) 105, 131, 181, 234, 296.  N = 7, K = 320,000, against a
+// kernel with the phases one after another: Roe 1609 -> 1430, Lax-Friedrichs 1523 -> 1346.  Measured and left out: face fluxes
 // in three warps of their own beside the issuer (359 us at N = 5, 320 at N = 4:
 // a face is a long chain, and three warps do not keep up).
 //
@@ -352,7 +348,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
             const int Gc = gok ? Gf : min(warp * FPW, 3 * E - 1);
             const int e = Gc / 3, f = Gc - 3 * e;
             const bool valid = gok && e < ne;
-            const int k = k0 + (valid ? e : 0);
+            [[maybe_unused]] const int k = k0 + (valid ? e : 0);
             float qbv[4];
             double qbdv[4];
 #pragma unroll
@@ -480,7 +476,7 @@ __device__ __forceinline__ void pipe_body(const SplitArgs& sa, const int bid, co
                 const int Gc = gok ? Gf : gbase;
                 const int e = Gc / 3, f = Gc - 3 * e;
                 const bool valid = gok && e < ne;
-                const int k = k0 + (valid ? e : 0);
+                [[maybe_unused]] const int k = k0 + (valid ? e : 0);
                 float own[4] = {0.f, 0.f, 0.f, 0.f}, nbr[4] = {0.f, 0.f, 0.f, 0.f};
                 float qbv[4];
                 double qbdv[4];
