@@ -106,3 +106,48 @@ def test_no_memory_for_rows(gpu_lib, tmp_path, N):
     solve: the stopping tolerance, and round-off of the norm)."""
     so = preload.compile_host(NO_ROWS, tmp_path / "no_rows.so")
     assert "solved" in preload.run(so, MATRIX_FREE, N)
+
+
+def test_solves_beside_each_other(gpu_lib):
+    """Two solvers whose iterations run in one cooperative launch, and Euler steps of a third context, from a host thread
+    each: every solve has the bits that it has alone."""
+    import concurrent.futures
+
+    import numpy as np
+
+    from hopefoam_gb300 import _lib as L
+    from hopefoam_gb300 import euler
+    from hopefoam_gb300.mesh import delaunay_square, periodic_square
+    from hopefoam_gb300.poisson import PressureSolver
+
+    def solver(n, N, seed):
+        m = delaunay_square(n, seed=seed)
+        return PressureSolver(m, N, tau_coef=1.0), np.random.default_rng(seed).standard_normal(m.K * (N + 1) * (N + 2) // 2)
+
+    jobs = [(*solver(2000, 3, 1), dict(pc=L.DG_PC_BLOCK_JACOBI, precision=L.DG_PREC_SPLIT)),
+            (*solver(900, 3, 2), dict(pc=L.DG_PC_MULTILEVEL, precision=L.DG_PREC_FP64))]
+    want = [ps.solve(b, rtol=1e-9, maxit=20000, **kw)[0] for ps, b, kw in jobs]
+    m = periodic_square(60, 60, 10.0, 10.0, perturb=0.1, seed=1)
+    ops = euler.reference_operators(4)
+    q = euler.isentropic_vortex(*euler.node_coords(m, ops["r"], ops["s"]), x0=5.0, y0=5.0)
+    ctx = euler.EulerContext(m, 4)
+    ctx.upload(q)
+    ctx.lserk4(1e-4, 60, precision=L.DG_PREC_SPLIT)
+    want_q = ctx.download()
+
+    def solve(ps, b, kw, x):
+        for _ in range(6):
+            assert np.array_equal(ps.solve(b, rtol=1e-9, maxit=20000, **kw)[0], x), kw
+
+    def step():
+        for _ in range(6):
+            ctx.upload(q)
+            ctx.lserk4(1e-4, 60, precision=L.DG_PREC_SPLIT)
+            assert np.array_equal(ctx.download(), want_q), "steps"
+
+    with concurrent.futures.ThreadPoolExecutor(3) as pool:
+        for f in [pool.submit(solve, *j, x) for j, x in zip(jobs, want)] + [pool.submit(step)]:
+            f.result()
+    for ps, _, _ in jobs:
+        ps.ctx.close()
+    ctx.close()
