@@ -410,8 +410,7 @@ def main():
                      "traffic": SPLIT_STAGE_TRAFFIC_N5 if (prec_name == "split" and order == 5 and args.nx == 256)
                      else None, "peak_kind": peak_kind, "bytes_per_elem_stage": bpe,
                      "frac_at_fp64_register_bytes": bpe_survey * mesh.K / per_launch_s / 1e9 / peak,
-                     "kernel": ("euler_stage_split_pipe_kernel<%d>" % order if prec_name == "split" and order <= 6
-                                else "euler_stage_%s_kernel<%d>" % (prec_name, order))},
+                     "kernel": "euler_stage_%s_kernel<%d>" % ({"split": "split_pipe", "fp64": "fp64_tc"}[prec_name], order)},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": n * 8, "d2h_bytes_per_step": n * 8},
         "gpu_launches": launches,
         "clocks": ck,

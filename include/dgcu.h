@@ -90,7 +90,8 @@ typedef struct dg_opts {
 typedef struct dg_info {
     int32_t K, order, Np, Ng, Nfp, Nfq, n_bfaces;
     void* stream;            /* the context's cudaStream_t */
-    size_t device_bytes;     /* device memory held by the context */
+    size_t device_bytes;     /* device memory of the context's states, operators and traces; what a
+                                pressure operator, a limiter or the split stage hold comes on top */
 } dg_info;
 
 typedef struct dg_solve_stats {
@@ -177,10 +178,9 @@ int dg_set_element_dt(dg_ctx* ctx, const double* dtk_host);
  * order, each over the disjoint meshes of its cases); dg_batch_run advances
  * every group nsteps LSERK4 steps in one CUDA-graph launch (captured on the
  * first run with these arguments, replayed after).  dg_batch_tune measures
- * launch shapes on the live state (restored afterwards): CTAs per SM of the
- * split kernel where two fit, and three schedules: the groups one after
- * another on the whole GPU, side by side on streams with SM shares
- * proportional to their measured cost, or (split precision, orders <= 6, up
+ * three schedules on the live state (restored afterwards): the groups one after
+ * another on the whole GPU, side by side on streams with SM shares by what
+ * each needs beside the others, or (split precision, orders <= 6, up
  * to 8 groups) every stage of every group in one persistent mixed-order
  * launch, each group on its SM share; the fastest is kept.  No counterpart in the reference.  The groups must not
  * be used on their own streams while a dg_batch_run is in flight. */
@@ -196,10 +196,11 @@ int dg_batch_create(dg_ctx* const* groups, int n_groups, dg_batch** out);
 int dg_batch_destroy(dg_batch* batch);
 const char* dg_batch_last_error(const dg_batch* batch);
 int dg_batch_tune(dg_batch* batch, double dt, int flux, int precision, int steps_per_trial, dg_batch_tuning* result);
+/* ctas_per_sm is 1: a CTA takes an SM's registers. */
 int dg_batch_get_shape(const dg_batch* batch, int group, int* ctas_per_sm, int* sm_budget, int* concurrent);
 /* Fixes the schedule (0, 1 or 2 as in dg_batch_tuning.concurrent) without
- * measuring; SM shares from the last tuning, else in proportion to each
- * group's element nodes.  DG_ERR_UNSUPPORTED when schedule 2 is not possible. */
+ * measuring; SM shares from the last tuning, else by each group's elements
+ * and order.  DG_ERR_UNSUPPORTED when schedule 2 is not possible. */
 int dg_batch_set_schedule(dg_batch* batch, int schedule, int precision);
 int dg_batch_run(dg_batch* batch, double dt, int nsteps, int flux, int precision, double* ms);
 
@@ -210,7 +211,10 @@ int dg_batch_run(dg_batch* batch, double dt, int nsteps, int flux, int precision
  * boundary faces are homogeneous Dirichlet (fixesValue, :157-209).  Builds
  * the reference stiffness parts and the block-Jacobi inverse on the device.
  * Replaces the per-element assembly of laplacianFunc (:63-288) and
- * dgMatrix::assembleMatrix (dgMatrices/dgMatrix/dgMatrix.C:383-438). */
+ * dgMatrix::assembleMatrix (dgMatrices/dgMatrix/dgMatrix.C:383-438).  The
+ * first FP64 solve adds assembled rows, 32 Np (Np + 1) bytes an element and at
+ * most 8 GB (above, or where the memory is missing, the solves are
+ * matrix-free); both are held until the operator is set up again or the context destroyed. */
 int dg_ipdg_setup(dg_ctx* ctx, double tau_coef);
 
 /* Boundary types of the operator per boundary slot (the context's boundary
