@@ -29,7 +29,7 @@
 // whose fluxes leave that bound or stay too far below it, whose density or
 // energy varies too much (kFluxSlack, kRhoDepth, kEnergyDepth), or with values that
 // are not finite or outside the FP32 exponent range, is left to plain FP64 after the
-// tiles, as euler_fp64.cu does it (plain_element).  All of this is per element:
+// tiles, as euler_fp64.cu does it (plain_elements).  All of this is per element:
 // results do not depend on an element's place in the mesh.
 //
 // Measured, LSERK4 stage in a queue of steps, against the kernel of euler_fp64.cu: K = 32768,
@@ -257,89 +257,116 @@ __device__ __forceinline__ void stage_update(const EulerArgs& a, size_t idx, dou
     }
 }
 
-// Stage of element k in plain FP64 by the 128 threads of its group,
-// operation for operation as euler_stage_fp64_kernel forms it
+// Stage of nb <= D::PB elements of a group in plain FP64 by its 128 threads,
+// operation for operation as euler_stage_fp64_kernel forms it; element b is
+// gk0 + ((list >> 4 b) & 7), sc(i) scratch value i.  Several at once: at low orders one
+// element leaves most threads idle.  With every element on this route (K = 32768,
+// N = 1, 3, 5; K = 9800, N = 7, a right-hand side): 980, 1736, 3516, 3683 us one at a time with
+// rolled loops, 398, 1020, 2293, 2098 so; euler_fp64.cu 168, 817, 2616, 2256.
 template <int N, typename Sc>
-__device__ __noinline__ void plain_element(const EulerArgs& a, int k, int t, int sub, Sc sc) {
+__device__ __forceinline__ void plain_elements(const EulerArgs& a, int gk0, uint32_t list, int nb, int t, int sub, Sc sc) {
     using D = OzDims<N>;
-    constexpr int Np = D::Np, Ng = D::Ng, Nfp = D::Nfp, Nfq = D::Nfq, NB = D::NB, NF = D::NF;
-    const double* qe = a.qin + (size_t)k * 4 * Np;
-    const double* gk = a.geo + (size_t)k * 4;
-    const double rx = gk[0], sx = gk[1], ry = gk[2], sy = gk[3], gamma = a.gamma;
+    constexpr int Np = D::Np, Ng = D::Ng, Nfp = D::Nfp, Nfq = D::Nfq, NB = D::NB, NF = D::NF, SS = D::PLAIN_SCRATCH;
+    const double gamma = a.gamma;
+    auto element = [&](int b) { return gk0 + (int)((list >> (4 * b)) & 7u); };
 #pragma unroll 1
-    for (int g = t; g < Ng; g += 128) {
+    for (int it = t; it < nb * Ng; it += 128) {
+        const int b = it / Ng, g = it - b * Ng, k = element(b);
+        const double *qe = a.qin + (size_t)k * 4 * Np, *gk = a.geo + (size_t)k * 4;
         double q[4] = {0, 0, 0, 0}, fx[4], fy[4];
-#pragma unroll 1
+#pragma unroll 3
         for (int p = 0; p < Np; p++) {
-            const double w = a.ops.Vg[g * Np + p];
-#pragma unroll 1
-            for (int v = 0; v < 4; v++) q[v] += w * qe[v * Np + p];
+            const double w = __ldg(a.ops.Vg + g * Np + p);
+#pragma unroll
+            for (int v = 0; v < 4; v++) q[v] += w * __ldg(qe + v * Np + p);
         }
         euler_phys_flux(gamma, q, fx, fy);
-#pragma unroll 1
+        const double rx = gk[0], sx = gk[1], ry = gk[2], sy = gk[3];
+#pragma unroll
         for (int v = 0; v < 4; v++) {
-            *sc(v * Ng + g) = rx * fx[v] + ry * fy[v];
-            *sc((4 + v) * Ng + g) = sx * fx[v] + sy * fy[v];
+            *sc(b * SS + v * Ng + g) = rx * fx[v] + ry * fy[v];
+            *sc(b * SS + (4 + v) * Ng + g) = sx * fx[v] + sy * fy[v];
         }
     }
     // face fluxes, a thread a point; the wave speeds of a face meet in the scratch
-    const int f = t / Nfq, i = t - f * Nfq;
-    double nx = 0, ny = 0, fsc = 0, qm[4], qp[4];
-    if (t < NF) {
-        const int c = a.conn[(size_t)k * 3 + f];
-        face_normal(f, rx, sx, ry, sy, nx, ny, fsc);
-#pragma unroll 1
-        for (int v = 0; v < 4; v++) {
-            double m = 0, p = 0;
-#pragma unroll 1
-            for (int j = 0; j < Nfp; j++) {
-                const double w = a.ops.If[i * Nfp + j];
-                m += w * qe[v * Np + (f * N + j) % NB];
-                double o;
-                if (c >= 0) {
-                    const int fn = c & 3, jj = ((c >> 2) & 1) ? (N - j) : j;
-                    o = a.qin[((size_t)(c >> 3) * 4 + v) * Np + (fn * N + jj) % NB];
-                } else {
-                    o = a.btrace[((size_t)(-1 - c) * 4 + v) * Nfp + j];
-                }
-                p += w * o;
+    const int b = t / NF, fq = t - b * NF, f = fq / Nfq, i = fq - f * Nfq;
+    const bool face = t < nb * NF;
+    double nx = 0, ny = 0, fsc = 0, qm[4] = {0, 0, 0, 0}, qp[4] = {0, 0, 0, 0};
+    if (face) {
+        const int k = element(b), c = a.conn[(size_t)k * 3 + f];
+        const double *qe = a.qin + (size_t)k * 4 * Np, *gk = a.geo + (size_t)k * 4;
+        face_normal(f, gk[0], gk[1], gk[2], gk[3], nx, ny, fsc);
+        const int fn = c & 3;
+        const bool turned = (c >> 2) & 1;
+        const double* qn = c >= 0 ? a.qin + (size_t)(c >> 3) * 4 * Np : a.btrace + (size_t)(-1 - c) * 4 * Nfp;
+        const int stride = c >= 0 ? Np : Nfp;
+#pragma unroll 2
+        for (int j = 0; j < Nfp; j++) {
+            const double w = __ldg(a.ops.If + i * Nfp + j);
+            const int own = (f * N + j) % NB, other = c >= 0 ? (fn * N + (turned ? N - j : j)) % NB : j;
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                qm[v] += w * __ldg(qe + v * Np + own);
+                qp[v] += w * __ldg(qn + v * stride + other);
             }
-            qm[v] = m;
-            qp[v] = p;
         }
-        if (a.flux != 1) *sc(8 * Ng + 4 * NF + t) = fmax(wave_speed(gamma, nx, ny, qm), wave_speed(gamma, nx, ny, qp));
+        if (a.flux != 1) *sc(b * SS + 8 * Ng + 4 * NF + fq) = fmax(wave_speed(gamma, nx, ny, qm), wave_speed(gamma, nx, ny, qp));
     }
     if (a.flux != 1) group_sync(sub);
-    if (t < NF) {
+    if (face) {
         double F[4], lam = 0;
         if (a.flux == 1) {
             roe_flux(gamma, nx, ny, qm, qp, F);
         } else {
 #pragma unroll 1
-            for (int j = 0; j < Nfq; j++) lam = fmax(lam, *sc(8 * Ng + 4 * NF + f * Nfq + j));
+            for (int j = 0; j < Nfq; j++) lam = fmax(lam, *sc(b * SS + 8 * Ng + 4 * NF + f * Nfq + j));
             lf_flux(gamma, nx, ny, lam, qm, qp, F);
         }
-#pragma unroll 1
-        for (int v = 0; v < 4; v++) *sc(8 * Ng + v * NF + t) = fsc * F[v];
+#pragma unroll
+        for (int v = 0; v < 4; v++) *sc(b * SS + 8 * Ng + v * NF + fq) = fsc * F[v];
     }
     group_sync(sub);
 #pragma unroll 1
-    for (int it = t; it < 4 * Np; it += 128) {
-        const int v = it / Np, p = it - v * Np;
+    for (int it = t; it < nb * 4 * Np; it += 128) {
+        const int b = it / (4 * Np), r = it - b * 4 * Np, v = r / Np, p = r - v * Np, k = element(b);
         double acc = 0, acc2 = 0, accf = 0;
-#pragma unroll 1
+#pragma unroll 4
         for (int g = 0; g < Ng; g++) {
-            acc += a.ops.Sr[p * Ng + g] * *sc(v * Ng + g);
-            acc2 += a.ops.Ss[p * Ng + g] * *sc((4 + v) * Ng + g);
+            acc += __ldg(a.ops.Sr + p * Ng + g) * *sc(b * SS + v * Ng + g);
+            acc2 += __ldg(a.ops.Ss + p * Ng + g) * *sc(b * SS + (4 + v) * Ng + g);
         }
         acc += acc2;
-#pragma unroll 1
-        for (int q = 0; q < NF; q++) accf += a.ops.Lift[p * NF + q] * *sc(8 * Ng + v * NF + q);
-        const size_t idx = (size_t)k * 4 * Np + it;
+#pragma unroll 3
+        for (int q = 0; q < NF; q++) accf += __ldg(a.ops.Lift + p * NF + q) * *sc(b * SS + 8 * Ng + v * NF + q);
+        const size_t idx = (size_t)k * 4 * Np + r;
         stage_update(a, idx, step_of(a, k) * (acc - accf), a.qin[idx],
                      a.mode == MODE_LSERK ? a.res[idx] : a.mode == MODE_SSP2 ? a.qold[idx] : 0.0);
     }
     group_sync(sub);
+}
+
+// The elements of the block's tiles that are left to plain FP64 (none, as a rule), by one
+// group's threads.  The group's flags are thread 0's stores, the last tile's with no
+// barrier behind it yet: every thread must read the same, since plain_elements has the
+// group's barriers inside.  A call, after the tiles, so that it costs their loop no registers.
+template <int N>
+__device__ __noinline__ void plain_pass(const OzArgs& oa, unsigned char* smem, int t, int sub) {
+    using D = OzDims<N>;
+    const int tile_elems = 8 * oa.groups, K = oa.e.K;
+    group_sync(sub);
+    for (int k0 = (int)blockIdx.x * tile_elems; k0 < K; k0 += (int)gridDim.x * tile_elems) {
+        const int gk0 = k0 + 8 * sub;
+        uint32_t fl = oa.flags[gk0 >> 3] & ((1u << max(0, min(8, K - gk0))) - 1u);
+        while (fl) {
+            uint32_t list = 0;
+            int nb = 0;
+            for (; fl && nb < D::PB; fl &= fl - 1) list |= (uint32_t)(__ffs((int)fl) - 1) << (4 * nb++);
+            plain_elements<N>(oa.e, gk0, list, nb, t, sub, [&](int j) {
+                return j < D::A1_SCRATCH ? striped(smem + D::OFF_A1, sub, j, D::A1S, 32 * D::K1 * 2)
+                                         : striped(smem + D::OFF_A2, sub, j - D::A1_SCRATCH, D::A2S, 2048);
+            });
+        }
+    }
 }
 
 }  // namespace
@@ -878,17 +905,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) euler_stage_fp64_tc_kernel(OzAr
                 }
             }
         }
-        // the elements left to plain FP64 (none, as a rule), after the tiles so that
-        // the call costs the loop above no registers.  The group's flags are thread 0's
-        // stores, the last tile's with no barrier behind it yet: every thread must read
-        // the same, since plain_element has the group's barrier inside
-        group_sync(sub);
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-            for (uint32_t fl = oa.flags[oa.groups * tile + sub]; fl; fl &= fl - 1) {
-                const int k = tile * tile_elems + 8 * sub + __ffs((int)fl) - 1;
-                if (k < a.K)
-                    plain_element<N>(a, k, t, sub, [&](int j) { return striped(A1, sub, j, D::A1S, 32 * K1 * 2); });
-            }
+        plain_pass<N>(oa, smem, t, sub);
     }
     umma::fence_before_sync();
     __syncthreads();

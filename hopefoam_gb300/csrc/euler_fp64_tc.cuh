@@ -76,7 +76,13 @@ struct OzDims {
     static constexpr int OFF_BAR = (OFF_TMEM + 4 + 7) / 8 * 8;    // mbarriers
     static constexpr int SMEM = OFF_BAR + (8 + 2 * NSLOT) * 8;
     static_assert(SMEM <= 232448, "shared memory");
-    static_assert((8 * Ng + 5 * NF) * 8 <= oz::kSlices * 32 * K1 * 2, "scratch of the plain route");
+    // the plain route: scratch values per element, those of a group in the first operand and
+    // in both, and how many elements it takes at once
+    static constexpr int PLAIN_SCRATCH = 8 * Ng + 5 * NF;
+    static constexpr int A1_SCRATCH = oz::kSlices * 32 * K1 * 2 / 8, A12_SCRATCH = A1_SCRATCH + oz::kSlices * 2048 / 8;
+    static constexpr int cmin(int a, int b) { return a < b ? a : b; }
+    static constexpr int PB = cmin(8, cmin(128 / NF, A12_SCRATCH / PLAIN_SCRATCH));
+    static_assert(PB >= 1 && PB * NF <= 128 && PB * PLAIN_SCRATCH <= A12_SCRATCH, "scratch of the plain route");
     static_assert(32 * Np * 8 <= oz::kSlices * 2048, "result staging");
 };
 
