@@ -113,48 +113,62 @@ OzImage oz_build(const dgb::RefOps& o) {
                             bound(o.dLift, (size_t)n * D::NF, D::NF));
     im.eb[D::NP2] = ebV;
     im.eb[D::NP2 + 1] = ebI;
-    // largest possible |accumulator| per result column and digit group, the
-    // activation digits at their largest (128): |a| sum |b|
-    long long worst1 = 0, worst2 = 0;
-    std::vector<long long> acc2((size_t)8 * D::NP2, 0);
-    auto put = [&](int piece, int P, int KP, int n, int k, double v, int eb, std::vector<long long>* acc) {
-        unsigned char* base = im.bytes.data() + D::piece_off(piece);
+    // FP16 bits of every digit, and where the pieces are
+    uint16_t half[257];
+    for (int d = -128; d <= 128; d++) half[d + 128] = oz::half_bits(d);
+    size_t at[D::PIECES];
+    for (size_t i = 0, o = 0; i < (size_t)D::PIECES; o += D::piece_bytes((int)i++)) at[i] = o;
+    // digits of one operator value into a piece; |digit| into the sums of its result column, by digit
+    auto put = [&](int piece, int P, int KP, int n, int k, double v, int eb, std::vector<int>& sum) {
+        unsigned char* base = im.bytes.data() + at[piece];
         const uint64_t y = oz::biased(v, eb);
         for (int j = 0; j < oz::kSlices; j++) {
             const int d = oz::digit(y, j);
-            const uint16_t h = oz::half_bits(d);
-            memcpy(base + oz_off(j * P + n, k, KP), &h, 2);
-            for (int s = j; acc && s < std::min(8, j + oz::kSlices); s++) (*acc)[(size_t)s * P + n] += 128ll * (d < 0 ? -d : d);
+            memcpy(base + oz_off(j * P + n, k, KP), &half[d + 128], 2);
+            sum[(size_t)j * P + n] += d < 0 ? -d : d;
         }
     };
+    // largest possible |accumulator| over the columns and digit groups i + j = s, the
+    // activation digits at their largest (128): |a| sum |b|
+    auto worst = [&](const std::vector<int>& sum, int P) {
+        long long m = 0;
+        for (int n = 0; n < P; n++)
+            for (int s = 0; s < 8; s++) {
+                long long t = 0;
+                for (int j = std::max(0, s - oz::kSlices + 1); j <= std::min(s, oz::kSlices - 1); j++) t += sum[(size_t)j * P + n];
+                m = std::max(m, 128 * t);
+            }
+        return m;
+    };
+    long long worst1 = 0;
+    std::vector<int> sum2((size_t)oz::kSlices * D::NP2, 0);
     // own nodes -> face points; neighbour face nodes -> face points
     {
-        std::vector<long long> a1((size_t)8 * 32, 0), a3((size_t)8 * 32, 0);
+        std::vector<int> s1((size_t)oz::kSlices * 32, 0), s3((size_t)oz::kSlices * 32, 0);
         for (int f = 0; f < 3; f++)
             for (int i = 0; i < D::Nfq; i++)
                 for (int j = 0; j < D::Nfp; j++) {
                     const double v = o.If[(size_t)i * D::Nfp + j];
-                    put(0, 32, D::K1, f * D::Nfq + i, (f * N + j) % D::NB, v, ebI, &a1);
-                    put(1, 32, 32, f * D::Nfq + i, f * D::Nfp + j, v, ebI, &a3);
+                    put(0, 32, D::K1, f * D::Nfq + i, (f * N + j) % D::NB, v, ebI, s1);
+                    put(1, 32, 32, f * D::Nfq + i, f * D::Nfp + j, v, ebI, s3);
                 }
-        for (long long x : a1) worst1 = std::max(worst1, x);
-        for (long long x : a3) worst1 = std::max(worst1, x);
+        worst1 = std::max(worst(s1, 32), worst(s3, 32));
     }
     for (int c = 0; c < D::NC; c++) {
-        std::vector<long long> a((size_t)8 * 16, 0);
+        std::vector<int> s1((size_t)oz::kSlices * 16, 0);
         for (int p = 0; p < 16 && 16 * c + p < D::Ng; p++) {
             const int g = 16 * c + p;
-            for (int k = 0; k < D::Np; k++) put(D::piece_b1(c), 16, D::K1, p, k, o.dVg[(size_t)g * D::Np + k], ebV, &a);
+            for (int k = 0; k < D::Np; k++) put(D::piece_b1(c), 16, D::K1, p, k, o.dVg[(size_t)g * D::Np + k], ebV, s1);
             for (int n = 0; n < D::Np; n++) {
-                put(D::piece_b2(c), D::NP2, 32, n, 2 * p, o.dSr[(size_t)n * D::Ng + g], im.eb[n], &acc2);
-                put(D::piece_b2(c), D::NP2, 32, n, 2 * p + 1, o.dSs[(size_t)n * D::Ng + g], im.eb[n], &acc2);
+                put(D::piece_b2(c), D::NP2, 32, n, 2 * p, o.dSr[(size_t)n * D::Ng + g], im.eb[n], sum2);
+                put(D::piece_b2(c), D::NP2, 32, n, 2 * p + 1, o.dSs[(size_t)n * D::Ng + g], im.eb[n], sum2);
             }
         }
-        for (long long x : a) worst1 = std::max(worst1, x);
+        worst1 = std::max(worst1, worst(s1, 16));
     }
     for (int n = 0; n < D::Np; n++)
-        for (int q = 0; q < D::NF; q++) put(3, D::NP2, 32, n, q, -o.dLift[(size_t)n * D::NF + q], im.eb[n], &acc2);
-    for (long long x : acc2) worst2 = std::max(worst2, x);
+        for (int q = 0; q < D::NF; q++) put(3, D::NP2, 32, n, q, -o.dLift[(size_t)n * D::NF + q], im.eb[n], sum2);
+    const long long worst2 = worst(sum2, D::NP2);
     bool fits = true;
     auto ratio = [](double v, int eb) { return std::ldexp(std::fabs(v), 1022 - eb); };
     for (int g = 0; g < D::Ng; g++) {
