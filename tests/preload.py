@@ -23,7 +23,9 @@ def compile_host(src, out, *more):
 
 def run(so, code, *args, timeout=300):
     """`code` in a child process with `so` loaded first; its output."""
-    env = dict(os.environ, LD_PRELOAD=so, PYTHONPATH=ROOT + os.pathsep + HERE)
+    before = lambda *p: ":".join(filter(None, p))
+    env = dict(os.environ, LD_PRELOAD=before(so, os.environ.get("LD_PRELOAD")),
+               PYTHONPATH=before(ROOT, HERE, os.environ.get("PYTHONPATH")))
     r = subprocess.run([sys.executable, "-c", code, *map(str, args)], cwd=ROOT, env=env, capture_output=True, text=True,
                        timeout=timeout)
     assert r.returncode == 0, r.stdout + r.stderr
